@@ -60,13 +60,16 @@ struct TempoLaunch {
   int smem_bytes;            // capacity of the dynamic shared buffer
 };
 
-// Per-CTA workspace: three FP64 complex matrices of wcap elements (W, theta
-// copy / temporaries, carry) and one double-float complex one (mixed form).
-inline long long tempo_work_bytes(long long wcap) { return wcap * (3 * 16 + 16); }
+// Global room for the QR bookkeeping of the widest split (1152 columns, 36
+// bytes each), used when a launch has little shared memory.
+constexpr long long QR_BOOK_BYTES = 48 * 1024;
 
-// precision: 0 = complex128 (FP64 Jacobi), 1 = mixed (double-float Jacobi
-// on the FP32 pipe; FP64 sites, contractions, rotation angles, norms, rank
-// decisions and read-out)
+// Per-CTA workspace: four matrices of wcap 16-byte elements (the QR's row
+// factor, theta / temporaries, carry, the split's working matrix).
+inline long long tempo_work_bytes(long long wcap) { return wcap * (4 * 16) + QR_BOOK_BYTES; }
+
+// precision: 0 = complex128 (FP64), 1 = mixed (double-float on the FP32 pipe;
+// FP64 rank decisions and read-out)
 cudaError_t launch_tempo_order(InstState* state, int* order, int n, cudaStream_t stream);
 cudaError_t launch_tempo(const TempoLaunch& L, int precision, int grid, int block,
                          int smem_bytes, cudaStream_t stream);
@@ -120,9 +123,9 @@ struct PtLaunch {
   int smem_bytes;
 };
 
-// Per-CTA PT workspace: four FP64 complex matrices (working matrix, U,
-// carry, theta) and one double-float matrix.
-inline long long pt_work_bytes(long long wcap) { return wcap * (4 * 16 + 16); }
+// Per-CTA PT workspace: five matrices of wcap 16-byte elements (U, carry,
+// theta, the QR's row factor, the split's working matrix).
+inline long long pt_work_bytes(long long wcap) { return wcap * (5 * 16) + QR_BOOK_BYTES; }
 
 cudaError_t launch_pt(const PtLaunch& L, int precision, int grid, int block, cudaStream_t stream);
 

@@ -166,6 +166,16 @@ __device__ __forceinline__ cff cff_scale(const cff& a, ff s) {
   return r;
 }
 
+// x * 2^e for a double-float complex x: exact (two float multiplications by
+// a power of two) unless it leaves the float range.
+__device__ __forceinline__ cff cff_ldexp(cff x, float p2) {
+  x.x.hi *= p2;
+  x.x.lo *= p2;
+  x.y.hi *= p2;
+  x.y.lo *= p2;
+  return x;
+}
+
 __device__ __forceinline__ cff cff_conj(cff a) {
   a.y.hi = -a.y.hi;
   a.y.lo = -a.y.lo;

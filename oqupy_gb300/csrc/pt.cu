@@ -46,6 +46,110 @@ struct RowMajor {
   __device__ zc operator()(int r, int c) const { return p[(size_t)r * ld + c]; }
 };
 
+// The oriented matrix of a PT split: X(r, c) (complex128), or its conjugate
+// transpose, in the split's arithmetic.
+template <typename T, class Acc>
+struct PtSource {
+  typedef QA<T> Q;
+  const Acc& X;
+  bool trans;
+  __device__ __forceinline__ zc at(int r, int c) const { return trans ? X(c, r) : X(r, c); }
+  __device__ __forceinline__ unsigned key(int r, int c) const { return QA<double>::mag_key(at(r, c)); }
+  __device__ __forceinline__ int exponent(unsigned key) const { return QA<double>::key_exponent(key); }
+  __device__ __forceinline__ void load(typename Q::E* W, int R, int N, int e) const {
+    const double p2 = ldexp(1.0, -e);
+    for (int idx = threadIdx.x; idx < R * N; idx += blockDim.x) {
+      const int c = idx / R, r = idx - c * R;
+      const zc x = cscale(at(r, c), p2);
+      W[idx] = Q::from(trans ? cconj(x) : x);
+    }
+  }
+};
+
+struct PtBufs {
+  zc* Tg;        // U output / temporaries
+  zc* Cg;        // carry
+  SplitBufs sb;
+};
+
+// Truncated split of the m x n matrix X:
+//   U  (m x kk, column-major, in Tg)      left singular vectors,
+//   C  (kk x n, row-major, in Cg)         S V^H (the carry),
+// with kk the kept rank of the relative tail rule.  The caller copies U to its
+// destination after the call (U never aliases X, so X may be the destination).
+// The contractions that form U and C are FP64 in both forms.  Returns kk
+// (>= 1); on failure sets *status (nonzero) and returns 0.
+template <bool MIXED, class Acc>
+__device__ int split_generic(const Acc& X, int m, int n, double epsrel, float qr_delta, int cap, const PtBufs& b,
+                             SplitShared& sh, PtState* st) {
+  typedef typename StepType<MIXED>::T T;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const bool trans = n > m;
+  const int R = trans ? n : m, N = trans ? m : n;
+  const PtSource<T, Acc> src{X, trans};
+  const SplitOut<T> o = oriented_split<T>(src, R, N, epsrel, qr_delta, b.sb, sh);
+  const int kk = o.kk;
+  if (tid == 0) {
+    st->sweeps64 += sh.jsh.sweeps;  // mixed form: FP64 fallback sweeps only
+    st->sweepsff += MIXED ? sh.jsh.sweeps32 : 0;
+    st->flops_alg += 4.0 * (6.0 * R * (double)N * N + 20.0 * (double)N * N * N);
+    if (sh.jsh.status != ST_OK || kk > cap) st->status = (sh.jsh.status != ST_OK) ? sh.jsh.status : ST_CHI_OVERFLOW;
+  }
+  if (sh.jsh.status != ST_OK || kk > cap) {
+    __syncthreads();
+    return 0;
+  }
+  // the kept columns in FP64 and the units of X, their norms replaced by 1 / s
+  // (U = W / s, C = U^H X) or 1 / s^2 (U = X W / s^2, C = W^H)
+  const bool wt = o.flip ? !trans : trans;
+  const int ld = wt ? n : m;
+  zc* W = reinterpret_cast<zc*>(o.W);
+  const double scale = ldexp(1.0, o.e);
+  const int* perm = sh.book.perm;
+  for (int idx = tid; idx < kk * ld; idx += nt) {
+    const int j = idx / ld, r = idx - j * ld;
+    const size_t q = (size_t)perm[j] * ld + r;
+    W[q] = cscale(QA<T>::to(o.W[q]), scale);
+  }
+  for (int j = tid; j < kk; j += nt) {
+    const double s = sh.book.norm[perm[j]];
+    sh.book.norm[perm[j]] = 1.0 / (wt ? s * s : s);
+  }
+  __syncthreads();
+  const double* sinv = sh.book.norm;
+  if (!wt) {
+    for (int idx = tid; idx < m * kk; idx += nt) {
+      const int j = idx / m, row = idx - j * m;
+      const int pj = perm[j];
+      b.Tg[idx] = cscale(W[(size_t)pj * m + row], sinv[pj]);
+    }
+    for (int idx = tid; idx < kk * n; idx += nt) {
+      const int j = idx / n, col = idx - j * n;
+      const int pj = perm[j];
+      const zc* u = W + (size_t)pj * m;
+      zc acc = mk<double>(0, 0);
+      for (int row = 0; row < m; ++row) cjfma(acc, u[row], X(row, col));
+      b.Cg[idx] = cscale(acc, sinv[pj]);
+    }
+  } else {
+    for (int idx = tid; idx < m * kk; idx += nt) {
+      const int j = idx / m, row = idx - j * m;
+      const int pj = perm[j];
+      const zc* w = W + (size_t)pj * n;
+      zc acc = mk<double>(0, 0);
+      for (int col = 0; col < n; ++col) cfma(acc, X(row, col), w[col]);
+      b.Tg[idx] = cscale(acc, sinv[pj]);
+    }
+    for (int idx = tid; idx < kk * n; idx += nt) {
+      const int j = idx / n, col = idx - j * n;
+      b.Cg[idx] = cconj(W[(size_t)perm[j] * n + col]);
+    }
+  }
+  if (tid == 0) st->flops_alg += 8.0 * (double)m * n * kk;
+  __syncthreads();
+  return kk;
+}
+
 template <bool MIXED>
 struct PtCtx {
   const PtLaunch* L;
@@ -55,7 +159,7 @@ struct PtCtx {
   const zc* infl;
   const zc* neg;
   zc* caps;
-  SplitBufs b;
+  PtBufs b;
   zc* Xg;  // theta buffer
   long long slot;
   __device__ zc* site(int k) const { return sites + (long long)k * slot; }
@@ -70,8 +174,7 @@ __device__ void sweep_rl(PtCtx<MIXED>& c, PtShared& sh, int k) {
   const int l = c.dims[k].x, r = c.dims[k].y;
   const int m = D * r, n = l;
   ColMajor X{A, m};
-  const int kk = split_generic<MIXED>(X, m, n, c.I->epsrel, c.I->qr_delta, c.I->cap, c.b, sh.ssh, &sh.st.status,
-                                      &sh.st.sweeps64, &sh.st.sweepsff, &sh.st.flops_alg);
+  const int kk = split_generic<MIXED>(X, m, n, c.I->epsrel, c.I->qr_delta, c.I->cap, c.b, sh.ssh, &sh.st);
   if (kk == 0) return;
   for (int idx = tid; idx < m * kk; idx += nt) A[idx] = c.b.Tg[idx];
   // absorb into k-1: (l2, D, n) x (kk, n)^T -> (l2, D, kk)
@@ -105,8 +208,7 @@ __device__ void sweep_lr(PtCtx<MIXED>& c, PtShared& sh, int k) {
   const int l = c.dims[k].x, r = c.dims[k].y;
   const int m = l * D, n = r;
   RowMajor X{A, r};
-  const int kk = split_generic<MIXED>(X, m, n, c.I->epsrel, c.I->qr_delta, c.I->cap, c.b, sh.ssh, &sh.st.status,
-                                      &sh.st.sweeps64, &sh.st.sweepsff, &sh.st.flops_alg);
+  const int kk = split_generic<MIXED>(X, m, n, c.I->epsrel, c.I->qr_delta, c.I->cap, c.b, sh.ssh, &sh.st);
   if (kk == 0) return;
   // U (m x kk, column-major in Tg) -> site [l][a][j]
   for (int idx = tid; idx < m * kk; idx += nt) {
@@ -255,8 +357,7 @@ __device__ void pt_step(PtCtx<MIXED>& c, PtShared& sh) {
       break;
     }
     ColMajor X{c.Xg, m};
-    const int kk = split_generic<MIXED>(X, m, n, I.epsrel, I.qr_delta, I.cap, c.b, sh.ssh, &sh.st.status,
-                                        &sh.st.sweeps64, &sh.st.sweepsff, &sh.st.flops_alg);
+    const int kk = split_generic<MIXED>(X, m, n, I.epsrel, I.qr_delta, I.cap, c.b, sh.ssh, &sh.st);
     if (kk == 0) return;
     // U((x,a), j) -> site [j][a][x]
     for (int idx = tid; idx < m * kk; idx += nt) {
@@ -330,13 +431,14 @@ __global__ void __launch_bounds__(PT_THREADS) pt_kernel(PtLaunch L) {
     c.neg = I->has_neg ? ((const zc*)L.neg + I->neg_base) : nullptr;
     c.caps = (zc*)L.caps + I->caps_base;
     unsigned char* work = (unsigned char*)L.work + (long long)blockIdx.x * L.work_stride;
-    c.b.Wg = (zc*)work;
-    c.b.Tg = c.b.Wg + L.wcap;
+    c.b.Tg = (zc*)work;
     c.b.Cg = c.b.Tg + L.wcap;
     c.Xg = c.b.Cg + L.wcap;
-    c.b.Wffg = (cff*)(c.Xg + L.wcap);
-    c.b.smem = dsm;
-    c.b.smem_bytes = L.smem_bytes;
+    c.b.sb.Wg = c.Xg + L.wcap;
+    c.b.sb.Xg = c.Xg + 2 * L.wcap;
+    c.b.sb.bkg = work + L.wcap * 80;
+    c.b.sb.smem = dsm;
+    c.b.sb.smem_bytes = L.smem_bytes;
     if (threadIdx.x == 0) sh.st = L.state[i];
     __syncthreads();
     if (sh.st.status == ST_OK && sh.st.step == 0) pt_initialize<MIXED>(c, sh);

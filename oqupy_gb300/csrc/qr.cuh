@@ -1,6 +1,6 @@
-// Rank-revealing QR preconditioner + one-sided Jacobi on the reduced factor:
-// the truncated bond split of both precision forms for splits of >= 8
-// columns (smaller splits run plain Jacobi, jacobi.cuh).
+// Rank-revealing QR + one-sided Jacobi on the reduced factor: the truncated
+// bond split of both precision forms for splits of >= 8 columns (smaller
+// splits run plain Jacobi, jacobi.cuh).
 //
 // Replaces, like jacobi.cuh, the truncated SVD that the reference obtains
 // from tensornetwork's split_node_full_svd(max_truncation_err=epsrel,
@@ -8,709 +8,431 @@
 // with the rank rule chi = #{i : sqrt(sum_{j>=i} s_j^2) > epsrel * s_0}
 // (oqupy/mps_mpo.py:452-457).
 //
-// The oriented matrix A (R x N, R >= N) is factorised A P = Q R by
-// Householder QR with column pivoting, stopped at the first step k whose
-// remaining block has Frobenius norm below delta |R_00|.  One-sided Jacobi
-// then orthogonalises the columns of Z = P R[0:k, :]^H (N x k): the pivoted
-// R is graded, so Z converges in few sweeps, and it has only k columns.
-// With Z V = W orthogonal, A ~= (Q V) Sigma (W / Sigma)^H, so W = A^H U Sigma:
-// the caller receives the conjugate-side factor (N x k, ld N).  The dropped
+// The oriented matrix A (R x N, R >= N) is factorised A P = Q R with column
+// pivoting, stopped at the first step k whose remaining block has Frobenius
+// norm below delta times the largest initial column norm.  One-sided Jacobi
+// then orthogonalises the columns of Z = P R[0:k, :]^H (N x k): the pivoted R
+// is graded, so Z converges in few sweeps, and it has only k columns.  With
+// Z V = W orthogonal, A ~= (Q V) Sigma (W / Sigma)^H, so W = A^H U Sigma: the
+// caller receives the conjugate-side factor (N x k, ld N).  The dropped
 // block's squared norm belongs to the tail of every kept index and is added
 // to the tail sums, so the rank decision is that of the full decomposition up
 // to delta.
 //
-// Arithmetic (template parameter T):
-//   double -- complex128 form: FP64 throughout; delta at the factorisation's
-//             own backward-error level (1e-14 by default);
-//   ff     -- mixed form: double-float (ff.cuh) on the FP32 pipe; delta
-//             min(1e-3 epsrel, 1e-9) by default.
-// Norms, the descending sort, the tail sums and the rank decision are FP64 in
-// both (jacobi_finish).
-//
-// Synchronisation: one __syncthreads per QR column.  No columns are
-// exchanged: column p_i chosen at step i keeps its storage; a short list of
-// the unchosen columns is exchanged instead.  The pivot, the remaining mass
-// and the reflector scalars are computed redundantly by every warp from data
-// no thread writes during the step (partial norms and the column list are
-// double-buffered by step parity; the diagonal R_ii is stored one step late,
-// when no warp reads that column any more).
+// Q itself is never used, so R comes from modified Gram-Schmidt: R is as
+// accurate as the Householder one (backward stable), the projection of a
+// column on the pivot column needs no reflector scalars -- the coefficient
+// conj(p) . x / |p|^2 takes one reciprocal square root, evaluated while the
+// inner products are being formed -- and row i of R is just those inner
+// products.
 #pragma once
+
+#include <climits>
 
 #include "jacobi.cuh"
 
 namespace otb {
 
-template <typename T>
-struct QA;
+constexpr int SPLIT_NMAX = 1152;  // max columns of a split (D * chi_cap <= 1152)
 
-// Householder scalars of a column x (rows i..) with head x0 and squared norm
-// n2: v0 = e (|x0| + |x|), alpha = -e |x| (the new diagonal), beta =
-// 1 / (|x| (|x| + |x0|)) (H = I - beta v v^H), inv = 1 / v0, tau = beta |v0|^2
-// (the unit-diagonal form), e = x0 / |x0| (1 for x0 = 0); a zero column gives
-// H = I.
-template <typename E, typename S>
-struct Refl {
-  E v0, alpha, inv;
-  S beta;
-  double tau;
+// The split's per-column results and, while the QR runs, its bookkeeping.
+struct SplitBook {
+  double norm[SPLIT_NMAX];
+  int perm[SPLIT_NMAX];
 };
 
-template <>
-struct QA<double> {
-  typedef cx<double> E;  // element of the working matrix
-  typedef double S;      // accurate real scalar
-  static constexpr bool kFF = false;
-  static __device__ __forceinline__ E from(cx<double> z) { return z; }
-  static __device__ __forceinline__ cx<double> to(const E& e) { return e; }
-  static __device__ __forceinline__ S zero() { return 0.0; }
-  static __device__ __forceinline__ S fromd(double d) { return d; }
-  static __device__ __forceinline__ double tod(S s) { return s; }
-  static __device__ __forceinline__ S add(S a, S b) { return a + b; }
-  static __device__ __forceinline__ S mul(S a, S b) { return a * b; }
-  static __device__ __forceinline__ S shfl(S v, int off) { return __shfl_xor_sync(0xffffffffu, v, off, 32); }
-  static __device__ __forceinline__ S abs2_acc(const E& x, S acc) { return fma(x.x, x.x, fma(x.y, x.y, acc)); }
-  static __device__ __forceinline__ float abs2f(const E& x) { return (float)fma(x.x, x.x, x.y * x.y); }
-  // (wr, wi) += conj(a) x
-  static __device__ __forceinline__ void dotj(S& wr, S& wi, const E& a, const E& x) {
-    wr = fma(a.x, x.x, fma(a.y, x.y, wr));
-    wi = fma(a.x, x.y, fma(-a.y, x.x, wi));
-  }
-  static __device__ __forceinline__ S fin(S v) { return v; }
-  // x - a (bx + i by)
-  static __device__ __forceinline__ E sub_scaled(const E& x, const E& a, S bx, S by) {
-    return mk<double>(x.x - fma(a.x, bx, -a.y * by), x.y - fma(a.x, by, a.y * bx));
-  }
-  static __device__ __forceinline__ E conj(const E& x) { return mk<double>(x.x, -x.y); }
-  static __device__ __forceinline__ E zeroE() { return mk<double>(0.0, 0.0); }
-  static __device__ __forceinline__ E oneE() { return mk<double>(1.0, 0.0); }
-  static __device__ __forceinline__ E mulc(const E& a, const E& b) { return cmul(a, b); }
-  // FP64: evaluated by one lane of each warp and broadcast (the FP64 pipe is
-  // the narrow one)
-  static constexpr bool kAllLanes = false;
-  static __device__ __forceinline__ Refl<E, S> reflector(S n2, const E& x0) {
-    Refl<E, S> r;
-    const double nrm = sqrt(fmax(n2, 0.0));
-    const double a0 = sqrt(x0.x * x0.x + x0.y * x0.y);
-    const double ex = (a0 > 0.0) ? x0.x / a0 : 1.0, ey = (a0 > 0.0) ? x0.y / a0 : 0.0;
-    const double m = a0 + nrm;
-    r.v0 = mk<double>(ex * m, ey * m);
-    r.alpha = mk<double>(-ex * nrm, -ey * nrm);
-    r.inv = (m > 0.0) ? mk<double>(ex / m, -ey / m) : mk<double>(0.0, 0.0);
-    r.beta = (nrm > 0.0) ? 1.0 / (nrm * m) : 0.0;
-    r.tau = (nrm > 0.0) ? m / nrm : 0.0;
-    return r;
-  }
-  static __device__ __forceinline__ Refl<E, S> bcast(Refl<E, S> r) {
-    r.v0.x = __shfl_sync(0xffffffffu, r.v0.x, 0);
-    r.v0.y = __shfl_sync(0xffffffffu, r.v0.y, 0);
-    r.alpha.x = __shfl_sync(0xffffffffu, r.alpha.x, 0);
-    r.alpha.y = __shfl_sync(0xffffffffu, r.alpha.y, 0);
-    r.inv.x = __shfl_sync(0xffffffffu, r.inv.x, 0);
-    r.inv.y = __shfl_sync(0xffffffffu, r.inv.y, 0);
-    r.beta = __shfl_sync(0xffffffffu, r.beta, 0);
-    r.tau = __shfl_sync(0xffffffffu, r.tau, 0);
-    return r;
-  }
+// QR bookkeeping (36 bytes a column): squared norms of the unchosen columns
+// and their FP32 keys by list position, the list itself (column of every
+// position), all double-buffered by step parity, and the inverse pivot norms.
+struct QrBook {
+  unsigned char* p;
+  int N;
+  template <typename S>
+  __device__ S* n2(int par) const { return reinterpret_cast<S*>(p) + par * N; }
+  template <typename S>
+  __device__ S* rinv() const { return reinterpret_cast<S*>(p) + 2 * N; }
+  __device__ float* key(int par) const { return reinterpret_cast<float*>(p + (size_t)24 * N) + par * N; }
+  __device__ short* list(int par) const { return reinterpret_cast<short*>(p + (size_t)32 * N) + par * N; }
 };
-
-template <>
-struct QA<ff> {
-  typedef cff E;
-  typedef ff S;
-  static constexpr bool kFF = true;
-  static __device__ __forceinline__ E from(cx<double> z) { return cff_from(z); }
-  static __device__ __forceinline__ cx<double> to(const E& e) { return cff_to(e); }
-  static __device__ __forceinline__ S zero() { return ff_make(0.f, 0.f); }
-  static __device__ __forceinline__ S fromd(double d) { return ff_from(d); }
-  static __device__ __forceinline__ double tod(S s) { return ff_to(s); }
-  static __device__ __forceinline__ S add(S a, S b) { return ff_add(a, b); }
-  static __device__ __forceinline__ S mul(S a, S b) { return ff_mul(a, b); }
-  static __device__ __forceinline__ S shfl(S v, int off) { return ff_shfl_xor(v, off); }
-  static __device__ __forceinline__ S abs2_acc(const E& x, S acc) { return ff_fma(x.x, x.x, ff_fma(x.y, x.y, acc)); }
-  static __device__ __forceinline__ float abs2f(const E& x) { return fmaf(x.x.hi, x.x.hi, x.y.hi * x.y.hi); }
-  // wr + i wi += conj(a) x as compensated accumulators (ffp_acc): the
-  // (hi, lo) pair is left unnormalised inside a loop; fin() normalises it
-  static __device__ __forceinline__ void dotj(S& wr, S& wi, const E& a, const E& x) {
-    ffp_acc(a.x.hi, a.x.lo, x.x.hi, x.x.lo, wr.hi, wr.lo);
-    ffp_acc(a.y.hi, a.y.lo, x.y.hi, x.y.lo, wr.hi, wr.lo);
-    ffp_acc(a.x.hi, a.x.lo, x.y.hi, x.y.lo, wi.hi, wi.lo);
-    ffp_acc(-a.y.hi, -a.y.lo, x.x.hi, x.x.lo, wi.hi, wi.lo);
-  }
-  static __device__ __forceinline__ S fin(S v) { return ffacc_norm(v.hi, v.lo); }
-  // x - a (bx + i by), each component one compensated accumulation
-  static __device__ __forceinline__ E sub_scaled(const E& x, const E& a, S bx, S by) {
-    E r;
-    float h = x.x.hi, l = x.x.lo;
-    ffp_acc(-a.x.hi, -a.x.lo, bx.hi, bx.lo, h, l);
-    ffp_acc(a.y.hi, a.y.lo, by.hi, by.lo, h, l);
-    r.x = ffacc_norm(h, l);
-    h = x.y.hi;
-    l = x.y.lo;
-    ffp_acc(-a.x.hi, -a.x.lo, by.hi, by.lo, h, l);
-    ffp_acc(-a.y.hi, -a.y.lo, bx.hi, bx.lo, h, l);
-    r.y = ffacc_norm(h, l);
-    return r;
-  }
-  static __device__ __forceinline__ E conj(const E& x) {
-    E r = x;
-    r.y.hi = -r.y.hi;
-    r.y.lo = -r.y.lo;
-    return r;
-  }
-  static __device__ __forceinline__ E zeroE() {
-    E r;
-    r.x = ff_make(0.f, 0.f);
-    r.y = r.x;
-    return r;
-  }
-  static __device__ __forceinline__ E oneE() {
-    E r;
-    r.x = ff_make(1.f, 0.f);
-    r.y = ff_make(0.f, 0.f);
-    return r;
-  }
-  static __device__ __forceinline__ E mulc(const E& a, const E& b) {
-    E r;
-    r.x = ff_sub(ff_mul(a.x, b.x), ff_mul(a.y, b.y));
-    r.y = ff_add(ff_mul(a.x, b.y), ff_mul(a.y, b.x));
-    return r;
-  }
-  // double-float on the FP32 pipe: evaluated by every lane (n2 and x0 are
-  // the same in all lanes), no FP64 instruction and no broadcast
-  static constexpr bool kAllLanes = true;
-  static __device__ __forceinline__ Refl<E, S> reflector(S n2, const E& x0) {
-    Refl<E, S> r;
-    const ff z = ff_make(0.f, 0.f);
-    const ff nrm = ff_sqrt(n2);
-    const ff a0 = ff_sqrt(ff_fma(x0.x, x0.x, ff_mul(x0.y, x0.y)));
-    ff ex = ff_make(1.f, 0.f), ey = z;
-    if (a0.hi > 0.f) {
-      const ff ia = ff_recip(a0);
-      ex = ff_mul(x0.x, ia);
-      ey = ff_mul(x0.y, ia);
-    }
-    const ff m = ff_add(a0, nrm);
-    r.v0.x = ff_mul(ex, m);
-    r.v0.y = ff_mul(ey, m);
-    r.alpha.x = ff_make(-ff_mul(ex, nrm).hi, -ff_mul(ex, nrm).lo);
-    r.alpha.y = ff_make(-ff_mul(ey, nrm).hi, -ff_mul(ey, nrm).lo);
-    r.inv.x = z;
-    r.inv.y = z;
-    r.beta = z;
-    r.tau = 0.0;
-    if (m.hi > 0.f) {
-      const ff im = ff_recip(m);
-      r.inv.x = ff_mul(ex, im);
-      const ff t = ff_mul(ey, im);
-      r.inv.y = ff_make(-t.hi, -t.lo);
-    }
-    if (nrm.hi > 0.f) {
-      r.beta = ff_recip(ff_mul(nrm, m));
-      r.tau = ff_to(ff_mul(m, ff_recip(nrm)));
-    }
-    return r;
-  }
-  static __device__ __forceinline__ Refl<E, S> bcast(Refl<E, S> r) { return r; }
-};
+__host__ __device__ constexpr size_t qr_book_bytes(int N) { return (size_t)36 * N + 16; }
 
 // Default relative cut of the QR (the remaining block's Frobenius norm over
-// |R_00|) for each arithmetic.
+// the largest initial column norm) for each arithmetic.
 __device__ __forceinline__ float qr_default_delta(bool ffarith, double epsrel) {
   return ffarith ? (float)fmin(1e-3 * epsrel, 1e-9) : 1e-14f;
 }
 
-// Householder QR with column pivoting of X (R x N, column-major ld R), in
-// place, without column exchanges.  Workspace: cn holds 2 N floats (partial
-// squared column norms by column, double-buffered by step parity), lists
-// 2 N shorts (by step parity: positions 0..i-1 the columns chosen at steps
-// 0..i-1, positions i..N-1 the unchosen ones).  Returns k and writes
-// colstep[j] (N ints, in cn's storage, valid after the call) = the step at
-// which column j was chosen, N for never; for i < k, X[j * R + i] = R[i][j]
-// for every column j with colstep[j] >= i (colstep[j] == i: the diagonal of
-// step i).  *tail2 is the remaining squared mass at the stop (0 when all N
-// steps ran).
+// Lanes per column of a QR step, from the operand's shape only (an instance's
+// rounding must not depend on the launch shape or on the batch it is in).  As
+// for the Jacobi pairs, wider groups repeat a column's scalar work in more
+// warps: few lanes while many columns are left, more once they run out.
+__device__ __forceinline__ int qr_group(int rows, int cols) {
+  int G = rows > 160 ? 32 : (rows > 64 ? 16 : 8);
+  while (G < 32 && G * cols <= 96 && rows > 2 * G) G <<= 1;
+  return G;
+}
+
+// About 1 / (|v| |c|) from squared norms; columns below 1e-15 (zero columns
+// among them) count as 1e-15, which only makes the bound a loose one.
+__device__ __forceinline__ float inverse_bound(float v2, float c2) {
+  return rsqrt_est(fmaxf(v2, 1e-30f)) * rsqrt_est(fmaxf(c2, 1e-30f));
+}
+
+// One Gram-Schmidt projection by a group of G lanes (lane gl): (wr, wi) =
+// v^H c, c <- c - v beta (wr + i wi), s2 = |c|^2 (of the new column; all
+// results in every lane).  rb is about 1 / (|v| |c|).  RC rows a lane at a time in registers (all of its
+// rows with ALL: R <= RC G), so that the rows' chains overlap.
+template <typename T, int G, int RC, bool ALL>
+__device__ __forceinline__ void project_rc(const typename QA<T>::E* v, typename QA<T>::E* c, int R, int gl,
+                                           bool act, typename QA<T>::S beta, float rb, typename QA<T>::S& wr,
+                                           typename QA<T>::S& wi, typename QA<T>::S& s2) {
+  typedef QA<T> Q;
+  typedef typename Q::E E;
+  wr = wi = s2 = Q::zero();
+  E a[RC], x[RC];
+  for (int r0 = gl; r0 < (ALL ? gl + 1 : R); r0 += RC * G) {
+#pragma unroll
+    for (int q = 0; q < RC; ++q) {
+      const bool in = act && r0 + q * G < R;
+      a[q] = in ? v[r0 + q * G] : Q::zeroE();
+      x[q] = in ? c[r0 + q * G] : Q::zeroE();
+    }
+#pragma unroll
+    for (int q = 0; q < RC; ++q) Q::dotj(wr, wi, a[q], x[q]);
+  }
+  Q::template dot_sum<G>(wr, wi, rb);
+  const typename Q::S bx = Q::mul(beta, wr), by = Q::mul(beta, wi);
+  for (int r0 = gl; r0 < (ALL ? gl + 1 : R); r0 += RC * G) {
+#pragma unroll
+    for (int q = 0; q < RC; ++q) {
+      if (!ALL) {
+        const bool in = act && r0 + q * G < R;
+        a[q] = in ? v[r0 + q * G] : Q::zeroE();
+        x[q] = in ? c[r0 + q * G] : Q::zeroE();
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < RC; ++q) {
+      x[q] = Q::sub_scaled(x[q], a[q], bx, by);
+      s2 = Q::abs2_acc(x[q], s2);
+    }
+#pragma unroll
+    for (int q = 0; q < RC; ++q)
+      if (act && r0 + q * G < R) c[r0 + q * G] = x[q];
+  }
+  s2 = Q::fin(Q::template group_sum<G>(s2));
+}
+
 template <typename T>
-__device__ int qrcp_inplace(typename QA<T>::E* X, int R, int N, float delta, float* cn, short* lists,
-                            float* tail2) {
+__device__ __forceinline__ void project(const typename QA<T>::E* v, typename QA<T>::E* c, int R, int G, int gl,
+                                        bool act, typename QA<T>::S beta, float rb, typename QA<T>::S& wr,
+                                        typename QA<T>::S& wi, typename QA<T>::S& s2) {
+  if (G == 8) {
+    if (R <= 32)
+      project_rc<T, 8, 4, true>(v, c, R, gl, act, beta, rb, wr, wi, s2);
+    else
+      project_rc<T, 8, 4, false>(v, c, R, gl, act, beta, rb, wr, wi, s2);
+  } else if (G == 16) {
+    if (R <= 32)
+      project_rc<T, 16, 2, true>(v, c, R, gl, act, beta, rb, wr, wi, s2);
+    else if (R <= 64)
+      project_rc<T, 16, 4, true>(v, c, R, gl, act, beta, rb, wr, wi, s2);
+    else
+      project_rc<T, 16, 4, false>(v, c, R, gl, act, beta, rb, wr, wi, s2);
+  } else {
+    if (R <= 64)
+      project_rc<T, 32, 2, true>(v, c, R, gl, act, beta, rb, wr, wi, s2);
+    else
+      project_rc<T, 32, 4, false>(v, c, R, gl, act, beta, rb, wr, wi, s2);
+  }
+}
+
+// Pivoted Gram-Schmidt QR of X (R x N, column-major ld R; destroyed).
+// Returns k and writes Z (N x k, ld N): Z[q, i] = conj(R[i, q]), zero where
+// column q was chosen before step i; Z's storage holds N x N.  *tail2 is the
+// remaining squared mass at the stop (0 when all N steps ran).
+//
+// One __syncthreads per step, no column moves: every warp finds the pivot
+// (largest squared norm, first list position on ties) and the remaining mass
+// from the list's keys; every column's group forms its inner product with the
+// pivot column, updates the column and leaves its new squared norm, key and
+// list entry in the other buffer.  A step is bound by the chain key ->
+// pivot -> inner product -> reduction -> update (and, per CTA, by the
+// double-float or FP64 issue rate while many columns are left).  Against the
+// Householder form it replaces (reflector norm and scalars by every warp,
+// three dependent reductions per step) a step of a 45 x 22 double-float
+// operand takes 5700 instead of 8000 clocks, of a 57 x 26 FP64 one 14000
+// instead of 22000.
+template <typename T>
+__device__ int pivoted_qr(typename QA<T>::E* X, int R, int N, float delta, const QrBook& bk, typename QA<T>::E* Z,
+                          float* tail2) {
   typedef QA<T> Q;
   typedef typename Q::E E;
   typedef typename Q::S S;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane32 = tid & 31, warp = tid >> 5, nw = nt >> 5;
   for (int j = warp; j < N; j += nw) {
-    float acc = 0.f;
+    S acc = Q::zero();
     const E* c = X + (size_t)j * R;
-    for (int r = lane32; r < R; r += 32) acc += Q::abs2f(c[r]);
-    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (lane32 == 0) cn[j] = acc;
+    for (int r = lane32; r < R; r += 32) acc = Q::abs2_acc(c[r], acc);
+    acc = Q::fin(Q::template group_sum<32>(acc));
+    if (lane32 == 0) {
+      bk.n2<S>(0)[j] = acc;
+      bk.key(0)[j] = Q::tof(acc);
+      bk.list(0)[j] = (short)j;
+    }
   }
-  for (int j = tid; j < N; j += nt) lists[j] = (short)j;
+  for (int idx = tid; idx < N * N; idx += nt) Z[idx] = Q::zeroE();
   __syncthreads();
-  float r00 = 0.f, t2 = 0.f;
+  float cut = 0.f, t2 = 0.f;
   int k = N;
-  int pend_p = -1;  // thread 0: column and value of the previous step's diagonal
-  E pend_a = Q::zeroE();
   for (int i = 0; i < N; ++i) {
-    const float* cur = cn + (i & 1) * N;
-    float* nxt = cn + ((i + 1) & 1) * N;
-    const short* Lc = lists + (i & 1) * N;
-    short* Ln = lists + ((i + 1) & 1) * N;
-    // (a) pivot (largest partial norm, lowest list position on ties) and
-    // remaining mass over the unchosen columns, by every warp; the xor
-    // butterfly leaves bitwise-identical results in every lane, and every
-    // warp reduces the same data in the same order
-    float bv = -1.f, sum = 0.f;
-    int bq = N;
-    for (int q = i + lane32; q < N; q += 32) {
-      const float v = cur[Lc[q]];
+    const int n = N - i, cur = i & 1, nxt = cur ^ 1;
+    const float* key = bk.key(cur);
+    const short* list = bk.list(cur);
+    float bv = 0.f, sum = 0.f;
+    int bq = INT_MAX;
+    for (int q = lane32; q < n; q += 32) {
+      const float v = key[q];
       sum += v;
-      if (v > bv) {
+      if (bq == INT_MAX || v > bv) {
         bv = v;
         bq = q;
       }
     }
-    for (int off = 16; off > 0; off >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-      const int oq = __shfl_xor_sync(0xffffffffu, bq, off);
-      if (ov > bv || (ov == bv && oq < bq)) {
-        bv = ov;
-        bq = oq;
-      }
-      sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    }
+    const unsigned best = __reduce_max_sync(0xffffffffu, __float_as_uint(bv));
+    const int pos = (int)__reduce_min_sync(0xffffffffu, __float_as_uint(bv) == best ? (unsigned)bq : (unsigned)INT_MAX);
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
     if (i == 0) {
-      r00 = bv;
-    } else if (sum < delta * delta * r00) {
+      cut = delta * delta * __uint_as_float(best);
+    } else if (sum < cut) {
       k = i;
       t2 = sum;
       break;
     }
-    const int pos = bq;
-    const int p = Lc[pos];
-    // next step's list (the other parity buffer, read by no one in this
-    // step): history through position i, the unchosen columns after it
-    for (int q = i - 1 + tid; q < N; q += nt) {
-      if (q >= 0) Ln[q] = (q == i) ? (short)p : ((q == pos) ? Lc[i] : Lc[q]);
-    }
-    // the previous step's diagonal: its column is read by no one any more
-    if (tid == 0 && pend_p >= 0) X[(size_t)pend_p * R + (i - 1)] = pend_a;
-    // (b) reflector of column p, rows i..R-1 (column p is not written in
-    // this step): H = I - beta v v^H, v = x - alpha e_i, alpha = -e |x|,
-    // v_i = e (|x_i| + |x|), beta = 1 / (|x| (|x| + |x_i|)), e = x_i / |x_i|
-    const E* v = X + (size_t)p * R;
-    S n2 = Q::zero();
-    for (int r = i + lane32; r < R; r += 32) n2 = Q::abs2_acc(v[r], n2);
-    for (int off = 16; off > 0; off >>= 1) n2 = Q::add(n2, Q::shfl(n2, off));
-    Refl<E, S> rf;
-    if (Q::kAllLanes || lane32 == 0) rf = Q::reflector(n2, v[i]);
-    rf = Q::bcast(rf);
+    const int p = list[pos];
+    const S np = bk.n2<S>(cur)[pos];
+    const S ri = Q::rsqrt(np);
+    const S beta = Q::mul(ri, ri);
     if (tid == 0) {
-      pend_p = p;
-      pend_a = rf.alpha;
+      bk.rinv<S>()[i] = ri;
+      Z[(size_t)i * N + p] = Q::realE(np);
     }
-    const E v0 = rf.v0;
-    const S beta = rf.beta;
-    // (c) apply H to the other unchosen columns (list positions i..N-1 but
-    // pos), refresh their partial norms (rows > i) in the other buffer
-    const int G = jacobi_group(R - i);
+    const E* v = X + (size_t)p * R;
+    const int nrest = n - 1;
+    const int G = qr_group(R, nrest);
     const int gl = tid & (G - 1), group = tid / G, ngroups = nt / G;
-    const int nrest = N - i - 1;
     for (int tb = 0; tb < nrest; tb += ngroups) {
+      if (tb + (warp * 32) / G >= nrest) break;   // no column left for this warp
       const int t = tb + group;
       const bool act = t < nrest;
-      const int q = i + t + ((i + t >= pos) ? 1 : 0);
-      const int j = act ? Lc[q] : p;
+      const int q = act ? t + (t >= pos ? 1 : 0) : pos;
+      const int j = list[q];
+      const float rb = inverse_bound(__uint_as_float(best), key[q]);
       E* cj = X + (size_t)j * R;
-      S wr = Q::zero(), wi = Q::zero();
-      if (act) {
-        for (int r = i + gl; r < R; r += G) Q::dotj(wr, wi, (r == i) ? v0 : v[r], cj[r]);
+      S wr, wi, s2;
+      project<T>(v, cj, R, G, gl, act, beta, rb, wr, wi, s2);
+      if (act && gl == 0) {
+        bk.n2<S>(nxt)[t] = s2;
+        bk.key(nxt)[t] = Q::tof(s2);
+        bk.list(nxt)[t] = (short)j;
+        E z;
+        z.x = wr;
+        z.y = wi;
+        Z[(size_t)i * N + j] = z;
       }
-      wr = Q::fin(wr);
-      wi = Q::fin(wi);
-      for (int off = G >> 1; off > 0; off >>= 1) {
-        wr = Q::add(wr, Q::shfl(wr, off));
-        wi = Q::add(wi, Q::shfl(wi, off));
-      }
-      float s2 = 0.f;
-      if (act) {
-        const S bx = Q::mul(beta, wr), by = Q::mul(beta, wi);
-        for (int r = i + gl; r < R; r += G) {
-          const E x = Q::sub_scaled(cj[r], (r == i) ? v0 : v[r], bx, by);
-          cj[r] = x;
-          if (r > i) s2 += Q::abs2f(x);
-        }
-      }
-      for (int off = G >> 1; off > 0; off >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, off, 32);
-      if (act && gl == 0) nxt[j] = s2;
     }
     __syncthreads();
   }
-  if (tid == 0 && pend_p >= 0) X[(size_t)pend_p * R + (k - 1)] = pend_a;
-  // a stop at step k leaves warps that may still be reading cn in that
-  // step's pivot search
-  __syncthreads();
-  // colstep from the final list (buffer k & 1), over cn's storage
-  const short* L = lists + (k & 1) * N;
-  int* colstep = reinterpret_cast<int*>(cn);
-  for (int q = tid; q < N; q += nt) colstep[L[q]] = (q < k) ? q : N;
+  __syncthreads();   // a stop at step k leaves warps that may still be reading the keys
+  // rows of R: conj(inner products) over the pivot norms
+  for (int idx = tid; idx < N * k; idx += nt) Z[idx] = Q::conj_scale(Z[idx], bk.rinv<S>()[idx / N]);
   __syncthreads();
   *tail2 = t2;
   return k;
 }
 
-// Unpivoted Householder QR of Z (M x K, M >= K, column-major ld), in place,
-// one __syncthreads per column: on return the upper triangle of Z[0:K, :]
-// holds R, below the diagonal column i holds its reflector w_i scaled to
-// w_i[i] = 1 (implicit), and tau[i] (FP64) makes H_i = I - tau_i w_i w_i^H,
-// Z = H_0 H_1 ... H_{K-1} [R; 0].  The reflector scalars are computed by
-// every warp from column i, which no thread writes during step i; column
-// i's scaling and diagonal are written in step i + 1, when no warp reads it.
+// Unpivoted Gram-Schmidt QR of Z (M x K, M >= K, column-major ld M), in place:
+// on return column i of Z is 1 / rinv[i] times the i-th column of Q and R2
+// (K x K, ld K) holds R.  Like pivoted_qr without the search.  Q is not used
+// as an orthogonal matrix: Z V = Q (R2 V) holds to rounding whatever its
+// orthogonality, and R2 is backward stable.
 template <typename T>
-__device__ void householder_unit(typename QA<T>::E* Z, int M, int K, int ld, double* tau) {
+__device__ void plain_qr(typename QA<T>::E* Z, int M, int K, typename QA<T>::E* R2, typename QA<T>::S* rinv,
+                         typename QA<T>::S* n2) {
   typedef QA<T> Q;
   typedef typename Q::E E;
   typedef typename Q::S S;
   const int tid = threadIdx.x, nt = blockDim.x, lane32 = tid & 31;
-  E pinv = Q::zeroE(), palpha = Q::zeroE();   // previous column's 1 / v_i and diagonal
+  for (int j = tid >> 5; j < K; j += nt >> 5) {
+    S acc = Q::zero();
+    for (int r = lane32; r < M; r += 32) acc = Q::abs2_acc(Z[(size_t)j * M + r], acc);
+    acc = Q::fin(Q::template group_sum<32>(acc));
+    if (lane32 == 0) n2[j] = acc;
+  }
+  for (int idx = tid; idx < K * K; idx += nt) R2[idx] = Q::zeroE();
+  __syncthreads();
   for (int i = 0; i < K; ++i) {
-    if (i > 0) {
-      E* c = Z + (size_t)(i - 1) * ld;
-      for (int r = i + tid; r < M; r += nt) c[r] = Q::mulc(c[r], pinv);
-      if (tid == 0) c[i - 1] = palpha;
+    const S np = n2[i];
+    const S ri = Q::rsqrt(np);
+    const S beta = Q::mul(ri, ri);
+    if (tid == 0) {
+      rinv[i] = ri;
+      R2[(size_t)i * K + i] = Q::realE(np);
     }
-    const E* v = Z + (size_t)i * ld;
-    S n2 = Q::zero();
-    for (int r = i + lane32; r < M; r += 32) n2 = Q::abs2_acc(v[r], n2);
-    for (int off = 16; off > 0; off >>= 1) n2 = Q::add(n2, Q::shfl(n2, off));
-    Refl<E, S> rf;
-    if (Q::kAllLanes || lane32 == 0) rf = Q::reflector(n2, v[i]);
-    rf = Q::bcast(rf);
-    if (tid == 0) tau[i] = rf.tau;
-    pinv = rf.inv;
-    palpha = rf.alpha;
-    const E v0 = rf.v0;
-    const S beta = rf.beta;
-    const int G = jacobi_group(M - i);
-    const int gl = tid & (G - 1), group = tid / G, ngroups = nt / G;
+    const E* v = Z + (size_t)i * M;
     const int nrest = K - i - 1;
+    const int G = qr_group(M, nrest);
+    const int gl = tid & (G - 1), group = tid / G, ngroups = nt / G;
     for (int tb = 0; tb < nrest; tb += ngroups) {
+      if (tb + (tid >> 5) * 32 / G >= nrest) break;
       const int t = tb + group;
       const bool act = t < nrest;
-      E* cj = Z + (size_t)(act ? i + 1 + t : i) * ld;
-      S wr = Q::zero(), wi = Q::zero();
-      if (act) {
-        for (int r = i + gl; r < M; r += G) Q::dotj(wr, wi, (r == i) ? v0 : v[r], cj[r]);
-      }
-      wr = Q::fin(wr);
-      wi = Q::fin(wi);
-      for (int off = G >> 1; off > 0; off >>= 1) {
-        wr = Q::add(wr, Q::shfl(wr, off));
-        wi = Q::add(wi, Q::shfl(wi, off));
-      }
-      if (act) {
-        const S bx = Q::mul(beta, wr), by = Q::mul(beta, wi);
-        for (int r = i + gl; r < M; r += G) cj[r] = Q::sub_scaled(cj[r], (r == i) ? v0 : v[r], bx, by);
+      E* cj = Z + (size_t)(act ? i + 1 + t : i) * M;
+      S wr, wi, s2;
+      const int j = act ? i + 1 + t : i;
+      const float rb = inverse_bound(Q::tof(np), Q::tof(n2[j]));
+      project<T>(v, cj, M, G, gl, act, beta, rb, wr, wi, s2);
+      if (act && gl == 0) n2[j] = s2;
+      if (act && gl == 0) {
+        E z;
+        z.x = wr;
+        z.y = wi;
+        R2[(size_t)(i + 1 + t) * K + i] = z;
       }
     }
     __syncthreads();
   }
-  if (K > 0) {
-    E* c = Z + (size_t)(K - 1) * ld;
-    for (int r = K + tid; r < M; r += nt) c[r] = Q::mulc(c[r], pinv);
-    if (tid == 0) c[K - 1] = palpha;
-  }
+  for (int idx = tid; idx < K * K; idx += nt) R2[idx] = Q::scaleE(R2[idx], rinv[idx % K]);
   __syncthreads();
 }
 
-// Y <- Q Y for the first ncols columns of Y (M x ncols, ld ldy), Q = H_0 ...
-// H_{K-1} as stored by householder_unit: reflectors applied last-first, one
-// __syncthreads each.
+// Sweeps, with an FP64 finish for a double-float matrix whose double-float
+// sweeps did not settle (converted in place -- both elements are 16 bytes --
+// swept, converted back).  Leaves the FP64 column norms times `scale` in
+// norm[] and the sweep counts in sh; returns the FP64 sweeps.
 template <typename T>
-__device__ void apply_q_unit(const typename QA<T>::E* Z, int M, int K, int ld, const double* tau,
-                             typename QA<T>::E* Y, int ncols, int ldy) {
+__device__ int jacobi_norms(typename QA<T>::E* W, int m, int n, int ld, double scale, double* norm, JacobiShared* sh) {
+  typedef QA<T> Q;
+  typedef typename Q::S S;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  int sw = jacobi_sweeps<T>(W, m, n, ld, reinterpret_cast<S*>(norm), sh);
+  int sw64 = Q::kFF ? 0 : sw;
+  bool settled = sw < JACOBI_MAX_SWEEPS;
+  if (Q::kFF && !(settled || sh->noise_converged)) {
+    cx<double>* Wd = reinterpret_cast<cx<double>*>(W);
+    for (int j = 0; j < n; ++j)
+      for (int r = tid; r < m; r += nt) Wd[(size_t)j * ld + r] = Q::to(W[(size_t)j * ld + r]);
+    __syncthreads();
+    sw64 = jacobi_sweeps<double>(Wd, m, n, ld, norm, sh);
+    for (int j = 0; j < n; ++j)
+      for (int r = tid; r < m; r += nt) W[(size_t)j * ld + r] = Q::from(Wd[(size_t)j * ld + r]);
+    __syncthreads();
+    settled = false;
+  }
+  if (!settled) {   // the sweeps' squared norms are not those of the result
+    const int lane32 = tid & 31;
+    for (int j = tid >> 5; j < n; j += nt >> 5) {
+      S acc = Q::zero();
+      for (int r = lane32; r < m; r += 32) acc = Q::abs2_acc(W[(size_t)j * ld + r], acc);
+      acc = Q::fin(Q::template group_sum<32>(acc));
+      if (lane32 == 0) reinterpret_cast<S*>(norm)[j] = acc;
+    }
+    __syncthreads();
+  }
+  for (int j = tid; j < n; j += nt) {
+    const double n2 = Q::tod(reinterpret_cast<S*>(norm)[j]);
+    norm[j] = n2 < 0.0 ? 0.0 : scale * sqrt(n2);   // NaN stays NaN
+  }
+  if (tid == 0) sh->sweeps32 = Q::kFF ? sw : 0;
+  __syncthreads();
+  return sw64;
+}
+
+// The split driver on X (R x N, ld R, the oriented matrix over `scale`, a
+// power of two; destroyed), with Zg (R x N elements) as spare global storage,
+// zs / zs_bytes spare shared memory and bkg spare global bookkeeping of
+// qr_book_bytes(N).  x_shared says whether X itself is in shared memory.
+// delta <= 0 selects the default cut.  Returns the kept rank; *Wout holds
+// V_A Sigma (in the units of A / scale; N x k, ld N) with book->norm (in the
+// units of A) / book->perm describing its columns in descending order.
+template <typename T>
+__device__ int qr_jacobi_truncate(typename QA<T>::E* X, bool x_shared, int R, int N, double scale,
+                                  typename QA<T>::E* Zg, unsigned char* zs, size_t zs_bytes, unsigned char* bkg,
+                                  double epsrel, float delta, SplitBook* book, JacobiShared* sh,
+                                  typename QA<T>::E** Wout) {
   typedef QA<T> Q;
   typedef typename Q::E E;
   typedef typename Q::S S;
   const int tid = threadIdx.x, nt = blockDim.x;
-  const E one = Q::oneE();
-  for (int i = K - 1; i >= 0; --i) {
-    const E* w = Z + (size_t)i * ld;
-    const S ti = Q::fromd(tau[i]);
-    const int G = jacobi_group(M - i);
-    const int gl = tid & (G - 1), group = tid / G, ngroups = nt / G;
-    for (int jb = 0; jb < ncols; jb += ngroups) {
-      const int j = jb + group;
-      const bool act = j < ncols;
-      E* y = Y + (size_t)(act ? j : 0) * ldy;
-      S sr = Q::zero(), si = Q::zero();
-      if (act) {
-        for (int r = i + gl; r < M; r += G) Q::dotj(sr, si, (r == i) ? one : w[r], y[r]);
-      }
-      sr = Q::fin(sr);
-      si = Q::fin(si);
-      for (int off = G >> 1; off > 0; off >>= 1) {
-        sr = Q::add(sr, Q::shfl(sr, off));
-        si = Q::add(si, Q::shfl(si, off));
-      }
-      if (act) {
-        const S bx = Q::mul(ti, sr), by = Q::mul(ti, si);
-        for (int r = i + gl; r < M; r += G) y[r] = Q::sub_scaled(y[r], (r == i) ? one : w[r], bx, by);
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// The split driver.  W (R x N, FP64, ld R) holds the oriented matrix and is
-// scratch afterwards; X (R x N elements of QA<T>::E) is the QR workspace; zs /
-// zs_bytes is spare shared memory for the Jacobi operand.  delta <= 0 selects
-// the default cut.  Returns the kept rank; *Wout (FP64, N x k, ld N, in X's
-// storage) holds V_A Sigma with norm / perm describing its columns as in
-// jacobi_finish.
-template <typename T>
-__device__ int qr_jacobi_truncate(cx<double>* W, int R, int N, typename QA<T>::E* X, unsigned char* zs,
-                                  size_t zs_bytes, double epsrel, float delta, double* norm, int* perm,
-                                  JacobiShared* sh, cx<double>** Wout) {
-  typedef QA<T> Q;
-  typedef typename Q::E E;
-  constexpr bool FF = Q::kFF;
-  const int tid = threadIdx.x;
-  const int nt = blockDim.x;
-  // scale by a power of two so that the largest entry is of order one (exact
-  // in FP64; keeps the double-float exponents in range)
-  double mx = 0.0;
-  for (int idx = tid; idx < R * N; idx += nt) mx = fmax(mx, fmax(fabs(W[idx].x), fabs(W[idx].y)));
-  for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  if ((tid & 31) == 0) sh->red[tid >> 5] = mx;
-  __syncthreads();
-  if (tid == 0) {
-    double v = 0.0;
-    for (int w = 0; w < nt / 32; ++w) v = fmax(v, sh->red[w]);
-    sh->red[32] = (v > 0.0 && isfinite(v)) ? ldexp(1.0, ilogb(v)) : 1.0;
-  }
-  __syncthreads();
-  const double scale = sh->red[32];
-  const double inv = 1.0 / scale;
-  for (int idx = tid; idx < R * N; idx += nt) X[idx] = Q::from(cscale(W[idx], inv));
-  __syncthreads();
-  // QR bookkeeping in the (not yet used) norm / perm arrays: partial norms
-  // (2 N floats) then colstep (N ints) in norm[], column lists (2 N shorts)
-  // in perm[]
-  float* cn = reinterpret_cast<float*>(norm);
-  if (!(delta > 0.f)) delta = qr_default_delta(FF, epsrel);
-  float tail2;
-  const int k = qrcp_inplace<T>(X, R, N, delta, cn, reinterpret_cast<short*>(perm), &tail2);
-  const int* colstep = reinterpret_cast<const int*>(norm);
-  // Z = P R[0:k, :]^H: row q (original column q of A), column i
-  E* Z = ((size_t)N * k * sizeof(E) <= zs_bytes) ? reinterpret_cast<E*>(zs) : reinterpret_cast<E*>(W);
-  for (int idx = tid; idx < N * k; idx += nt) {
-    const int i = idx / N, q = idx - i * N;
-    Z[idx] = (colstep[q] >= i) ? Q::conj(X[(size_t)q * R + i]) : Q::zeroE();
-  }
-  __syncthreads();
-  int sw, sw64 = 0;
-  bool done;
-  cx<double>* O = reinterpret_cast<cx<double>*>(X);
-  if (k >= 8 && 2 * k <= N) {
-    // Second (unpivoted) QR, Z = Q2 [R2; 0]: the Jacobi runs on the k x k R2
-    // instead of the N rows of Z, the rank is decided from R2's singular
-    // values (those of Z), and W = Q2 [W2; 0] is formed for the kept columns
-    // only, in sorted order.  X's storage: [0, N kk) the kept columns,
-    // [N k, N k + k^2) R2, then tau (k doubles): N k + k^2 + k <= R N for
-    // 2 k <= N <= R.
-    E* R2 = X + (size_t)N * k;
-    double* tau = reinterpret_cast<double*>(X + (size_t)N * k + (size_t)k * k);
-    householder_unit<T>(Z, N, k, N, tau);
-    for (int idx = tid; idx < k * k; idx += nt) {
-      const int c = idx / k, r = idx - c * k;
-      R2[idx] = (r <= c) ? Z[(size_t)c * N + r] : Q::zeroE();
-    }
-    __syncthreads();
-    cx<double>* R2d = reinterpret_cast<cx<double>*>(R2);
-    if (FF) {
-      sw = jacobi_sweeps_ff(reinterpret_cast<cff*>(R2), k, k, k, sh);
-      done = sw < JACOBI_MAX_SWEEPS || sh->noise_converged;
-      for (int idx = tid; idx < k * k; idx += nt) R2d[idx] = cscale(Q::to(R2[idx]), scale);
-      __syncthreads();
-      if (!done) sw64 = jacobi_sweeps<double>(R2d, k, k, k, nullptr, 0, sh);
+  if (!(delta > 0.f)) delta = qr_default_delta(Q::kFF, epsrel);
+  double* norm = book->norm;
+  int* perm = book->perm;
+  QrBook bk;
+  bk.N = N;
+  bk.p = reinterpret_cast<unsigned char*>(book);
+  if (qr_book_bytes(N) > sizeof(SplitBook)) {   // more than 383 columns
+    if (qr_book_bytes(N) <= zs_bytes) {
+      bk.p = zs;
+      zs += (qr_book_bytes(N) + 15) & ~(size_t)15;
+      zs_bytes -= (qr_book_bytes(N) + 15) & ~(size_t)15;
     } else {
-      sw64 = jacobi_sweeps<double>(R2d, k, k, k, nullptr, 0, sh);
-      sw = 0;
-      for (int idx = tid; idx < k * k; idx += nt) R2d[idx] = cscale(R2d[idx], scale);
+      bk.p = bkg;
+    }
+  }
+  // (the inverse pivot norms at bytes 16 N .. 24 N outlive the sweeps, which
+  // use norm[0, k), and the ranking, which uses perm)
+  // Z in shared memory when all N columns fit; the kept k may fit later
+  E* Z = ((size_t)N * N * sizeof(E) <= zs_bytes) ? reinterpret_cast<E*>(zs) : Zg;
+  float tail2;
+  const int k = pivoted_qr<T>(X, R, N, delta, bk, Z, &tail2);
+  const double t2 = (double)tail2 * scale * scale;
+  const bool second = k >= 8 && 2 * k <= N;
+  if (Z == Zg) {
+    E* to = (size_t)N * k * sizeof(E) <= zs_bytes ? reinterpret_cast<E*>(zs) : (x_shared && !second ? X : Zg);
+    if (to != Z) {
+      for (int idx = tid; idx < N * k; idx += nt) to[idx] = Z[idx];
+      Z = to;
       __syncthreads();
     }
-    if (tid == 0) sh->sweeps32 = sw;
-    const int kk = jacobi_finish<double>(R2d, k, k, k, epsrel, norm, perm, sh, sw64,
-                                         (double)tail2 * scale * scale);
-    if (tid == 0) sh->sweeps = sw64;
-    E* Y = X;
-    for (int idx = tid; idx < N * kk; idx += nt) {
-      const int j = idx / N, r = idx - j * N;
-      Y[idx] = (r < k) ? Q::from(cscale(R2d[(size_t)perm[j] * k + r], inv)) : Q::zeroE();
-    }
-    __syncthreads();
-    apply_q_unit<T>(Z, N, k, N, tau, Y, kk, N);
-    for (int idx = tid; idx < N * kk; idx += nt) O[idx] = cscale(Q::to(Y[idx]), scale);
-    // the kept columns are stored sorted: norms in that order, identity perm
-    for (int j = tid; j < kk; j += nt) tau[j] = norm[perm[j]];
-    __syncthreads();
-    for (int j = tid; j < kk; j += nt) {
-      norm[j] = tau[j];
-      perm[j] = j;
-    }
-    __syncthreads();
-    *Wout = O;
-    return kk;
   }
-  if (FF) {
-    sw = jacobi_sweeps_ff(reinterpret_cast<cff*>(Z), N, k, N, sh);
-    done = sw < JACOBI_MAX_SWEEPS || sh->noise_converged;
-    for (int idx = tid; idx < N * k; idx += nt) O[idx] = cscale(Q::to(Z[idx]), scale);
-    __syncthreads();
-    // FP64 fallback: if the double-float sweeps did not settle, finish the
-    // (nearly orthogonal) matrix with FP64 sweeps; their count is reported
-    if (!done) {
-      sw64 = jacobi_sweeps<double>(O, N, k, N, nullptr, 0, sh);
-      done = true;
-    }
-  } else {
-    sw64 = jacobi_sweeps<double>(reinterpret_cast<cx<double>*>(Z), N, k, N, nullptr, 0, sh);
-    sw = 0;
-    for (int idx = tid; idx < N * k; idx += nt) O[idx] = cscale(Q::to(Z[idx]), scale);
-    __syncthreads();
-  }
-  if (tid == 0) sh->sweeps32 = sw;
-  const int kk = jacobi_finish<double>(O, N, k, N, epsrel, norm, perm, sh, sw64, (double)tail2 * scale * scale);
-  if (tid == 0) sh->sweeps = sw64;
-  __syncthreads();
-  *Wout = O;
-  return kk;
-}
-
-// ---------------------------------------------------------------------------
-// Double-float input and output (the mixed form's TEMPO step keeps sites,
-// carries and theta in double-float): no FP64 instruction per matrix element.
-// ---------------------------------------------------------------------------
-
-// x * 2^e for a double-float complex x: exact (two float multiplications by
-// a power of two) unless it leaves the float range.
-__device__ __forceinline__ cff cff_ldexp(cff x, float p2) {
-  x.x.hi *= p2;
-  x.x.lo *= p2;
-  x.y.hi *= p2;
-  x.y.lo *= p2;
-  return x;
-}
-
-// FP64 norms of the n columns of W (m rows, ld), accumulated in double-float.
-__device__ inline void cff_column_norms(const cff* W, int m, int n, int ld, double* norm) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int j = tid / 32; j < n; j += nt / 32) {
-    const int l = tid & 31;
-    ff acc = ff_make(0.f, 0.f);
-    const cff* c = W + (size_t)j * ld;
-    for (int r = l; r < m; r += 32) acc = ff_fma(c[r].x, c[r].x, ff_fma(c[r].y, c[r].y, acc));
-    for (int off = 16; off > 0; off >>= 1) acc = ff_add(acc, ff_shfl_xor(acc, off));
-    if (l == 0) norm[j] = ff_to(ff_sqrt(acc));
-  }
-  __syncthreads();
-}
-
-// FP64 sweeps on a double-float matrix whose double-float sweeps did not
-// settle: converted in place (both 16-byte elements), swept, converted back.
-__device__ inline int cff_fp64_fallback(cff* W, int m, int n, int ld, JacobiShared* sh) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  cx<double>* Wd = reinterpret_cast<cx<double>*>(W);
-  for (int j = 0; j < n; ++j)
-    for (int r = tid; r < m; r += nt) {
-      const size_t q = (size_t)j * ld + r;
-      Wd[q] = cff_to(W[q]);
-    }
-  __syncthreads();
-  const int sw = jacobi_sweeps<double>(Wd, m, n, ld, nullptr, 0, sh);
-  for (int j = 0; j < n; ++j)
-    for (int r = tid; r < m; r += nt) {
-      const size_t q = (size_t)j * ld + r;
-      W[q] = cff_from(Wd[q]);
-    }
-  __syncthreads();
-  return sw;
-}
-
-// The split driver on a double-float input already in X (R x N, ld R,
-// scaled by 1 / scale, a power of two), with Zbuf (R x N) as spare global
-// storage and zs / zs_bytes spare shared memory.  Returns the kept rank;
-// *Wout (double-float, N x kk or N x k, ld N, in original units) holds
-// V_A Sigma with norm / perm as in jacobi_finish (the k <= N / 2 branch
-// stores its kept columns sorted, perm the identity).
-__device__ inline int qr_jacobi_truncate_ff(cff* X, int R, int N, double scale, cff* Zbuf, unsigned char* zs,
-                                            size_t zs_bytes, double epsrel, float delta, double* norm,
-                                            int* perm, JacobiShared* sh, cff** Wout) {
-  typedef QA<ff> Q;
-  const int tid = threadIdx.x;
-  const int nt = blockDim.x;
-  const float up = (float)scale;    // power of two in float range for the data this path sees
-  float* cn = reinterpret_cast<float*>(norm);
-  if (!(delta > 0.f)) delta = qr_default_delta(true, epsrel);
-  float tail2;
-  const int k = qrcp_inplace<ff>(X, R, N, delta, cn, reinterpret_cast<short*>(perm), &tail2);
-  const int* colstep = reinterpret_cast<const int*>(norm);
-  cff* Z = ((size_t)N * k * sizeof(cff) <= zs_bytes) ? reinterpret_cast<cff*>(zs) : Zbuf;
-  for (int idx = tid; idx < N * k; idx += nt) {
-    const int i = idx / N, q = idx - i * N;
-    Z[idx] = (colstep[q] >= i) ? Q::conj(X[(size_t)q * R + i]) : Q::zeroE();
-  }
-  __syncthreads();
-  const double t2 = (double)tail2 * scale * scale;
-  if (k >= 8 && 2 * k <= N) {
-    // second QR, Jacobi on the k x k R2, kept columns transformed back
-    // (as in qr_jacobi_truncate)
-    cff* R2 = X + (size_t)N * k;
-    double* tau = reinterpret_cast<double*>(X + (size_t)N * k + (size_t)k * k);
-    householder_unit<ff>(Z, N, k, N, tau);
-    for (int idx = tid; idx < k * k; idx += nt) {
-      const int c = idx / k, r = idx - c * k;
-      R2[idx] = (r <= c) ? Z[(size_t)c * N + r] : Q::zeroE();
-    }
-    __syncthreads();
-    const int sw = jacobi_sweeps_ff(R2, k, k, k, sh);
-    int sw64 = 0;
-    if (!(sw < JACOBI_MAX_SWEEPS || sh->noise_converged)) sw64 = cff_fp64_fallback(R2, k, k, k, sh);
-    if (tid == 0) sh->sweeps32 = sw;
-    cff_column_norms(R2, k, k, k, norm);
-    for (int j = tid; j < k; j += nt) norm[j] *= scale;
-    __syncthreads();
+  if (second) {
+    // Second QR, Z = Q2 R2: the Jacobi runs on the k x k R2 instead of the N
+    // rows of Z (same singular values), and W = Q2 (R2 V) is formed for the
+    // kept columns only, in sorted order.  X's storage: R2 and, behind it,
+    // the kept columns: k^2 + N k <= R N for 2 k <= N <= R.
+    E* R2 = X;
+    E* Y = X + (size_t)k * k;
+    S* rinv = bk.rinv<S>();
+    plain_qr<T>(Z, N, k, R2, rinv, bk.n2<S>(0));
+    const int sw64 = jacobi_norms<T>(R2, k, k, k, scale, norm, sh);
     const int kk = jacobi_rank(k, epsrel, norm, perm, sh, sw64, t2);
-    if (tid == 0) sh->sweeps = sw64;
-    cff* Y = X;
-    for (int idx = tid; idx < N * kk; idx += nt) {
-      const int j = idx / N, r = idx - j * N;
-      Y[idx] = (r < k) ? R2[(size_t)perm[j] * k + r] : Q::zeroE();
+    for (int idx = tid; idx < k * kk; idx += nt) {
+      const int j = idx / k, i = idx - j * k;
+      E* e = R2 + (size_t)perm[j] * k + i;
+      *e = Q::scaleE(*e, rinv[i]);
     }
     __syncthreads();
-    apply_q_unit<ff>(Z, N, k, N, tau, Y, kk, N);
-    for (int idx = tid; idx < N * kk; idx += nt) Y[idx] = cff_ldexp(Y[idx], up);
-    for (int j = tid; j < kk; j += nt) tau[j] = norm[perm[j]];
+    for (int idx = tid; idx < N * kk; idx += nt) {
+      const int j = idx / N, r = idx - j * N;
+      const E* y = R2 + (size_t)perm[j] * k;
+      typename Q::Acc acc = Q::acc_zero();
+      for (int i = 0; i < k; ++i) Q::acc_fma(acc, Z[(size_t)i * N + r], y[i]);
+      Y[idx] = Q::acc_value(acc);
+    }
+    // the kept columns are stored sorted: norms in that order, identity perm
+    for (int j = tid; j < kk; j += nt) norm[k + j] = norm[perm[j]];   // 2 k <= N
     __syncthreads();
     for (int j = tid; j < kk; j += nt) {
-      norm[j] = tau[j];
+      norm[j] = norm[k + j];
       perm[j] = j;
     }
     __syncthreads();
     *Wout = Y;
     return kk;
   }
-  const int sw = jacobi_sweeps_ff(Z, N, k, N, sh);
-  int sw64 = 0;
-  if (!(sw < JACOBI_MAX_SWEEPS || sh->noise_converged)) sw64 = cff_fp64_fallback(Z, N, k, N, sh);
-  if (tid == 0) sh->sweeps32 = sw;
-  cff_column_norms(Z, N, k, N, norm);
-  for (int j = tid; j < k; j += nt) norm[j] *= scale;
-  __syncthreads();
+  const int sw64 = jacobi_norms<T>(Z, N, k, N, scale, norm, sh);
   const int kk = jacobi_rank(k, epsrel, norm, perm, sh, sw64, t2);
-  if (tid == 0) sh->sweeps = sw64;
-  for (int idx = tid; idx < N * k; idx += nt) Z[idx] = cff_ldexp(Z[idx], up);
-  __syncthreads();
   *Wout = Z;
   return kk;
 }

@@ -1,13 +1,11 @@
-// Generic truncated bond split for one CTA, used by the PT-TEMPO build.
+// Truncated bond split of one CTA, shared by the TEMPO step and the PT-TEMPO
+// build.
 //
-// X is an m x n complex128 matrix read through an accessor X(row, col).  The
-// split orients itself so that the Jacobi columns are the smaller side, runs
-// the QR-preconditioned Jacobi (qr.cuh; plain Jacobi, jacobi.cuh, below 8
-// columns) in FP64 or double-float, and returns
-//   U  (m x kk, column-major, in Tg)      left singular vectors,
-//   C  (kk x n, row-major, in Cg)         S V^H (the carry),
-// with kk the kept rank of the relative tail rule.  The caller copies U to its
-// destination after the call (U never aliases X, so X may be the destination).
+// oriented_split() reads the oriented matrix A (R x N, R >= N) through an
+// accessor -- key(r, c): magnitude key, exponent(key): its power of two,
+// load(X, R, N, e): X = A 2^-e in the split's arithmetic -- and runs the
+// QR-preconditioned Jacobi (qr.cuh; plain Jacobi, jacobi.cuh, below 8
+// columns).
 #pragma once
 
 #include "qr.cuh"
@@ -16,112 +14,107 @@ namespace otb {
 
 typedef cx<double> zc;
 
-constexpr int SPLIT_NMAX = 1152;  // max Jacobi columns (D * cap <= 9 * 128)
+constexpr int QR_MIN_COLS = 8;
 
+// The splits' arithmetic of a precision form.
+template <bool MIXED>
+struct StepType {
+  typedef double T;
+};
+template <>
+struct StepType<true> {
+  typedef ff T;
+};
+
+struct SplitShared {
+  SplitBook book;
+  JacobiShared jsh;
+  unsigned mag[32];   // largest magnitudes by warp
+};
+
+// Per-CTA working storage: global matrices of wcap 16-byte elements and the
+// dynamic shared memory.
 struct SplitBufs {
-  zc* Wg;      // global working matrix
-  zc* Tg;      // global U output / temporaries
-  zc* Cg;      // carry
-  cff* Wffg;   // global double-float matrix (mixed form)
+  void* Wg;             // spare matrix (the QR's row factor when it does not fit in shared memory)
+  void* Xg;             // working matrix when it does not fit in shared memory
+  unsigned char* bkg;   // QR bookkeeping of more than 383 columns when shared memory is too small
   unsigned char* smem;
   int smem_bytes;
 };
 
-struct SplitShared {
-  JacobiShared jsh;
-  double norm[SPLIT_NMAX];
-  int perm[SPLIT_NMAX];
+// Result of oriented_split: W's columns book.perm[0 .. kk) are, with sigma =
+// book.norm[...] and all of W over `scale`,
+//   flip false: A V Sigma (R x N, ld R);   flip true: A^H U Sigma (N x k, ld N)
+// for the oriented A (R x N).
+template <typename T>
+struct SplitOut {
+  typename QA<T>::E* W;
+  int kk;
+  int e;       // scale = 2^e
+  bool flip;
 };
 
-// Returns kk (>= 1); on failure sets *status (nonzero) and returns 0.
-template <bool MIXED, class Acc>
-__device__ int split_generic(const Acc& X, int m, int n, double epsrel, float qr_delta, int cap, SplitBufs& b,
-                             SplitShared& sh, int* status, int* sweeps64, int* sweepsff,
-                             double* flops) {
+template <typename T, class Acc>
+__device__ __forceinline__ SplitOut<T> oriented_split(const Acc& A, int R, int N, double epsrel, float qr_delta,
+                                                      const SplitBufs& b, SplitShared& sh) {
+  typedef QA<T> Q;
+  typedef typename Q::E E;
   const int tid = threadIdx.x, nt = blockDim.x;
-  const bool trans = n > m;
-  const int R = trans ? n : m, N = trans ? m : n;
-  size_t used = 0;
-  auto take = [&](size_t bytes) -> void* {
-    bytes = (bytes + 15) & ~(size_t)15;
-    if (used + bytes > (size_t)b.smem_bytes) return nullptr;
-    void* p = b.smem + used;
-    used += bytes;
-    return p;
-  };
-  // QR / double-float workspace (16 bytes per element in both forms)
-  const bool flip = N >= 8;
-  cff* Wff = nullptr;
-  if (MIXED || flip) {
-    Wff = (cff*)take((size_t)R * N * sizeof(cff));
-    if (!Wff) Wff = b.Wffg;
-  }
-  zc* W = (zc*)take((size_t)R * N * sizeof(zc));
-  if (!W) W = b.Wg;
-  // W = X (R = m) or X^H (R = n), column-major with leading dimension R
+  SplitOut<T> o;
+  const size_t xbytes = (size_t)R * N * sizeof(E);
+  const bool x_shared = xbytes <= (size_t)b.smem_bytes;
+  E* X = x_shared ? reinterpret_cast<E*>(b.smem) : reinterpret_cast<E*>(b.Xg);
+  // power-of-two scale from the largest magnitude (exact)
+  unsigned mx = 0u;
   for (int idx = tid; idx < R * N; idx += nt) {
     const int c = idx / R, r = idx - c * R;
-    W[idx] = trans ? cconj(X(c, r)) : X(r, c);
+    mx = max(mx, A.key(r, c));
   }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((tid & 31) == 0) sh.mag[tid >> 5] = mx;
   __syncthreads();
-  // the QR-preconditioned driver (qr.cuh) returns X^H U (N x kk, ld N)
-  // instead of X V (R x N, ld R): the same two branches below, swapped
-  zc* Wr = W;
-  const size_t spare = (size_t)b.smem_bytes > used ? (size_t)b.smem_bytes - used : 0;
-  int kk;
-  if (flip && MIXED)
-    kk = qr_jacobi_truncate<ff>(W, R, N, Wff, b.smem + used, spare, epsrel, qr_delta, sh.norm, sh.perm,
-                                &sh.jsh, &Wr);
-  else if (flip)
-    kk = qr_jacobi_truncate<double>(W, R, N, reinterpret_cast<zc*>(Wff), b.smem + used, spare, epsrel,
-                                    qr_delta, sh.norm, sh.perm, &sh.jsh, &Wr);
-  else if (MIXED)
-    kk = jacobi_truncate_mixed(W, R, N, Wff, epsrel, sh.norm, sh.perm, &sh.jsh);
-  else
-    kk = jacobi_truncate_fp64(W, R, N, R, epsrel, sh.norm, sh.perm, &sh.jsh);
-  W = Wr;
-  *sweeps64 += sh.jsh.sweeps;  // mixed form: FP64 fallback sweeps only
-  *sweepsff += MIXED ? sh.jsh.sweeps32 : 0;
-  *flops += 4.0 * (6.0 * R * (double)N * N + 20.0 * (double)N * N * N);
-  if (sh.jsh.status != ST_OK || kk > cap) {
-    if (tid == 0) *status = (sh.jsh.status != ST_OK) ? sh.jsh.status : ST_CHI_OVERFLOW;
-    __syncthreads();
-    return 0;
-  }
-  if (!(flip ? !trans : trans)) {
-    // U = W[:, perm] / s;  C = U^H X
-    for (int idx = tid; idx < m * kk; idx += nt) {
-      const int j = idx / m, row = idx - j * m;
-      const int pj = sh.perm[j];
-      b.Tg[idx] = cscale(W[(size_t)pj * m + row], 1.0 / sh.norm[pj]);
-    }
-    for (int idx = tid; idx < kk * n; idx += nt) {
-      const int j = idx / n, col = idx - j * n;
-      const int pj = sh.perm[j];
-      const zc* u = W + (size_t)pj * m;
-      zc acc = mk<double>(0, 0);
-      for (int row = 0; row < m; ++row) cjfma(acc, u[row], X(row, col));
-      b.Cg[idx] = cscale(acc, 1.0 / sh.norm[pj]);
-    }
-  } else {
-    // W = X^H V orthogonal: U = X W[:, perm] / s^2, C = W[:, perm]^H
-    for (int idx = tid; idx < m * kk; idx += nt) {
-      const int j = idx / m, row = idx - j * m;
-      const int pj = sh.perm[j];
-      const double sj = sh.norm[pj];
-      const zc* w = W + (size_t)pj * n;
-      zc acc = mk<double>(0, 0);
-      for (int col = 0; col < n; ++col) cfma(acc, X(row, col), w[col]);
-      b.Tg[idx] = cscale(acc, 1.0 / (sj * sj));
-    }
-    for (int idx = tid; idx < kk * n; idx += nt) {
-      const int j = idx / n, col = idx - j * n;
-      b.Cg[idx] = cconj(W[(size_t)sh.perm[j] * n + col]);
-    }
-  }
-  *flops += 8.0 * (double)m * n * kk;
+  mx = (tid & 31) < (nt >> 5) ? sh.mag[tid & 31] : 0u;
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  o.e = A.exponent(mx);
+  A.load(X, R, N, o.e);
   __syncthreads();
-  return kk;
+  const double scale = ldexp(1.0, o.e);
+  o.flip = N >= QR_MIN_COLS;
+  if (o.flip) {
+    const size_t used = x_shared ? xbytes : 0;
+    o.kk = qr_jacobi_truncate<T>(X, x_shared, R, N, scale, reinterpret_cast<E*>(b.Wg), b.smem + used,
+                                 (size_t)b.smem_bytes - used, b.bkg, epsrel, qr_delta, &sh.book, &sh.jsh, &o.W);
+    return o;
+  }
+  const int sw64 = jacobi_norms<T>(X, R, N, R, scale, sh.book.norm, &sh.jsh);
+  o.kk = jacobi_rank(N, epsrel, sh.book.norm, sh.book.perm, &sh.jsh, sw64, 0.0);
+  o.W = X;
+  return o;
 }
+
+// Accessor of the oriented matrix over a plain array of the split's own
+// element type: A(r, c) = src[c * lds + r], or its conjugate transpose
+// A(r, c) = conj(src[r * lds + c]).
+template <typename T>
+struct PlainSource {
+  typedef QA<T> Q;
+  typedef typename Q::E E;
+  const E* src;
+  int lds;
+  bool trans;
+  __device__ __forceinline__ E at(int r, int c) const {
+    return trans ? src[(size_t)r * lds + c] : src[(size_t)c * lds + r];
+  }
+  __device__ __forceinline__ unsigned key(int r, int c) const { return Q::mag_key(at(r, c)); }
+  __device__ __forceinline__ int exponent(unsigned key) const { return Q::key_exponent(key); }
+  __device__ __forceinline__ void load(E* X, int R, int N, int e) const {
+    const typename Q::P p2 = Q::pow2(-e);
+    for (int idx = threadIdx.x; idx < R * N; idx += blockDim.x) {
+      const int c = idx / R, r = idx - c * R;
+      const E x = Q::ldexpE(at(r, c), p2);
+      X[idx] = trans ? Q::conj(x) : x;
+    }
+  }
+};
 
 }  // namespace otb

@@ -23,8 +23,11 @@
 //
 // Site tensors live in a per-instance ring of fixed-capacity slots, layout
 // [l][a][r] (row-major), 16 bytes per element: complex128 in the complex128
-// form (tempo_step, below), double-float pairs in the mixed form
-// (tempo_step_ff, tempo_ff.cuh).  That layout is also the column-major
+// form, double-float pairs in the mixed form (tempo_step<double> and
+// tempo_step<ff>).  In the mixed form every contraction, QR and Jacobi rotation
+// runs on the FP32 pipe; the FP64 pipe only sees per-split and per-step
+// quantities (kept singular values, the rank decision, the D x D propagators
+// and influences, the D-entry state).  That layout is also the column-major
 // (a r) x l matrix the right-to-left sweep factorises, so sweep splits need
 // no reshuffle.
 #include <math.h>
@@ -36,47 +39,32 @@
 #include "capi_util.h"
 
 #include "engine.h"
-#include "qr.cuh"
+#include "split.cuh"
 
 namespace otb {
 
 constexpr int TEMPO_THREADS = 512;   // largest CTA of the batched kernel (launch bound)
 constexpr int STATIC_THREADS = 256;  // CTA of the allocation-free single-instance kernel
-constexpr int NMAX = 1152;   // max columns of a split (D * cap <= 1152)
-
-typedef cx<double> zc;
 
 struct Bufs {
-  zc* sites;
+  void* sites;
   int2* dims;
   const zc* infl;
   const zc* props;
   zc* out;
-  zc* Wg;            // global working matrix
-  zc* Tg;            // global theta copy / temporaries
-  zc* Cg;            // carry S V^H
-  cff* Wffg;         // global double-float working matrix (mixed form)
-  unsigned char* smem;
-  int smem_bytes;
+  void* Tg;            // theta / temporaries
+  void* Cg;            // carry S V^H / read-out vectors
+  SplitBufs sb;
 };
 
+template <typename T>
 struct SharedStep {
+  typedef typename QA<T>::E E;
   InstState st;
-  JacobiShared jsh;
-  double norm[NMAX];
-  int perm[NMAX];
-  cff pf[3][81];   // mixed form: P1, P2 and the site's influence in double-float
+  SplitShared ss;
+  E pf[3][81];   // P1, P2 and the site's influence
   int inst;
 };
-
-// Truncated split of the R x N (R >= N) matrix A = op(src): op is the
-// identity (A(row,c) = src[c*lds+row]) or the conjugate transpose
-// (A(row,c) = conj(src[row*lds+c])).  On return *Wout holds A V (FP64,
-// orthogonal columns, ld R) -- or, when *flip is set (the QR-preconditioned
-// mixed driver), A^H U (FP64, N x kept, ld N) -- with sh.norm / sh.perm /
-// return value as in jacobi_finish.  Shared memory is used for the working
-// matrices that fit.
-constexpr int QR_MIN_COLS = 8;
 
 // Device clock in ns (the launch timeline recorded per instance).
 __device__ __forceinline__ long long globaltimer_ns() {
@@ -85,52 +73,36 @@ __device__ __forceinline__ long long globaltimer_ns() {
   return (long long)t;
 }
 
-__device__ __noinline__ int split(const zc* src, int lds, bool src_trans, int R, int N, double epsrel, float qr_delta,
-                     Bufs& b, SharedStep& sh, zc** Wout, bool* flip) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  size_t used = 0;
-  auto take = [&](size_t bytes) -> void* {
-    bytes = (bytes + 15) & ~(size_t)15;
-    if (used + bytes > (size_t)b.smem_bytes) return nullptr;
-    void* p = b.smem + used;
-    used += bytes;
-    return p;
-  };
-  // QR workspace (16 bytes per element in both forms: cff or complex128)
-  const bool qr = N >= QR_MIN_COLS;
-  cff* Wff = nullptr;
-  if (qr) {
-    Wff = (cff*)take((size_t)R * N * sizeof(cff));
-    if (!Wff) Wff = b.Wffg;
-  }
-  zc* W = (zc*)take((size_t)R * N * sizeof(zc));
-  if (!W) W = b.Wg;
-  for (int idx = tid; idx < R * N; idx += nt) {
-    const int c = idx / R, row = idx - c * R;
-    W[idx] = src_trans ? cconj(src[(size_t)row * lds + c]) : src[(size_t)c * lds + row];
-  }
-  __syncthreads();
-  int kk;
-  *flip = false;
-  if (qr) {
-    *flip = true;
-    const size_t spare = (size_t)b.smem_bytes > used ? (size_t)b.smem_bytes - used : 0;
-    return qr_jacobi_truncate<double>(W, R, N, reinterpret_cast<zc*>(Wff), b.smem + used, spare, epsrel,
-                                      qr_delta, sh.norm, sh.perm, &sh.jsh, Wout);
-  }
-  kk = jacobi_truncate_fp64(W, R, N, R, epsrel, sh.norm, sh.perm, &sh.jsh);
-  *Wout = W;
-  return kk;
+// One split of the step: its own function, so that the step's registers are
+// not live inside it.
+template <typename T>
+__device__ __noinline__ SplitOut<T> split(const PlainSource<T>& src, int R, int N, double epsrel, float qr_delta,
+                                          const SplitBufs& b, SplitShared& sh) {
+  return oriented_split<T>(src, R, N, epsrel, qr_delta, b, sh);
 }
 
-}  // namespace otb
+// The kept columns' scale factors in place of their norms, one FP64 division
+// each, for a W that is 2^-e times the factor: 2^e / s (wt false) or 2^e / s^2
+// (wt true).
+template <typename T>
+__device__ __forceinline__ const typename QA<T>::S* kept_inverses(SplitShared& sh, int kk, bool wt, int e) {
+  typedef typename QA<T>::S S;
+  S* sinv = reinterpret_cast<S*>(sh.book.norm);
+  for (int j = threadIdx.x; j < kk; j += blockDim.x) {
+    const int pj = sh.book.perm[j];
+    const double s = sh.book.norm[pj];
+    sinv[pj] = QA<T>::fromd(ldexp(1.0, e) / (wt ? s * s : s));
+  }
+  __syncthreads();
+  return sinv;
+}
 
-#include "tempo_ff.cuh"
-
-namespace otb {
-
-__device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, Bufs& b,
-                           SharedStep& sh) {
+template <typename T>
+__device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, const Bufs& b, SharedStep<T>& sh) {
+  typedef QA<T> Q;
+  typedef typename Q::E E;
+  typedef typename Q::S S;
+  typedef typename Q::Acc Acc;
   const int tid = threadIdx.x;
   const int nt = blockDim.x;
   if (tid == 0) sh.st = L.state[i];
@@ -141,53 +113,61 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, Bufs& 
   const long long slot_elems = (long long)cap * D * cap;
   const int step = sh.st.step + 1;
   const long long window = min((long long)step, (long long)I.dkmax + 1);
-  zc* const sites = b.sites + I.site_base;
+  E* const sites = reinterpret_cast<E*>(b.sites) + I.site_base;
   int2* const dims = b.dims + I.dims_base;
   const zc* P1 = b.props + I.prop_base;
   const zc* P2 = P1 + D * D;
+  E* const Tf = reinterpret_cast<E*>(b.Tg);   // theta / temporaries
+  E* const Cf = reinterpret_cast<E*>(b.Cg);   // carry / read-out vectors
   int splits = 0, sw64 = 0, sw32 = 0;
-  double flops = 0.0;  // algorithmic flops of this step (thread 0's copy is used)
+  double flops = 0.0;
+  // the step's propagators in the step's arithmetic, staged once
+  for (int idx = tid; idx < D * D; idx += nt) {
+    sh.pf[0][idx] = Q::from(P1[idx]);
+    sh.pf[1][idx] = Q::from(P2[idx]);
+  }
+  __syncthreads();
 
 #define SLOT(k) ((sh.st.head + (k)) % I.nslots)
 #define SITE(k) (sites + (long long)SLOT(k) * slot_elems)
 #define DIMS(k) (dims[SLOT(k)])
 
-  // 1. first half-step propagator on the newest site: A[l][b][0] = sum_a P1[b][a] A[l][a][0]
+  // 1. first half-step propagator on the newest site
   {
     const int k = sh.st.nsites - 1;
-    zc* A = SITE(k);
+    E* A = SITE(k);
     const int l = DIMS(k).x;
     for (int idx = tid; idx < l * D; idx += nt) {
       const int ll = idx / D, bb = idx - ll * D;
-      zc acc = mk<double>(0, 0);
-      for (int a = 0; a < D; ++a) cfma(acc, P1[bb * D + a], A[ll * D + a]);
-      b.Tg[idx] = acc;
+      Acc f = Q::acc_zero();
+      for (int a = 0; a < D; ++a) Q::acc_fma(f, sh.pf[0][bb * D + a], A[ll * D + a]);
+      Tf[idx] = Q::acc_value(f);
     }
     __syncthreads();
-    for (int idx = tid; idx < l * D; idx += nt) A[idx] = b.Tg[idx];
+    for (int idx = tid; idx < l * D; idx += nt) A[idx] = Tf[idx];
     __syncthreads();
   }
 
   // 2. trace out the oldest site (sum_north = ones) and merge into the next
   if (sh.st.nsites > window) {
-    zc* A0 = SITE(0);
-    zc* A1 = SITE(1);
+    E* A0 = SITE(0);
+    E* A1 = SITE(1);
     const int r0 = DIMS(0).y;
     const int r1 = DIMS(1).y;
     for (int c = tid; c < r0; c += nt) {
-      zc acc = mk<double>(0, 0);
-      for (int a = 0; a < D; ++a) acc = acc + A0[a * r0 + c];
-      b.Cg[c] = acc;
+      E acc = A0[c];
+      for (int a = 1; a < D; ++a) acc = Q::add(acc, A0[a * r0 + c]);
+      Cf[c] = acc;
     }
     __syncthreads();
     for (int idx = tid; idx < D * r1; idx += nt) {
       const int a = idx / r1, rr = idx - a * r1;
-      zc acc = mk<double>(0, 0);
-      for (int c = 0; c < r0; ++c) cfma(acc, b.Cg[c], A1[((long long)c * D + a) * r1 + rr]);
-      b.Tg[idx] = acc;
+      Acc f = Q::acc_zero();
+      for (int c = 0; c < r0; ++c) Q::acc_fma(f, Cf[c], A1[((long long)c * D + a) * r1 + rr]);
+      Tf[idx] = Q::acc_value(f);
     }
     __syncthreads();
-    for (int idx = tid; idx < D * r1; idx += nt) A1[idx] = b.Tg[idx];
+    for (int idx = tid; idx < D * r1; idx += nt) A1[idx] = Tf[idx];
     __syncthreads();
     if (tid == 0) {
       dims[(sh.st.head + 1) % I.nslots] = make_int2(1, r1);
@@ -201,16 +181,17 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, Bufs& 
   // 3. zip-up: theta[(x,a),(r,m)] = I_dk[a,m] sum_c C[x,c,m] A[c,a,r]
   int cxd = 1, ccd = 1;
   for (int k = 0; k < K; ++k) {
-    zc* A = SITE(k);
+    E* A = SITE(k);
     const int r = DIMS(k).y;
     const int dk = K - 1 - k;
     const zc* Im = (k == 0 && sh.st.ovr_active) ? (b.props + I.ovr_base)
                                                  : (b.infl + I.infl_base + (long long)dk * D * D);
+    for (int idx = tid; idx < D * D; idx += nt) sh.pf[2][idx] = Q::from(Im[idx]);
+    __syncthreads();
     const int m = cxd * D;
     const int n = r * D;
-    const zc* C = b.Cg;
     const bool last = (k == K - 1);
-    // theta into Tg: column-major (ld m) for a split, site layout for the last site
+    // theta into Tf: column-major (ld m) for a split, site layout for the last site
     for (int idx = tid; idx < m * n; idx += nt) {
       int row, col;
       if (last) {
@@ -222,71 +203,74 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, Bufs& 
       }
       const int x = row / D, a = row - x * D;
       const int rr = col / D, mr = col - rr * D;
-      zc acc = mk<double>(0, 0);
+      Acc f = Q::acc_zero();
       if (k == 0) {
-        acc = A[a * r + rr];
+        Q::acc_fma(f, sh.pf[2][a * D + mr], A[a * r + rr]);
       } else {
+        Acc g = Q::acc_zero();
         for (int c = 0; c < ccd; ++c)
-          cfma(acc, C[(long long)x * (ccd * D) + c * D + mr], A[((long long)c * D + a) * r + rr]);
+          Q::acc_fma(g, Cf[(long long)x * (ccd * D) + c * D + mr], A[((long long)c * D + a) * r + rr]);
+        Q::acc_fma(f, sh.pf[2][a * D + mr], Q::acc_value(g));
       }
-      b.Tg[idx] = cmul(Im[a * D + mr], acc);
+      Tf[idx] = Q::acc_value(f);
     }
     __syncthreads();
     if (last) {
-      for (int idx = tid; idx < m * n; idx += nt) A[idx] = b.Tg[idx];
+      for (int idx = tid; idx < m * n; idx += nt) A[idx] = Tf[idx];
       if (tid == 0) dims[SLOT(k)] = make_int2(cxd, n);
       __syncthreads();
       break;
     }
     const bool trans = n > m;
-    zc* W;
-    bool flip;
-    const int kk = trans ? split(b.Tg, m, true, n, m, I.epsrel, I.qr_delta, b, sh, &W, &flip)
-                         : split(b.Tg, m, false, m, n, I.epsrel, I.qr_delta, b, sh, &W, &flip);
+    const PlainSource<T> src{Tf, m, trans};
+    const SplitOut<T> o = split<T>(src, trans ? n : m, trans ? m : n, I.epsrel, I.qr_delta, b.sb, sh.ss);
+    const E* W = o.W;
+    const int kk = o.kk;
     {
       const double R = trans ? n : m, N = trans ? m : n;
       flops += 8.0 * m * n * ccd + 4.0 * (6.0 * R * N * N + 20.0 * N * N * N);
     }
     ++splits;
-    sw64 += sh.jsh.sweeps;
-    sw32 += sh.jsh.sweeps32;
-    if (sh.jsh.status != ST_OK || kk > cap) {
-      if (tid == 0) sh.st.status = (sh.jsh.status != ST_OK) ? sh.jsh.status : ST_CHI_OVERFLOW;
+    sw64 += sh.ss.jsh.sweeps;
+    sw32 += sh.ss.jsh.sweeps32;
+    if (sh.ss.jsh.status != ST_OK || kk > cap) {
+      if (tid == 0) sh.st.status = (sh.ss.jsh.status != ST_OK) ? sh.ss.jsh.status : ST_CHI_OVERFLOW;
       __syncthreads();
       break;
     }
-    // W = theta V (U S) or W = theta^H U (V S), by orientation and driver
-    const bool wt = flip ? !trans : trans;
+    // W 2^e = theta V (U S, ld m) or theta^H U (V S, ld n), by orientation and driver
+    const bool wt = o.flip ? !trans : trans;
+    const S* sinv = kept_inverses<T>(sh.ss, kk, wt, o.e);
     if (!wt) {
-      // U = W[:, perm] / s  -> site (cxd, D, kk);  carry = U^H theta
+      // U = W[:, perm] / s -> site (cxd, D, kk);  carry = U^H theta
       for (int idx = tid; idx < m * kk; idx += nt) {
         const int row = idx / kk, j = idx - row * kk;
-        const int pj = sh.perm[j];
-        A[idx] = cscale(W[(long long)pj * m + row], 1.0 / sh.norm[pj]);
+        const int pj = sh.ss.book.perm[j];
+        A[idx] = Q::scaleE(W[(long long)pj * m + row], sinv[pj]);
       }
       for (int idx = tid; idx < kk * n; idx += nt) {
         const int j = idx / n, col = idx - j * n;
-        const int pj = sh.perm[j];
-        const zc* u = W + (long long)pj * m;
-        const zc* th = b.Tg + (long long)col * m;
-        zc acc = mk<double>(0, 0);
-        for (int row = 0; row < m; ++row) cjfma(acc, u[row], th[row]);
-        b.Cg[idx] = cscale(acc, 1.0 / sh.norm[pj]);
+        const int pj = sh.ss.book.perm[j];
+        const E* u = W + (long long)pj * m;
+        const E* th = Tf + (long long)col * m;
+        Acc f = Q::acc_zero();
+        for (int row = 0; row < m; ++row) Q::acc_fmaj(f, u[row], th[row]);
+        Cf[idx] = Q::scaleE(Q::acc_value(f), sinv[pj]);
       }
     } else {
-      // W = theta^H V orthogonal: U = theta W[:, perm] / s^2, carry = W[:, perm]^H
+      // U = theta W[:, perm] / s^2 -> site;  carry = W[:, perm]^H
+      const typename Q::P up = Q::pow2(o.e);
       for (int idx = tid; idx < m * kk; idx += nt) {
         const int row = idx / kk, j = idx - row * kk;
-        const int pj = sh.perm[j];
-        const double sj = sh.norm[pj];
-        const zc* w = W + (long long)pj * n;
-        zc acc = mk<double>(0, 0);
-        for (int col = 0; col < n; ++col) cfma(acc, b.Tg[(long long)col * m + row], w[col]);
-        A[idx] = cscale(acc, 1.0 / (sj * sj));
+        const int pj = sh.ss.book.perm[j];
+        const E* w = W + (long long)pj * n;
+        Acc f = Q::acc_zero();
+        for (int col = 0; col < n; ++col) Q::acc_fma(f, Tf[(long long)col * m + row], w[col]);
+        A[idx] = Q::scaleE(Q::acc_value(f), sinv[pj]);
       }
       for (int idx = tid; idx < kk * n; idx += nt) {
         const int j = idx / n, col = idx - j * n;
-        b.Cg[idx] = cconj(W[(long long)sh.perm[j] * n + col]);
+        Cf[idx] = Q::ldexpE(Q::conj(W[(long long)sh.ss.book.perm[j] * n + col]), up);
       }
     }
     if (tid == 0) dims[SLOT(k)] = make_int2(cxd, kk);
@@ -298,76 +282,79 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, Bufs& 
   // 4. right-to-left sweep: site k as the column-major (D r) x l matrix
   if (sh.st.status == ST_OK) {
     for (int k = K - 1; k >= 1; --k) {
-      zc* A = SITE(k);
+      E* A = SITE(k);
       const int2 dA = DIMS(k);
       const int l = dA.x, r = dA.y;
       const int m = D * r, n = l;
       const bool trans = n > m;
-      zc* W;
-      bool flip;
-      const int kk = trans ? split(A, m, true, n, m, I.epsrel, I.qr_delta, b, sh, &W, &flip)
-                           : split(A, m, false, m, n, I.epsrel, I.qr_delta, b, sh, &W, &flip);
+      const PlainSource<T> src{A, m, trans};
+      const SplitOut<T> o = split<T>(src, trans ? n : m, trans ? m : n, I.epsrel, I.qr_delta, b.sb, sh.ss);
+      const E* W = o.W;
+      const int kk = o.kk;
       {
         const double R = trans ? n : m, N = trans ? m : n;
         flops += 4.0 * (6.0 * R * N * N + 20.0 * N * N * N) + 8.0 * DIMS(k - 1).x * D * (double)kk * n;
       }
       ++splits;
-      sw64 += sh.jsh.sweeps;
-      sw32 += sh.jsh.sweeps32;
-      if (sh.jsh.status != ST_OK || kk > cap) {
-        if (tid == 0) sh.st.status = (sh.jsh.status != ST_OK) ? sh.jsh.status : ST_CHI_OVERFLOW;
+      sw64 += sh.ss.jsh.sweeps;
+      sw32 += sh.ss.jsh.sweeps32;
+      if (sh.ss.jsh.status != ST_OK || kk > cap) {
+        if (tid == 0) sh.st.status = (sh.ss.jsh.status != ST_OK) ? sh.ss.jsh.status : ST_CHI_OVERFLOW;
         __syncthreads();
         break;
       }
-      const bool wt = flip ? !trans : trans;
+      const bool wt = o.flip ? !trans : trans;
+      const S* sinv = kept_inverses<T>(sh.ss, kk, wt, o.e);
       if (!wt) {
+        // carry = U^H A (U = W / s), then U -> site k (kk, D, r)
         for (int idx = tid; idx < kk * n; idx += nt) {
           const int j = idx / n, col = idx - j * n;
-          const int pj = sh.perm[j];
-          const zc* u = W + (long long)pj * m;
-          const zc* y = A + (long long)col * m;
-          zc acc = mk<double>(0, 0);
-          for (int row = 0; row < m; ++row) cjfma(acc, u[row], y[row]);
-          b.Cg[idx] = cscale(acc, 1.0 / sh.norm[pj]);
+          const int pj = sh.ss.book.perm[j];
+          const E* u = W + (long long)pj * m;
+          const E* y = A + (long long)col * m;
+          Acc f = Q::acc_zero();
+          for (int row = 0; row < m; ++row) Q::acc_fmaj(f, u[row], y[row]);
+          Cf[idx] = Q::scaleE(Q::acc_value(f), sinv[pj]);
         }
         __syncthreads();
         for (int idx = tid; idx < m * kk; idx += nt) {
           const int j = idx / m, row = idx - j * m;
-          const int pj = sh.perm[j];
-          A[idx] = cscale(W[(long long)pj * m + row], 1.0 / sh.norm[pj]);
+          const int pj = sh.ss.book.perm[j];
+          A[idx] = Q::scaleE(W[(long long)pj * m + row], sinv[pj]);
         }
       } else {
+        // U = A W[:, perm] / s^2 -> Tf, carry = W[:, perm]^H, then Tf -> site k
+        const typename Q::P up = Q::pow2(o.e);
         for (int idx = tid; idx < m * kk; idx += nt) {
           const int j = idx / m, row = idx - j * m;
-          const int pj = sh.perm[j];
-          const double sj = sh.norm[pj];
-          const zc* w = W + (long long)pj * n;
-          zc acc = mk<double>(0, 0);
-          for (int col = 0; col < n; ++col) cfma(acc, A[(long long)col * m + row], w[col]);
-          b.Tg[idx] = cscale(acc, 1.0 / (sj * sj));
+          const int pj = sh.ss.book.perm[j];
+          const E* w = W + (long long)pj * n;
+          Acc f = Q::acc_zero();
+          for (int col = 0; col < n; ++col) Q::acc_fma(f, A[(long long)col * m + row], w[col]);
+          Tf[idx] = Q::scaleE(Q::acc_value(f), sinv[pj]);
         }
         for (int idx = tid; idx < kk * n; idx += nt) {
           const int j = idx / n, col = idx - j * n;
-          b.Cg[idx] = cconj(W[(long long)sh.perm[j] * n + col]);
+          Cf[idx] = Q::ldexpE(Q::conj(W[(long long)sh.ss.book.perm[j] * n + col]), up);
         }
         __syncthreads();
-        for (int idx = tid; idx < m * kk; idx += nt) A[idx] = b.Tg[idx];
+        for (int idx = tid; idx < m * kk; idx += nt) A[idx] = Tf[idx];
       }
       if (tid == 0) dims[SLOT(k)] = make_int2(kk, r);
       __syncthreads();
       // absorb S V^H into site k-1: (l2, D, n) x (kk, n)^T -> (l2, D, kk)
-      zc* B = SITE(k - 1);
+      E* B = SITE(k - 1);
       const int l2 = DIMS(k - 1).x;
       for (int idx = tid; idx < l2 * D * kk; idx += nt) {
         const int la = idx / kk, j = idx - la * kk;
-        const zc* brow = B + (long long)la * n;
-        const zc* crow = b.Cg + (long long)j * n;
-        zc acc = mk<double>(0, 0);
-        for (int c = 0; c < n; ++c) cfma(acc, brow[c], crow[c]);
-        b.Tg[idx] = acc;
+        const E* brow = B + (long long)la * n;
+        const E* crow = Cf + (long long)j * n;
+        Acc f = Q::acc_zero();
+        for (int c = 0; c < n; ++c) Q::acc_fma(f, brow[c], crow[c]);
+        Tf[idx] = Q::acc_value(f);
       }
       __syncthreads();
-      for (int idx = tid; idx < l2 * D * kk; idx += nt) B[idx] = b.Tg[idx];
+      for (int idx = tid; idx < l2 * D * kk; idx += nt) B[idx] = Tf[idx];
       if (tid == 0) dims[SLOT(k - 1)] = make_int2(l2, kk);
       __syncthreads();
     }
@@ -379,10 +366,10 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, Bufs& 
 
   // 5. second half-step propagator as the new last site: A[r][b][0] = P2[b][r]
   {
-    zc* A = SITE(K);
+    E* A = SITE(K);
     for (int idx = tid; idx < D * D; idx += nt) {
       const int rr = idx / D, bb = idx - rr * D;
-      A[idx] = P2[bb * D + rr];
+      A[idx] = sh.pf[1][bb * D + rr];
     }
     if (tid == 0) {
       dims[SLOT(K)] = make_int2(D, 1);
@@ -394,31 +381,32 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, Bufs& 
   // 6. read-out: v <- sum_{c,a} v[c] A[c][a][r] over all sites, state = P2 v
   {
     int cur = 0;
-    // the two read-out vectors live in the carry buffer (dead after the sweep)
-    zc* const vv[2] = {b.Cg, b.Cg + cap};
-    if (tid == 0) vv[0][0] = mk<double>(1, 0);
+    E* const vv[2] = {Cf, Cf + cap};
+    if (tid == 0) {
+      vv[0][0] = Q::from(mk<double>(1.0, 0.0));
+    }
     __syncthreads();
     int maxb = 1;
     for (int k = 0; k < K; ++k) {
-      const zc* A = SITE(k);
+      const E* A = SITE(k);
       const int2 dA = DIMS(k);
       const int l = dA.x, r = dA.y;
       maxb = max(maxb, r);
       for (int rr = tid; rr < r; rr += nt) {
-        zc acc = mk<double>(0, 0);
+        Acc f = Q::acc_zero();
         for (int c = 0; c < l; ++c) {
-          zc part = mk<double>(0, 0);
-          for (int a = 0; a < D; ++a) part = part + A[((long long)c * D + a) * r + rr];
-          cfma(acc, vv[cur][c], part);
+          E part = A[((long long)c * D) * r + rr];
+          for (int a = 1; a < D; ++a) part = Q::add(part, A[((long long)c * D + a) * r + rr]);
+          Q::acc_fma(f, vv[cur][c], part);
         }
-        vv[cur ^ 1][rr] = acc;
+        vv[cur ^ 1][rr] = Q::acc_value(f);
       }
       __syncthreads();
       cur ^= 1;
     }
     if (tid < D) {
       zc acc = mk<double>(0, 0);
-      for (int c = 0; c < D; ++c) cfma(acc, P2[tid * D + c], vv[cur][c]);
+      for (int c = 0; c < D; ++c) cfma(acc, P2[tid * D + c], Q::to(vv[cur][c]));
       b.out[I.out_base + (long long)((step - I.out_origin) % I.out_cap) * D + tid] = acc;
     }
     if (tid == 0) {
@@ -440,21 +428,23 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, Bufs& 
 
 template <bool MIXED>
 __global__ void __launch_bounds__(TEMPO_THREADS, 1) tempo_kernel(TempoLaunch L) {
+  typedef typename StepType<MIXED>::T T;
   extern __shared__ __align__(16) unsigned char dsm[];
-  __shared__ SharedStep sh;
+  __shared__ SharedStep<T> sh;
   Bufs b;
-  b.sites = (zc*)L.sites;
+  b.sites = L.sites;
   b.dims = L.dims;
   b.infl = (const zc*)L.infl;
   b.props = (const zc*)L.props;
   b.out = (zc*)L.out;
   unsigned char* work = (unsigned char*)L.work + (long long)blockIdx.x * L.work_stride;
-  b.Wg = (zc*)work;
-  b.Tg = b.Wg + L.wcap;
-  b.Cg = b.Tg + L.wcap;
-  b.Wffg = (cff*)(b.Cg + L.wcap);
-  b.smem = dsm;
-  b.smem_bytes = L.smem_bytes;
+  b.sb.Wg = work;
+  b.Tg = work + L.wcap * 16;
+  b.Cg = work + L.wcap * 32;
+  b.sb.Xg = work + L.wcap * 48;
+  b.sb.bkg = work + L.wcap * 64;
+  b.sb.smem = dsm;
+  b.sb.smem_bytes = L.smem_bytes;
   for (;;) {
     if (threadIdx.x == 0) sh.inst = atomicAdd(L.queue, 1);
     __syncthreads();
@@ -465,10 +455,7 @@ __global__ void __launch_bounds__(TEMPO_THREADS, 1) tempo_kernel(TempoLaunch L) 
     const InstDev I = L.inst[i];
     const long long t0 = globaltimer_ns();
     for (int s = 0; s < L.nsteps; ++s) {
-      if (MIXED)
-        tempo_step_ff(L, I, i, b, sh);
-      else
-        tempo_step(L, I, i, b, sh);
+      tempo_step<T>(L, I, i, b, sh);
       __syncthreads();
       if (sh.st.status != ST_OK) break;
     }
@@ -582,20 +569,23 @@ static __device__ __align__(256) unsigned char g_tempo_static_scratch[STATIC_SCR
 template <bool MIXED>
 __global__ void __launch_bounds__(STATIC_THREADS)
     tempo_static_kernel(TempoLaunch L, InstDev I, const double* rho0, int nsteps, int* status_out) {
+  typedef typename StepType<MIXED>::T T;
   extern __shared__ __align__(16) unsigned char dsm[];
-  __shared__ SharedStep sh;
+  __shared__ SharedStep<T> sh;
   Bufs b;
-  b.sites = (zc*)L.sites;
+  b.sites = L.sites;
   b.dims = L.dims;
   b.infl = (const zc*)L.infl;
   b.props = (const zc*)L.props;
   b.out = (zc*)L.out;
-  b.Wg = (zc*)L.work;
-  b.Tg = b.Wg + L.wcap;
-  b.Cg = b.Tg + L.wcap;
-  b.Wffg = (cff*)(b.Cg + L.wcap);
-  b.smem = dsm;
-  b.smem_bytes = L.smem_bytes;
+  unsigned char* work = (unsigned char*)L.work;
+  b.sb.Wg = work;
+  b.Tg = work + L.wcap * 16;
+  b.Cg = work + L.wcap * 32;
+  b.sb.Xg = work + L.wcap * 48;
+  b.sb.bkg = nullptr;   // chi_cap * D <= 128: the bookkeeping always fits in shared memory
+  b.sb.smem = dsm;
+  b.sb.smem_bytes = L.smem_bytes;
   const int tid = threadIdx.x;
   if (tid == 0) sh.st = L.state[0];
   __syncthreads();
@@ -603,10 +593,7 @@ __global__ void __launch_bounds__(STATIC_THREADS)
     // first call on a zeroed MPS buffer: the initial state as a (1, D, 1) site
     // the mixed form keeps its sites in double-float
     for (int a = tid; a < I.D; a += blockDim.x) {
-      if (MIXED)
-        reinterpret_cast<cff*>(b.sites)[a] = cff_from(((const zc*)rho0)[a]);
-      else
-        b.sites[a] = ((const zc*)rho0)[a];
+      reinterpret_cast<typename QA<T>::E*>(b.sites)[a] = QA<T>::from(((const zc*)rho0)[a]);
     }
     if (tid == 0) {
       b.dims[0] = make_int2(1, 1);
@@ -621,10 +608,7 @@ __global__ void __launch_bounds__(STATIC_THREADS)
   const int first = sh.st.step;
   __syncthreads();
   for (int s = 0; s < nsteps; ++s) {
-    if (MIXED)
-      tempo_step_ff(L, I, 0, b, sh);
-    else
-      tempo_step(L, I, 0, b, sh);
+    tempo_step<T>(L, I, 0, b, sh);
     __syncthreads();
     if (sh.st.status != ST_OK) break;
   }
