@@ -65,10 +65,14 @@ typedef struct {
   int32_t precision;   /* OTB_PRECISION_* */
   int32_t chi_cap;     /* bond-dimension capacity of every site, chi_cap * D <= 1152 */
   int32_t out_cap;     /* states kept per instance (ring), >= 2 */
-  int32_t grid;        /* CTAs per launch, 0 = 3 per SM */
-  int32_t block;       /* threads per CTA (64..512, multiple of 32), 0 = 256 */
+  int32_t grid;        /* CTAs per launch, 0 = 2 per SM for blocks up
+                          to 256 threads, 1 per SM above */
+  int32_t block;       /* threads per CTA (64..512, multiple of 32), 0 =
+                          512 for batches of up to one instance per SM,
+                          256 for larger ones */
   int32_t smem_kb;     /* dynamic shared memory per CTA for working matrices
-                          (KiB, <= 200), 0 = 56 */
+                          (KiB, <= 200), 0 = 200 for one CTA per SM, 100
+                          for two */
   double qr_cut;       /* relative cut of the rank-revealing QR that precedes
                           the Jacobi SVD of every split of >= 8 columns: the
                           factorisation stops once the remaining block's
@@ -117,10 +121,9 @@ void otb_tempo_destroy(otb_tempo* h);
  * for every instance of the handle. */
 otb_status otb_tempo_advance(otb_tempo* h, int32_t nsteps, void* stream);
 /* Launch shape of the next advances (no reference counterpart: the
- * reference has no launch): block threads per CTA (64..512, 0 = 256),
- * smem_kb dynamic shared memory per CTA (<= 200, 0 = 56), grid CTAs (0 = 3
- * per SM for blocks up to 256 threads, 1 per SM above; capped at the grid
- * the handle's workspace was allocated for).  Used by the per-bond-bucket
+ * reference has no launch): block threads per CTA (64..512), smem_kb
+ * dynamic shared memory per CTA (<= 200), grid CTAs (capped at the grid the
+ * handle's workspace was allocated for); 0 = otb_tempo_config's defaults.  Used by the per-bond-bucket
  * launch-shape tuner. */
 otb_status otb_tempo_set_launch(otb_tempo* h, int32_t block, int32_t smem_kb, int32_t grid);
 /* States of steps [first_step, first_step+count) of one instance, each D

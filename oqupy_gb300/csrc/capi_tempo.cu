@@ -122,6 +122,21 @@ otb_status upload_inst(otb_tempo* h) {
   return OTB_OK;
 }
 
+// Launch shape where the caller gives none (block / smem_bytes / grid 0).
+// A kernel's registers allow 512 threads per SM.  A batch of at most one
+// instance per SM runs one 512-thread CTA with the largest shared-memory share
+// on each; more instances share an SM two by two (256 threads, 100 KiB): 253
+// spin-boson instances, 40 steps, 242 ms that way and 266 ms one by one; 95
+// converged ones (splits of ~75 x 34 columns), 12 steps, 212 and 176 ms.
+// CTAs of more than 256 threads (128 registers each) fill an SM alone.
+void launch_shape(otb_tempo* h, int block, int smem_bytes, int grid) {
+  const bool alone = h->n <= h->sms;
+  h->block = block > 0 ? block : (alone ? 512 : 256);
+  const int per_sm = h->block > 256 ? 1 : 2;
+  h->smem_bytes = smem_bytes > 0 ? smem_bytes : (per_sm == 1 || alone ? 200 : 100) * 1024;
+  h->grid = grid > 0 ? grid : std::max(1, std::min(h->n, per_sm * h->sms));
+}
+
 otb_status check_inst(otb_tempo* h, int32_t inst) {
   if (!h) return set_error(OTB_ERR_INVALID_ARG, "null handle");
   if (inst < 0 || inst >= h->n) return set_error(OTB_ERR_INVALID_ARG, "instance index out of range");
@@ -146,8 +161,6 @@ extern "C" otb_status otb_tempo_create(const otb_tempo_config* cfg, int32_t n,
   if (!(cfg->qr_cut >= 0.0) || !(cfg->qr_cut < 1.0))
     return set_error(OTB_ERR_INVALID_ARG, "qr_cut must be in [0, 1)");
   std::unique_ptr<otb_tempo> h(new otb_tempo());
-  h->block = cfg->block > 0 ? cfg->block : 256;
-  h->smem_bytes = cfg->smem_kb * 1024;
   h->n = n;
   h->precision = cfg->precision;
   h->cap = cfg->chi_cap;
@@ -278,15 +291,11 @@ extern "C" otb_status otb_tempo_create(const otb_tempo_config* cfg, int32_t n,
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // default launch shape: 3 CTAs of 256 threads per SM with 56 KiB smem;
-  // CTAs of more than 256 threads (128 registers each) fill an SM alone
-  const int per_sm = h->block > 256 ? 1 : 3;
   h->sms = std::max(sms, 1);
-  h->grid = cfg->grid > 0 ? cfg->grid : std::max(1, std::min(n, per_sm * h->sms));
+  launch_shape(h.get(), cfg->block, cfg->smem_kb * 1024, cfg->grid);
   // workspace for the widest default grid, so otb_tempo_set_launch can
   // switch shapes later (an explicit grid fixes it)
-  h->grid_alloc = cfg->grid > 0 ? cfg->grid : std::max(h->grid, std::min(n, 3 * h->sms));
-  if (h->smem_bytes == 0) h->smem_bytes = 56 * 1024;
+  h->grid_alloc = cfg->grid > 0 ? cfg->grid : std::max(h->grid, std::min(n, 2 * h->sms));
   h->wcap = (long long)(h->cap * h->Dmax) * (h->cap * h->Dmax);
   h->work_stride = tempo_work_bytes(h->wcap);
   if (!h->d_work.alloc((size_t)h->grid_alloc * h->work_stride)) return OTB_ERR_OOM;
@@ -346,11 +355,8 @@ extern "C" otb_status otb_tempo_set_launch(otb_tempo* h, int32_t block, int32_t 
     return set_error(OTB_ERR_INVALID_ARG, "block must be 0 or a multiple of 32 in [64, 512]");
   if (smem_kb < 0 || smem_kb > 200) return set_error(OTB_ERR_INVALID_ARG, "smem_kb must be in [0, 200]");
   if (grid < 0) return set_error(OTB_ERR_INVALID_ARG, "grid must be >= 0");
-  h->block = block > 0 ? block : 256;
-  h->smem_bytes = (smem_kb > 0 ? smem_kb : 56) * 1024;
-  const int per_sm = h->block > 256 ? 1 : 3;
-  const int want = grid > 0 ? grid : std::min(h->n, per_sm * h->sms);
-  h->grid = std::max(1, std::min(want, h->grid_alloc));
+  launch_shape(h, block, smem_kb * 1024, grid);
+  h->grid = std::max(1, std::min(h->grid, h->grid_alloc));
   return OTB_OK;
 }
 
