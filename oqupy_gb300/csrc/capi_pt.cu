@@ -3,6 +3,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -25,9 +26,18 @@ struct otb_pt {
   DevBuf d_inst, d_state, d_dims, d_sites, d_infl, d_neg, d_caps, d_work, d_queue, d_order;
   long long wcap = 0;
   long long work_stride = 0;
+  // completed builds: their bonds on the host (a completed build never changes)
+  std::mutex mutex;
+  std::vector<std::vector<int2>> final_dims;
+  // workspace of the sweeps, kept between calls up to SWEEP_KEEP_BYTES; a call
+  // that finds it in use (another thread's) allocates its own
+  std::mutex sweep_mutex;
+  DevBuf sweep_ws;
 };
 
 namespace {
+
+constexpr size_t SWEEP_KEEP_BYTES = (size_t)256 << 20;
 
 otb_status pt_check(otb_pt* h, int32_t inst) {
   if (!h) return set_error(OTB_ERR_INVALID_ARG, "null handle");
@@ -71,6 +81,7 @@ extern "C" otb_status otb_pt_create(const otb_pt_config* cfg, int32_t n, const o
   h->cap = cfg->chi_cap;
   h->inst.resize(n);
   h->state.assign(n, PtState{});
+  h->final_dims.resize(n);
   std::vector<double> infl, neg;
   long long site_total = 0, dims_total = 0, caps_total = 0;
   for (int i = 0; i < n; ++i) {
@@ -259,102 +270,143 @@ extern "C" otb_status otb_pt_get_cap(otb_pt* h, int32_t inst, int32_t step, doub
   return OTB_OK;
 }
 
-// The sweep of nh systems over process tensor inst: ptab holds n_props
-// propagator pairs (P1 then P2, D * D complex each), pidx (nh * num_steps,
-// host) the pair of system h at step k.  Every index is checked here, on the
-// host, before anything reaches the device.
-static otb_status dyn_run_impl(otb_pt* h, int32_t inst, int32_t nh, const double* ptab, int32_t n_props,
-                               const int32_t* pidx, const double* rho0, int32_t num_steps, double* out,
-                               void* stream) {
+namespace {
+
+// The completed build's bonds (OTB_ERR_INVALID_ARG while it is not complete).
+otb_status completed_dims(otb_pt* h, int32_t inst, std::vector<int2>& dims) {
+  std::lock_guard<std::mutex> lock(h->mutex);
+  if (h->final_dims[inst].empty()) {
+    otb_status st = pt_refresh(h, inst);
+    if (st) return st;
+    if (!h->state[inst].caps_done) return set_error(OTB_ERR_INVALID_ARG, "process tensor not complete");
+    std::vector<int2> d;
+    if ((st = pt_dims(h, inst, d))) return st;
+    h->final_dims[inst] = std::move(d);
+  }
+  dims = h->final_dims[inst];
+  return OTB_OK;
+}
+
+// Device memory of one sweep: the handle's kept workspace when it is free and
+// small enough, else an allocation of its own.
+struct SweepWorkspace {
+  otb_pt* h;
+  std::unique_lock<std::mutex> lock;
+  DevBuf own;
+  char* p = nullptr;
+  explicit SweepWorkspace(otb_pt* h_) : h(h_) {}
+  bool get(size_t bytes) {
+    lock = std::unique_lock<std::mutex>(h->sweep_mutex, std::try_to_lock);
+    if (lock.owns_lock() && bytes <= SWEEP_KEEP_BYTES) {
+      if (h->sweep_ws.bytes < bytes && !h->sweep_ws.alloc(bytes)) return false;
+      p = (char*)h->sweep_ws.p;
+      return true;
+    }
+    if (lock.owns_lock()) lock.unlock();
+    if (!own.alloc(bytes)) return false;
+    p = (char*)own.p;
+    return true;
+  }
+};
+
+struct Layout {
+  size_t total = 0;
+  size_t take(size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) & ~(size_t)255;
+    return at;
+  }
+};
+
+SweepLaunch sweep_launch(otb_pt* h, int32_t inst, int nh, int num_steps, const std::vector<int2>& dims) {
+  const PtDev& I = h->inst[inst];
+  SweepLaunch L{};
+  L.nh = nh;
+  L.D = I.D;
+  L.d = I.d;
+  L.num_steps = num_steps;
+  L.cap = I.cap;
+  L.max_bond = 1;
+  for (int k = 0; k < num_steps; ++k) L.max_bond = std::max(L.max_bond, std::max(dims[k].x, dims[k].y));
+  L.sites = (const double*)h->d_sites.p + 2 * I.site_base;
+  L.slot_elems = (long long)I.cap * I.D * I.cap;
+  L.dims = (const int2*)h->d_dims.p + I.dims_base;
+  L.caps = (const double*)h->d_caps.p + 2 * I.caps_base;
+  return L;
+}
+
+}  // namespace
+
+// The sweep of nh systems over process tensor inst: ptab(h) holds propagator
+// pairs (P1 then P2, D * D complex each), pidx (nh * num_steps, host) the pair
+// of system h at step k (null: pair h at every step; then p2 may hold the
+// second propagators apart from ptab's first ones).  Every index is checked
+// here, on the host, before anything reaches the device.
+static otb_status dyn_run_impl(otb_pt* h, int32_t inst, int32_t nh, const double* ptab, const double* p2,
+                               int32_t n_props, const int32_t* pidx, const double* rho0, int32_t num_steps,
+                               double* out, void* stream) {
   otb_status st = pt_check(h, inst);
   if (st) return st;
   const PtDev& I = h->inst[inst];
   if (!ptab || !rho0 || !out || nh < 1 || nh > 1024 || num_steps < 0 || num_steps > I.num_steps ||
-      n_props < 1 || (num_steps > 0 && !pidx))
+      n_props < 1 || (num_steps > 0 && !pidx && !p2))
     return set_error(OTB_ERR_INVALID_ARG, "bad arguments");
-  for (long long e = 0; e < (long long)nh * num_steps; ++e)
-    if (pidx[e] < 0 || pidx[e] >= n_props)
-      return set_error(OTB_ERR_INVALID_ARG, "propagator index out of range");
-  if ((st = pt_refresh(h, inst))) return st;
-  if (!h->state[inst].caps_done) return set_error(OTB_ERR_INVALID_ARG, "process tensor not complete");
+  if (pidx)
+    for (long long e = 0; e < (long long)nh * num_steps; ++e)
+      if (pidx[e] < 0 || pidx[e] >= n_props)
+        return set_error(OTB_ERR_INVALID_ARG, "propagator index out of range");
   std::vector<int2> dims;
-  if ((st = pt_dims(h, inst, dims))) return st;
+  if ((st = completed_dims(h, inst, dims))) return st;
   const int D = I.D;
-  DevBuf dtab, didx, drho, dv0, dv1, dout;
-  const size_t tb = (size_t)n_props * 2 * D * D * 16, vb = (size_t)nh * I.cap * D * 16;
-  const size_t ib = (size_t)nh * std::max(num_steps, 1) * sizeof(int32_t);
-  const size_t ob = (size_t)(num_steps + 1) * nh * D * 16;
-  const int max_chunks = (I.cap + 31) / 32;
-  DevBuf dpart, dcnt;
-  if (!dtab.alloc(tb) || !didx.alloc(ib) || !drho.alloc((size_t)nh * D * 16) || !dv0.alloc(vb) ||
-      !dv1.alloc(vb) || !dout.alloc(ob) || !dpart.alloc((size_t)nh * max_chunks * D * 16) ||
-      !dcnt.alloc((size_t)nh * sizeof(unsigned int)))
-    return OTB_ERR_OOM;
   cudaStream_t s = (cudaStream_t)stream;
-  if (!check_cuda(cudaMemcpyAsync(dtab.p, ptab, tb, cudaMemcpyHostToDevice, s), "upload") ||
-      (num_steps > 0 &&
-       !check_cuda(cudaMemcpyAsync(didx.p, pidx, (size_t)nh * num_steps * sizeof(int32_t),
-                                   cudaMemcpyHostToDevice, s), "upload")) ||
-      !check_cuda(cudaMemcpyAsync(drho.p, rho0, (size_t)nh * D * 16, cudaMemcpyHostToDevice, s), "upload") ||
-      !check_cuda(cudaMemsetAsync(dout.p, 0, ob, s), "memset") ||
-      !check_cuda(cudaMemsetAsync(dv0.p, 0, vb, s), "memset") ||
-      !check_cuda(cudaMemsetAsync(dcnt.p, 0, (size_t)nh * sizeof(unsigned int), s), "memset"))
-    return OTB_ERR_CUDA;
-  DynLaunch L;
-  L.nh = nh;
-  L.D = D;
-  L.d = I.d;
-  L.sites = (const double*)h->d_sites.p + 2 * I.site_base;
-  L.slot_elems = (long long)I.cap * D * I.cap;
-  L.dims = (const int2*)h->d_dims.p + I.dims_base;
-  L.caps = (const double*)h->d_caps.p + 2 * I.caps_base;
-  L.cap = I.cap;
-  L.ptab = (const double*)dtab.p;
-  L.pidx = (const int*)didx.p;
-  L.pidx_stride = num_steps;
-  L.vcur = (double*)dv0.p;
-  L.vnext = (double*)dv1.p;
-  L.out = (double*)dout.p;
-  L.partial = (double*)dpart.p;
-  L.counter = (unsigned int*)dcnt.p;
-  L.max_chunks = max_chunks;
-  L.k = 0;
-  L.fwd_hist = nullptr;
-  L.back_hist = nullptr;
-  L.deriv = nullptr;
-  L.hist_steps = 0;
-  if (!check_cuda(launch_dyn_init(L, (const double*)drho.p, s), "dyn init")) return OTB_ERR_CUDA;
-  // the whole sweep as one CUDA graph: one kernel node per step
-  cudaStream_t cs;
-  if (!check_cuda(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "stream")) return OTB_ERR_CUDA;
-  cudaEvent_t ready;
-  cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
-  cudaEventRecord(ready, s);
-  cudaStreamWaitEvent(cs, ready, 0);
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  bool ok = check_cuda(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "capture");
-  for (int k = 0; ok && k < num_steps; ++k) {
-    DynLaunch Lk = L;
-    Lk.k = k;
-    Lk.vcur = (k % 2 == 0) ? (double*)dv0.p : (double*)dv1.p;
-    Lk.vnext = (k % 2 == 0) ? (double*)dv1.p : (double*)dv0.p;
-    ok = check_cuda(launch_dyn_step(Lk, dims[k].y, cs), "dyn step");
+  if (num_steps == 0) {
+    // rho(0) = rho0 cap_0
+    double c0[2];
+    if (!check_cuda(cudaMemcpy(c0, (const double*)h->d_caps.p + 2 * I.caps_base, sizeof(c0), cudaMemcpyDeviceToHost),
+                    "read cap"))
+      return OTB_ERR_CUDA;
+    for (int e = 0; e < nh * D; ++e) {
+      const double x = rho0[2 * e], y = rho0[2 * e + 1];
+      out[2 * e] = x * c0[0] - y * c0[1];
+      out[2 * e + 1] = x * c0[1] + y * c0[0];
+    }
+    return OTB_OK;
   }
-  cudaError_t ce = cudaStreamEndCapture(cs, &graph);
-  ok = ok && check_cuda(ce, "end capture");
-  if (ok) ok = check_cuda(cudaGraphInstantiate(&exec, graph, 0), "instantiate");
-  if (ok) ok = check_cuda(cudaGraphLaunch(exec, cs), "graph launch");
-  if (ok) {
-    cudaEventRecord(ready, cs);
-    cudaStreamWaitEvent(s, ready, 0);
-    ok = check_cuda(cudaMemcpyAsync(out, dout.p, ob, cudaMemcpyDeviceToHost, s), "download") &&
-         check_cuda(cudaStreamSynchronize(s), "sync");
+  SweepLaunch L = sweep_launch(h, inst, nh, num_steps, dims);
+  const size_t mat = (size_t)2 * D * D;   // doubles of one D x D complex matrix
+  const size_t tb = (size_t)n_props * 2 * mat * 8, rb = (size_t)nh * D * 16;
+  const size_t ib = pidx ? (size_t)nh * num_steps * sizeof(int32_t) : 0;
+  const size_t ob = (size_t)(num_steps + 1) * nh * D * 16;
+  Layout lay;
+  const size_t o_tab = lay.take(tb), o_rho = lay.take(rb), o_idx = lay.take(ib);
+  const size_t in_bytes = lay.total;
+  const size_t o_q = lay.take((size_t)(pidx ? num_steps : 1) * nh * 2 * mat * 8);
+  const size_t o_b = lay.take((size_t)num_steps * I.cap * D * 16), o_out = lay.take(ob);
+  SweepWorkspace ws(h);
+  if (!ws.get(lay.total)) return OTB_ERR_OOM;
+  // the inputs in one copy
+  std::vector<char> in(in_bytes);
+  if (p2) {
+    for (int i = 0; i < nh; ++i) {
+      std::memcpy(in.data() + o_tab + (size_t)i * 2 * mat * 8, ptab + i * mat, mat * 8);
+      std::memcpy(in.data() + o_tab + ((size_t)i * 2 + 1) * mat * 8, p2 + i * mat, mat * 8);
+    }
+  } else {
+    std::memcpy(in.data() + o_tab, ptab, tb);
   }
-  if (exec) cudaGraphExecDestroy(exec);
-  if (graph) cudaGraphDestroy(graph);
-  cudaEventDestroy(ready);
-  cudaStreamDestroy(cs);
+  std::memcpy(in.data() + o_rho, rho0, rb);
+  if (pidx) std::memcpy(in.data() + o_idx, pidx, ib);
+  L.ptab = (const double*)(ws.p + o_tab);
+  L.rho0 = (const double*)(ws.p + o_rho);
+  L.pidx = pidx ? (const int*)(ws.p + o_idx) : nullptr;
+  L.qtab = (double*)(ws.p + o_q);
+  L.bcol = (double*)(ws.p + o_b);
+  L.out = (double*)(ws.p + o_out);
+  bool ok = check_cuda(cudaMemcpyAsync(ws.p, in.data(), in_bytes, cudaMemcpyHostToDevice, s), "upload") &&
+            check_cuda(launch_sweep_prepare(L, s), "sweep prepare") && check_cuda(launch_sweep(L, s), "sweep") &&
+            check_cuda(cudaMemcpyAsync(out, ws.p + o_out, ob, cudaMemcpyDeviceToHost, s), "download");
+  // the workspace is given back only when nothing on the stream uses it
+  if (!check_cuda(cudaStreamSynchronize(s), "sync")) ok = false;
   return ok ? OTB_OK : OTB_ERR_CUDA;
 }
 
@@ -379,15 +431,15 @@ extern "C" otb_status otb_dyn_session_create(otb_pt* h, int32_t inst, int32_t nh
   otb_status st = pt_check(h, inst);
   if (st) return st;
   if (!rho0 || nh < 1 || nh > 1024) return set_error(OTB_ERR_INVALID_ARG, "bad arguments");
-  if ((st = pt_refresh(h, inst))) return st;
-  if (!h->state[inst].caps_done) return set_error(OTB_ERR_INVALID_ARG, "process tensor not complete");
+  std::vector<int2> dims;
+  if ((st = completed_dims(h, inst, dims))) return st;
   std::unique_ptr<otb_dyn_session> ss(new otb_dyn_session());
   ss->pt = h;
   ss->inst = inst;
   ss->nh = nh;
   const PtDev& I = h->inst[inst];
   ss->num_steps = I.num_steps;
-  if ((st = pt_dims(h, inst, ss->dims))) return st;
+  ss->dims = std::move(dims);
   const int D = I.D;
   const size_t vb = (size_t)nh * I.cap * D * 16;
   const size_t ob = (size_t)(I.num_steps + 1) * nh * D * 16;
@@ -487,83 +539,50 @@ extern "C" otb_status otb_dyn_gradient(otb_pt* h, int32_t inst, int32_t nh, cons
   for (long long e = 0; e < (long long)nh * num_steps; ++e)
     if (prop_index[e] < 0 || prop_index[e] >= n_props)
       return set_error(OTB_ERR_INVALID_ARG, "propagator index out of range");
-  if ((st = pt_refresh(h, inst))) return st;
-  if (!h->state[inst].caps_done) return set_error(OTB_ERR_INVALID_ARG, "process tensor not complete");
   std::vector<int2> dims;
-  if ((st = pt_dims(h, inst, dims))) return st;
+  if ((st = completed_dims(h, inst, dims))) return st;
   // the target carries no bond: the sweep must end where the process tensor's bond closes
   if (dims[num_steps - 1].y != 1)
     return set_error(OTB_ERR_INVALID_ARG, "gradient needs num_steps = the process tensor's length (closed bond)");
-  int max_r = 1;
-  for (int k = 0; k < num_steps; ++k) max_r = std::max(max_r, std::max(dims[k].x, dims[k].y));
+  SweepLaunch L = sweep_launch(h, inst, nh, num_steps, dims);
   const int D = I.D;
-  const size_t tb = (size_t)n_props * 2 * D * D * 16, vb = (size_t)nh * I.cap * D * 16;
+  const size_t mat = (size_t)2 * D * D;
+  const size_t tb = (size_t)n_props * 2 * mat * 8, rb = (size_t)nh * D * 16;
   const size_t ib = (size_t)nh * num_steps * sizeof(int32_t);
   const size_t ob = (size_t)(num_steps + 1) * nh * D * 16;
-  const size_t fb = (size_t)nh * num_steps * I.cap * D * 16;
-  const size_t bb = (size_t)nh * (num_steps + 1) * I.cap * D * 16;
   const size_t cb = (size_t)nh * num_steps * D * D * D * 16;
-  const int max_chunks = (I.cap + 31) / 32;
-  DevBuf dtab, didx, drho, dtgt, dv0, dv1, dout, dpart, dcnt, dfwd, dback, dcore;
-  if (!dtab.alloc(tb) || !didx.alloc(ib) || !drho.alloc((size_t)nh * D * 16) ||
-      !dtgt.alloc((size_t)nh * D * 16) || !dv0.alloc(vb) || !dv1.alloc(vb) || !dout.alloc(ob) ||
-      !dpart.alloc((size_t)nh * max_chunks * D * 16) || !dcnt.alloc((size_t)nh * sizeof(unsigned int)) ||
-      !dfwd.alloc(fb) || !dback.alloc(bb) || !dcore.alloc(cb))
-    return OTB_ERR_OOM;
+  Layout lay;
+  const size_t o_tab = lay.take(tb), o_rho = lay.take(rb), o_tgt = lay.take(rb), o_idx = lay.take(ib);
+  const size_t in_bytes = lay.total;
+  const size_t o_q = lay.take((size_t)num_steps * nh * 2 * mat * 8);
+  const size_t o_b = lay.take((size_t)num_steps * I.cap * D * 16), o_out = lay.take(ob), o_core = lay.take(cb);
+  const size_t o_f = lay.take((size_t)nh * num_steps * I.cap * D * 16);
+  const size_t o_y = lay.take((size_t)nh * (num_steps + 1) * I.cap * D * 16);
+  SweepWorkspace ws(h);
+  if (!ws.get(lay.total)) return OTB_ERR_OOM;
+  std::vector<char> in(in_bytes);
+  std::memcpy(in.data() + o_tab, props, tb);
+  std::memcpy(in.data() + o_rho, rho0, rb);
+  std::memcpy(in.data() + o_tgt, target, rb);
+  std::memcpy(in.data() + o_idx, prop_index, ib);
+  L.ptab = (const double*)(ws.p + o_tab);
+  L.rho0 = (const double*)(ws.p + o_rho);
+  L.pidx = (const int*)(ws.p + o_idx);
+  L.qtab = (double*)(ws.p + o_q);
+  L.bcol = (double*)(ws.p + o_b);
+  L.out = (double*)(ws.p + o_out);
+  L.fwd_hist = (double*)(ws.p + o_f);
+  L.back_hist = (double*)(ws.p + o_y);
+  L.deriv = (double*)(ws.p + o_core);
   cudaStream_t s = (cudaStream_t)stream;
-  if (!check_cuda(cudaMemcpyAsync(dtab.p, props, tb, cudaMemcpyHostToDevice, s), "upload") ||
-      !check_cuda(cudaMemcpyAsync(didx.p, prop_index, ib, cudaMemcpyHostToDevice, s), "upload") ||
-      !check_cuda(cudaMemcpyAsync(drho.p, rho0, (size_t)nh * D * 16, cudaMemcpyHostToDevice, s), "upload") ||
-      !check_cuda(cudaMemcpyAsync(dtgt.p, target, (size_t)nh * D * 16, cudaMemcpyHostToDevice, s), "upload") ||
-      !check_cuda(cudaMemsetAsync(dout.p, 0, ob, s), "memset") ||
-      !check_cuda(cudaMemsetAsync(dv0.p, 0, vb, s), "memset") ||
-      !check_cuda(cudaMemsetAsync(dfwd.p, 0, fb, s), "memset") ||
-      !check_cuda(cudaMemsetAsync(dback.p, 0, bb, s), "memset") ||
-      !check_cuda(cudaMemsetAsync(dcnt.p, 0, (size_t)nh * sizeof(unsigned int), s), "memset"))
-    return OTB_ERR_CUDA;
-  DynLaunch L;
-  L.nh = nh;
-  L.D = D;
-  L.d = I.d;
-  L.sites = (const double*)h->d_sites.p + 2 * I.site_base;
-  L.slot_elems = (long long)I.cap * D * I.cap;
-  L.dims = (const int2*)h->d_dims.p + I.dims_base;
-  L.caps = (const double*)h->d_caps.p + 2 * I.caps_base;
-  L.cap = I.cap;
-  L.ptab = (const double*)dtab.p;
-  L.pidx = (const int*)didx.p;
-  L.pidx_stride = num_steps;
-  L.vcur = (double*)dv0.p;
-  L.vnext = (double*)dv1.p;
-  L.out = (double*)dout.p;
-  L.partial = (double*)dpart.p;
-  L.counter = (unsigned int*)dcnt.p;
-  L.max_chunks = max_chunks;
-  L.k = 0;
-  L.fwd_hist = (double*)dfwd.p;
-  L.back_hist = (double*)dback.p;
-  L.deriv = (double*)dcore.p;
-  L.hist_steps = num_steps;
-  if (!check_cuda(launch_dyn_init(L, (const double*)drho.p, s), "dyn init")) return OTB_ERR_CUDA;
-  for (int k = 0; k < num_steps; ++k) {
-    DynLaunch Lk = L;
-    Lk.k = k;
-    Lk.vcur = (k % 2 == 0) ? (double*)dv0.p : (double*)dv1.p;
-    Lk.vnext = (k % 2 == 0) ? (double*)dv1.p : (double*)dv0.p;
-    if (!check_cuda(launch_dyn_step(Lk, dims[k].y, s), "forward step")) return OTB_ERR_CUDA;
-  }
-  if (!check_cuda(launch_dyn_back_init(L, (const double*)dtgt.p, s), "adjoint init")) return OTB_ERR_CUDA;
-  for (int k = num_steps - 1; k >= 1; --k) {
-    DynLaunch Lk = L;
-    Lk.k = k;
-    if (!check_cuda(launch_dyn_back_step(Lk, dims[k].x, dims[k].y, s), "adjoint step")) return OTB_ERR_CUDA;
-  }
-  if (!check_cuda(launch_dyn_deriv(L, num_steps, max_r, s), "derivative cores")) return OTB_ERR_CUDA;
-  if (!check_cuda(cudaMemcpyAsync(out_states, dout.p, ob, cudaMemcpyDeviceToHost, s), "download") ||
-      !check_cuda(cudaMemcpyAsync(out_cores, dcore.p, cb, cudaMemcpyDeviceToHost, s), "download") ||
-      !check_cuda(cudaStreamSynchronize(s), "sync"))
-    return OTB_ERR_CUDA;
-  return OTB_OK;
+  bool ok = check_cuda(cudaMemcpyAsync(ws.p, in.data(), in_bytes, cudaMemcpyHostToDevice, s), "upload") &&
+            check_cuda(launch_sweep_prepare(L, s), "sweep prepare") && check_cuda(launch_sweep(L, s), "forward sweep") &&
+            check_cuda(launch_sweep_back(L, (const double*)(ws.p + o_tgt), s), "adjoint sweep") &&
+            check_cuda(launch_dyn_deriv(L, s), "derivative cores") &&
+            check_cuda(cudaMemcpyAsync(out_states, ws.p + o_out, ob, cudaMemcpyDeviceToHost, s), "download") &&
+            check_cuda(cudaMemcpyAsync(out_cores, ws.p + o_core, cb, cudaMemcpyDeviceToHost, s), "download");
+  if (!check_cuda(cudaStreamSynchronize(s), "sync")) ok = false;
+  return ok ? OTB_OK : OTB_ERR_CUDA;
 }
 
 extern "C" otb_status otb_dyn_run(otb_pt* h, int32_t inst, int32_t nh, const double* p1, const double* p2,
@@ -572,21 +591,11 @@ extern "C" otb_status otb_dyn_run(otb_pt* h, int32_t inst, int32_t nh, const dou
   if (st) return st;
   if (!p1 || !p2 || nh < 1 || nh > 1024 || num_steps < 0)
     return set_error(OTB_ERR_INVALID_ARG, "bad arguments");
-  const int D = h->inst[inst].D;
-  const size_t dd = (size_t)2 * D * D;   // doubles of one D x D complex matrix
-  std::vector<double> tab((size_t)nh * 2 * dd);
-  for (int i = 0; i < nh; ++i) {
-    std::copy(p1 + i * dd, p1 + (i + 1) * dd, tab.begin() + (size_t)i * 2 * dd);
-    std::copy(p2 + i * dd, p2 + (i + 1) * dd, tab.begin() + (size_t)i * 2 * dd + dd);
-  }
-  std::vector<int32_t> idx((size_t)nh * std::max(num_steps, 1));
-  for (int i = 0; i < nh; ++i)
-    for (int k = 0; k < num_steps; ++k) idx[(size_t)i * num_steps + k] = i;
-  return dyn_run_impl(h, inst, nh, tab.data(), nh, idx.data(), rho0, num_steps, out, stream);
+  return dyn_run_impl(h, inst, nh, p1, p2, nh, nullptr, rho0, num_steps, out, stream);
 }
 
 extern "C" otb_status otb_dyn_run_steps(otb_pt* h, int32_t inst, int32_t nh, const double* props,
                                         int32_t n_props, const int32_t* prop_index, const double* rho0,
                                         int32_t num_steps, double* out, void* stream) {
-  return dyn_run_impl(h, inst, nh, props, n_props, prop_index, rho0, num_steps, out, stream);
+  return dyn_run_impl(h, inst, nh, props, nullptr, n_props, prop_index, rho0, num_steps, out, stream);
 }

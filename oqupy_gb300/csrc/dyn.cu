@@ -20,10 +20,16 @@
 // sum is reproducible bit for bit: a CTA adds its bond chunk's terms in a
 // fixed order, and the last CTA of a system to finish (counted after a
 // memory fence) adds the chunks' partial sums in chunk order.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
 #include "common.cuh"
 #include "engine.h"
 
 namespace otb {
+
+namespace cg = cooperative_groups;
 
 typedef cx<double> zc;
 constexpr int DYN_RB = 32;       // output bond indices per CTA
@@ -44,11 +50,6 @@ __global__ void __launch_bounds__(DYN_THREADS) dyn_step_kernel(DynLaunch L) {
   const zc* v = (const zc*)L.vcur + (long long)h * L.cap * D;
   const zc* P1 = (const zc*)L.ptab + (long long)L.pidx[(long long)h * L.pidx_stride + k] * 2 * D * D;
   const zc* P2 = P1 + D * D;
-  if (L.fwd_hist && blockIdx.x == 0) {
-    // gradient sweep: keep v_k (the state with its bond leg at the start of step k)
-    zc* hv = (zc*)L.fwd_hist + ((long long)h * L.hist_steps + k) * L.cap * D;
-    for (int idx = tid; idx < l * D; idx += nt) hv[idx] = v[idx];
-  }
   for (int idx = tid; idx < l * D; idx += nt) {
     const int ll = idx / D, a = idx - ll * D;
     zc acc = mk<double>(0, 0);
@@ -115,60 +116,380 @@ __global__ void dyn_init_kernel(DynLaunch L, const double* rho0) {
   }
 }
 
-// Adjoint sweep of compute_gradient_and_dynamics (gradient.py:323-425): from
-// Y_{k+1} (bond r) to Y_k (bond l) through the transposed step,
-//     u[r][c]  = sum_e P2_hk[e][c] Y_{k+1}[r][e]
-//     w[l][b]  = sum_r T_k[l][r][b] u[r][b]
-//     Y_k[l][a] = sum_b P1_hk[b][a] w[l][b]
-// with the same propagator pairs as the forward sweep (controls and
-// transforms folded in), so Y_k equals the reference's backward node before
-// the pre-measurement control of step k.  Grid: (chunks of DYN_RB left bond
-// indices, systems); no reduction across CTAs.
-__global__ void __launch_bounds__(DYN_THREADS) dyn_back_step_kernel(DynLaunch L, int l, int r) {
-  extern __shared__ __align__(16) unsigned char dsm[];
-  const int h = blockIdx.y;
-  const int k = L.k;
+// ---------------------------------------------------------------------------
+// Whole sweeps: all steps of a system in one launch
+// ---------------------------------------------------------------------------
+//
+// A system's steps depend on each other but on no other system, so a sweep of
+// N steps is one kernel: a cluster of C CTAs (C = 1 for many systems) carries S
+// systems through all steps and exchanges the new states through distributed
+// shared memory, one cluster barrier per step.  With u_k = P1_k v_k a step is
+//     w[r][a]      = sum_l u_k[l][a] A_k[l][a][r]
+//     u_{k+1}[r]   = Q_k w[r],           Q_k  = d P1_{k+1} P2_k
+//     rho_h(k+1)   = d P2_k y,           y[a] = sum_l u_k[l][a] B_k[l][a],
+//     B_k[l][a]    = sum_r A_k[l][a][r] cap_{k+1}[r]
+// (d P2_k w is the state with its bond leg).  B depends on the process tensor
+// only and enters as one more column r of A_k, which makes the read-out part of
+// the contraction instead of a reduction over r; Q saves one of the two
+// propagator products per step.
+//
+// What bounds it: the FP64 pipe (a warp instruction takes 64 clocks of its
+// scheduler): 4 l r D multiply-adds per step and system, and for few systems
+// the step's chain of dependent phases.  Hence C splits the columns r of few
+// systems over SMs, S lets many systems share every load of A, and a column's
+// sum over l is split over G lanes where a CTA has fewer columns than threads.
+// One launch replaces a graph of N kernel nodes that had to be captured and
+// instantiated per call. Whole calls, 60 steps, bond 13, before and now: 8
+// systems 760 and 290 us, 1024 systems 1750 and 930 us, gradient of 24 driven
+// systems 1610 and 560 us.
+constexpr int SWEEP_THREADS = 256;
+
+__global__ void __launch_bounds__(SWEEP_THREADS) sweep_prepare_kernel(SweepLaunch L) {
   const int D = L.D;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const zc* A = (const zc*)L.sites + (long long)k * L.slot_elems;
-  const zc* P1 = (const zc*)L.ptab + (long long)L.pidx[(long long)h * L.pidx_stride + k] * 2 * D * D;
-  const zc* P2 = P1 + D * D;
-  const zc* Y = (const zc*)L.back_hist + ((long long)h * (L.hist_steps + 1) + k + 1) * L.cap * D;
-  zc* Yk = (zc*)L.back_hist + ((long long)h * (L.hist_steps + 1) + k) * L.cap * D;
-  zc* u = (zc*)dsm;              // r * D
-  zc* w = u + (size_t)r * D;     // DYN_RB * D
-  for (int idx = tid; idx < r * D; idx += nt) {
-    const int rr = idx / D, c = idx - rr * D;
-    zc acc = mk<double>(0, 0);
-    for (int e = 0; e < D; ++e) cfma(acc, P2[e * D + c], Y[rr * D + e]);
-    u[idx] = acc;
+  const int nt = gridDim.y * blockDim.x, t0 = blockIdx.y * blockDim.x + threadIdx.x;
+  const int k = blockIdx.x;
+  // B_k
+  {
+    const int2 dm = L.dims[k];
+    const zc* A = (const zc*)L.sites + (long long)k * L.slot_elems;
+    const zc* capn = (const zc*)L.caps + (long long)(k + 1) * L.cap;
+    zc* B = (zc*)L.bcol + (long long)k * L.cap * D;
+    // eight lanes per entry
+    const int g = t0 & 7;
+    for (int e0 = (t0 >> 3) & ~3; e0 < dm.x * D; e0 += nt >> 3) {   // warp-uniform trip count
+      const int e = e0 + ((t0 >> 3) & 3);
+      zc acc = mk<double>(0, 0);
+      if (e < dm.x * D)
+        for (int rr = g; rr < dm.y; rr += 8) cfma(acc, A[(size_t)e * dm.y + rr], capn[rr]);
+      for (int off = 4; off > 0; off >>= 1) {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, off);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, off);
+      }
+      if (g == 0 && e < dm.x * D) B[e] = acc;
+    }
   }
-  __syncthreads();
-  const int l0 = blockIdx.x * DYN_RB;
-  const int ln = min(DYN_RB, l - l0);
-  for (int idx = tid; idx < ln * D; idx += nt) {
-    const int li = idx / D, b = idx - li * D;
-    const zc* row = A + ((size_t)(l0 + li) * D + b) * r;
+  // Q_k and d P2_k of every system (of step 0 only when they do not change)
+  if (k > 0 && !L.pidx) return;
+  const double d = (double)L.d;
+  for (int idx = t0; idx < L.nh * D * D; idx += nt) {
+    const int h = idx / (D * D), e = idx - h * D * D;
+    const int a = e / D, c = e - a * D;
+    const int i0 = L.pidx ? L.pidx[(long long)h * L.num_steps + k] : h;
+    const int i1 = L.pidx ? L.pidx[(long long)h * L.num_steps + min(k + 1, L.num_steps - 1)] : h;
+    const zc* P2 = (const zc*)L.ptab + ((long long)i0 * 2 + 1) * D * D;
+    const zc* P1n = (const zc*)L.ptab + (long long)i1 * 2 * D * D;
     zc acc = mk<double>(0, 0);
-    for (int rr = 0; rr < r; ++rr) cfma(acc, row[rr], u[rr * D + b]);
-    w[idx] = cscale(acc, (double)L.d);
-  }
-  __syncthreads();
-  for (int idx = tid; idx < ln * D; idx += nt) {
-    const int li = idx / D, a = idx - li * D;
-    zc acc = mk<double>(0, 0);
-    for (int b = 0; b < D; ++b) cfma(acc, P1[b * D + a], w[li * D + b]);
-    Yk[(size_t)(l0 + li) * D + a] = acc;
+    for (int b = 0; b < D; ++b) cfma(acc, P1n[a * D + b], P2[b * D + c]);
+    zc* Q = (zc*)L.qtab + ((long long)(L.pidx ? k : 0) * L.nh + h) * 2 * D * D;
+    Q[e] = cscale(acc, d);
+    Q[D * D + e] = cscale(P2[e], d);
   }
 }
 
-// Y_N = the target (bond 1) for every system.
-__global__ void dyn_back_init_kernel(DynLaunch L, const double* target) {
-  const int h = blockIdx.x;
-  const int D = L.D;
-  zc* Y = (zc*)L.back_hist + ((long long)h * (L.hist_steps + 1) + L.hist_steps) * L.cap * D;
-  const zc* t = (const zc*)target + (long long)h * D;
-  for (int a = threadIdx.x; a < D; a += blockDim.x) Y[a] = t[a];
+// 16-byte asynchronous copy global -> shared.
+__device__ __forceinline__ void copy16(zc* dst, const zc* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+__device__ __forceinline__ void lane_sum(zc& v, int G) {
+  for (int off = G >> 1; off > 0; off >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+  }
+}
+
+// sum_a M[a ms] x[a] over D terms, the terms lane, lane + lg, ...; summed over
+// the lg lanes (1 or 4).
+__device__ __forceinline__ zc row_product(const zc* M, int ms, const zc* x, int D, int lane, int lg, bool act) {
+  zc acc = mk<double>(0, 0);
+  if (act)
+    for (int a = lane; a < D; a += lg) cfma(acc, M[a * ms], x[a]);
+  lane_sum(acc, lg);
+  return acc;
+}
+
+// This CTA's columns of step k, into shared memory: to[(l D + a) nc + cc].
+__device__ __forceinline__ void stage_columns(const SweepLaunch& L, int k, int2 dm, int c0, int nc, zc* to) {
+  const int D = L.D, r = dm.y;
+  const zc* A = (const zc*)L.sites + (long long)k * L.slot_elems + c0;
+  const zc* B = (const zc*)L.bcol + (long long)k * L.cap * D;
+  // one warp per row (no index division: the copies of a step take longer to
+  // address than to make)
+  for (int row = threadIdx.x >> 5; row < dm.x * D; row += SWEEP_THREADS / 32)
+    for (int cc = threadIdx.x & 31; cc < nc; cc += 32)
+      copy16(to + row * nc + cc, c0 + cc == r ? B + row : A + (size_t)row * r + cc);
+}
+
+// S systems per CTA; RECORD keeps v_k (gradient sweeps); DT as below.  With L.stage the next
+// step's columns (and propagators) are copied to shared memory while a step
+// computes: a step waits for no global load.
+template <int S, bool RECORD, int DT>
+__global__ void __launch_bounds__(SWEEP_THREADS) sweep_kernel(SweepLaunch L) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
+  const int D = DT ? DT : L.D, DD = D * D;   // DT: the Liouville dimension, 0 = given at run time
+  const int tid = threadIdx.x;
+  constexpr int nt = SWEEP_THREADS;
+  const int h0 = (int)(blockIdx.x / C) * S;
+  const int ns = min(S, L.nh - h0);
+  const int ustride = L.max_bond * D;               // one system's states
+  const int wstride = L.max_cols * D;               // one system's columns of this CTA
+  zc* const ub = (zc*)dsm;                          // [2][S][max_bond][D]
+  zc* const w = ub + (size_t)2 * S * ustride;       // [S][max_cols][D]
+  zc* const qb = w + (size_t)S * wstride;           // [2][S][2][D][D]
+  zc* const ab = qb + (size_t)4 * S * DD;           // [2][stage]
+  const int N = L.num_steps;
+  auto columns = [&](int2 dm, int& c0, int& nc) {   // [c0, c0 + nc) of the r + 1 (the last one is B)
+    const int per = (dm.y + C) / C;
+    c0 = c * per;
+    nc = max(0, min(per, dm.y + 1 - c0));
+  };
+  auto load_q = [&](int k) {
+    const zc* src = (const zc*)L.qtab + ((long long)(L.pidx ? k : 0) * L.nh + h0) * 2 * DD;
+    zc* dst = qb + (size_t)(k & 1) * 2 * S * DD;
+    for (int idx = tid; idx < ns * 2 * DD; idx += nt) copy16(dst + idx, src + idx);
+  };
+  int2 dm = L.dims[0], dn = N > 1 ? L.dims[1] : dm;
+  int c0, nc;
+  columns(dm, c0, nc);
+  if (L.stage) stage_columns(L, 0, dm, c0, nc, ab);
+  load_q(0);
+  // u_0 = P1_0 rho0, rho(0) = rho0 cap_0
+  for (int idx = tid; idx < ns * D; idx += nt) {
+    const int s = idx / D, a = idx - s * D, h = h0 + s;
+    const zc* P1 = (const zc*)L.ptab + (long long)(L.pidx ? L.pidx[(long long)h * N] : h) * 2 * DD;
+    const zc* r0 = (const zc*)L.rho0 + (long long)h * D;
+    zc acc = mk<double>(0, 0);
+    for (int b = 0; b < D; ++b) cfma(acc, P1[a * D + b], r0[b]);
+    ub[(size_t)s * ustride + a] = acc;
+    if (c == 0) {
+      ((zc*)L.out)[(long long)h * D + a] = cmul(r0[a], ((const zc*)L.caps)[0]);
+      if (RECORD) ((zc*)L.fwd_hist)[(long long)h * N * L.cap * D + a] = r0[a];
+    }
+  }
+  copies_done();
+  cluster.sync();   // also: every CTA of the cluster has started before its shared memory is written
+  for (int k = 0; k < N; ++k) {
+    const int l = dm.x, r = dm.y;
+    const zc* u = ub + (size_t)(k & 1) * S * ustride;
+    zc* un = ub + (size_t)((k + 1) & 1) * S * ustride;
+    const zc* q = qb + (size_t)(L.pidx ? k & 1 : 0) * 2 * S * DD;
+    const zc* as = ab + (size_t)(k & 1) * L.stage;
+    int c0n = 0, ncn = 0;
+    int2 dnn = dn;
+    if (k + 1 < N) {
+      columns(dn, c0n, ncn);
+      if (L.stage) stage_columns(L, k + 1, dn, c0n, ncn, ab + (size_t)((k + 1) & 1) * L.stage);
+      if (L.pidx) load_q(k + 1);
+      if (k + 2 < N) dnn = L.dims[k + 2];
+    }
+    const int outs = nc * D;
+    // G lanes share a column's sum over l where threads are left over
+    int G = 1;
+    while (G < 8 && 2 * G * outs <= nt && 4 * G <= l) G <<= 1;
+    const int g = tid & (G - 1);
+    for (int o0 = 0; o0 < outs; o0 += nt / G) {
+      const int o = o0 + tid / G;
+      const bool act = o < outs;
+      const int cc = act ? o / D : 0, a = act ? o - cc * D : 0;
+      zc acc[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) acc[s] = mk<double>(0, 0);
+      if (act) {
+        const bool last = c0 + cc == r;
+        const zc* col = L.stage ? as + a * nc + cc
+                        : last  ? (const zc*)L.bcol + (long long)k * L.cap * D + a
+                                : (const zc*)L.sites + (long long)k * L.slot_elems + (size_t)a * r + c0 + cc;
+        const size_t step = (size_t)D * (L.stage ? nc : last ? 1 : r);
+        for (int l0 = g; l0 < l; l0 += 4 * G) {
+          zc x[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            if (l0 + t * G < l) x[t] = col[(l0 + t * G) * step];
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            if (l0 + t * G < l) {
+#pragma unroll
+              for (int s = 0; s < S; ++s) cfma(acc[s], u[(size_t)s * ustride + (l0 + t * G) * D + a], x[t]);
+            }
+        }
+      }
+      for (int s = 0; s < S; ++s) lane_sum(acc[s], G);
+      if (act && g == 0)
+#pragma unroll
+        for (int s = 0; s < S; ++s) w[(size_t)s * wstride + cc * D + a] = acc[s];
+    }
+    __syncthreads();
+    // the next states (to every CTA of the cluster) and the read-out
+    const int n2 = ns * outs;
+    const int lg = (D == 4 && 4 * n2 <= nt) ? 4 : 1, lane = tid & (lg - 1);
+    for (int i0 = 0; i0 < n2; i0 += nt / lg) {
+      const int i = i0 + tid / lg;
+      const bool act = i < n2;
+      const int s = act && S > 1 ? i / outs : 0, o = act ? i - s * outs : 0;
+      const int cc = o / D, a = o - cc * D;
+      const bool last = c0 + cc == r;
+      const zc* M = q + (size_t)s * 2 * DD + a * D;
+      const zc* x = w + (size_t)s * wstride + cc * D;
+      const zc y = row_product(last ? M + DD : M, 1, x, D, lane, lg, act);
+      zc vr = y;
+      if (RECORD) vr = row_product(M + DD, 1, x, D, lane, lg, act);   // v_{k+1} = d P2_k w
+      if (act) {
+        if (last) {
+          if (lane == 0) ((zc*)L.out)[((long long)(k + 1) * L.nh + h0 + s) * D + a] = y;
+        } else {
+          zc* dst = un + (size_t)s * ustride + (size_t)(c0 + cc) * D + a;
+          if (C == 1) {
+            if (lane == 0) *dst = y;
+          } else {
+            for (int t = lane; t < C; t += lg) *cluster.map_shared_rank(dst, t) = y;
+          }
+          if (RECORD && lane == 0 && k + 1 < N)
+            ((zc*)L.fwd_hist)[(((long long)(h0 + s) * N + k + 1) * L.cap + c0 + cc) * D + a] = vr;
+        }
+      }
+    }
+    copies_done();
+    if (C == 1)
+      __syncthreads();
+    else
+      cluster.sync();
+    dm = dn;
+    dn = dnn;
+    c0 = c0n;
+    nc = ncn;
+  }
+}
+
+// Adjoint sweep of compute_gradient_and_dynamics (gradient.py:323-425): from
+// Y_{k+1} (bond r) to Y_k (bond l) through the transposed step,
+//     w[l][b]   = sum_r A_k[l][b][r] z[r][b],   z[r][c] = d sum_e P2_k[e][c] Y_{k+1}[r][e]
+//     Y_k[l][a] = sum_b P1_k[b][a] w[l][b]
+// with the same propagator pairs as the forward sweep (controls and
+// transforms folded in), so Y_k equals the reference's backward node before
+// the pre-measurement control of step k.  As sweep_kernel, one system per
+// cluster; the next z is (Q_{k-1})^T w.
+template <int DT>
+__global__ void __launch_bounds__(SWEEP_THREADS) sweep_back_kernel(SweepLaunch L, const double* target) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
+  const int D = DT ? DT : L.D, DD = D * D;
+  const int tid = threadIdx.x;
+  constexpr int nt = SWEEP_THREADS;
+  const int h = (int)(blockIdx.x / C);
+  const int zstride = L.max_bond * D;
+  zc* const zb = (zc*)dsm;                           // [2][max_bond][D]
+  zc* const w = zb + (size_t)2 * zstride;            // [max_cols][D]
+  zc* const qb = w + (size_t)L.max_cols * D;         // [2][P1_k, Q_{k-1}][D][D]
+  zc* const ab = qb + (size_t)4 * DD;                // [2][stage]
+  const int N = L.num_steps;
+  zc* const Y = (zc*)L.back_hist + (long long)h * (N + 1) * L.cap * D;
+  auto q_of = [&](int k) { return (const zc*)L.qtab + ((long long)(L.pidx ? k : 0) * L.nh + h) * 2 * DD; };
+  auto rows = [&](int2 dm, int& l0, int& nl) {       // this CTA's rows [l0, l0 + nl) of the l
+    const int per = (dm.x + C - 1) / C;
+    l0 = c * per;
+    nl = max(0, min(per, dm.x - l0));
+  };
+  auto prefetch = [&](int k, int2 dm, int l0, int nl) {
+    const zc* P1 = (const zc*)L.ptab + (long long)(L.pidx ? L.pidx[(long long)h * N + k] : h) * 2 * DD;
+    const zc* Qp = q_of(k - 1);
+    zc* qd = qb + (size_t)(k & 1) * 2 * DD;
+    for (int idx = tid; idx < DD; idx += nt) {
+      copy16(qd + idx, P1 + idx);
+      copy16(qd + DD + idx, Qp + idx);
+    }
+    if (L.stage) {
+      const zc* A = (const zc*)L.sites + (long long)k * L.slot_elems + (size_t)l0 * D * dm.y;
+      zc* to = ab + (size_t)(k & 1) * L.stage;
+      for (int e = tid; e < nl * D * dm.y; e += nt) copy16(to + e, A + e);
+    }
+  };
+  int2 dm = L.dims[N - 1], dn = N > 1 ? L.dims[N - 2] : dm;
+  int l0, nl;
+  rows(dm, l0, nl);
+  if (N > 1) prefetch(N - 1, dm, l0, nl);
+  // z_{N-1} = d P2_{N-1}^T target (bond 1)
+  for (int a = tid; a < D; a += nt) {
+    const zc* t = (const zc*)target + (long long)h * D;
+    const zc* P2d = q_of(N - 1) + DD;
+    zc acc = mk<double>(0, 0);
+    for (int e = 0; e < D; ++e) cfma(acc, P2d[e * D + a], t[e]);
+    zb[(size_t)((N - 1) & 1) * zstride + a] = acc;
+    if (c == 0) Y[(long long)N * L.cap * D + a] = t[a];
+  }
+  copies_done();
+  cluster.sync();
+  for (int k = N - 1; k >= 1; --k) {
+    const int r = dm.y;
+    const zc* z = zb + (size_t)(k & 1) * zstride;
+    zc* zn = zb + (size_t)((k - 1) & 1) * zstride;
+    const zc* q = qb + (size_t)(k & 1) * 2 * DD;
+    int l0n = 0, nln = 0;
+    int2 dnn = dn;
+    if (k > 1) {
+      rows(dn, l0n, nln);
+      prefetch(k - 1, dn, l0n, nln);
+      if (k > 2) dnn = L.dims[k - 2];
+    }
+    const zc* base = L.stage ? ab + (size_t)(k & 1) * L.stage
+                             : (const zc*)L.sites + (long long)k * L.slot_elems + (size_t)l0 * D * r;
+    const int outs = nl * D;
+    int G = 1;
+    while (G < 8 && 2 * G * outs <= nt && 4 * G <= r) G <<= 1;
+    const int g = tid & (G - 1);
+    for (int o0 = 0; o0 < outs; o0 += nt / G) {
+      const int o = o0 + tid / G;
+      const bool act = o < outs;
+      zc acc = mk<double>(0, 0);
+      if (act) {
+        const int b = o % D;
+        const zc* row = base + (size_t)o * r;
+        for (int r0 = g; r0 < r; r0 += 4 * G) {
+          zc x[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            if (r0 + t * G < r) x[t] = row[r0 + t * G];
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            if (r0 + t * G < r) cfma(acc, x[t], z[(r0 + t * G) * D + b]);
+        }
+      }
+      lane_sum(acc, G);
+      if (act && g == 0) w[o] = acc;
+    }
+    __syncthreads();
+    const int lg = (D == 4 && 8 * outs <= nt) ? 4 : 1, lane = tid & (lg - 1);
+    for (int o0 = 0; o0 < 2 * outs; o0 += nt / lg) {
+      const int o = o0 + tid / lg;
+      const bool act = o < 2 * outs, next = o >= outs;
+      const int i = act ? (next ? o - outs : o) : 0;
+      const int li = i / D, a = i - li * D;
+      const zc acc = row_product(q + (next ? DD : 0) + a, D, w + li * D, D, lane, lg, act);
+      if (act && next) {
+        zc* dst = zn + (size_t)(l0 + li) * D + a;
+        if (C == 1) {
+          if (lane == 0) *dst = acc;
+        } else {
+          for (int t = lane; t < C; t += lg) *cluster.map_shared_rank(dst, t) = acc;
+        }
+      } else if (act && lane == 0) {
+        Y[((long long)k * L.cap + l0 + li) * D + a] = acc;
+      }
+    }
+    copies_done();
+    if (C == 1)
+      __syncthreads();
+    else
+      cluster.sync();
+    dm = dn;
+    dn = dnn;
+    l0 = l0n;
+    nl = nln;
+  }
 }
 
 // Derivative cores: for every step n and system h,
@@ -179,7 +500,7 @@ __global__ void dyn_back_init_kernel(DynLaunch L, const double* target) {
 // post-measurement control of step n on leg a, the pre-measurement control
 // of step n+1 on leg e, the process tensor's transforms on the MPO legs).
 // Grid: (steps, systems).
-__global__ void __launch_bounds__(DYN_THREADS) dyn_deriv_kernel(DynLaunch L) {
+__global__ void __launch_bounds__(DYN_THREADS) dyn_deriv_kernel(SweepLaunch L) {
   extern __shared__ __align__(16) unsigned char dsm[];
   const int n = blockIdx.x;
   const int h = blockIdx.y;
@@ -188,8 +509,8 @@ __global__ void __launch_bounds__(DYN_THREADS) dyn_deriv_kernel(DynLaunch L) {
   const int2 dm = L.dims[n];
   const int l = dm.x, r = dm.y;
   const zc* A = (const zc*)L.sites + (long long)n * L.slot_elems;
-  const zc* v = (const zc*)L.fwd_hist + ((long long)h * L.hist_steps + n) * L.cap * D;
-  const zc* Y = (const zc*)L.back_hist + ((long long)h * (L.hist_steps + 1) + n + 1) * L.cap * D;
+  const zc* v = (const zc*)L.fwd_hist + ((long long)h * L.num_steps + n) * L.cap * D;
+  const zc* Y = (const zc*)L.back_hist + ((long long)h * (L.num_steps + 1) + n + 1) * L.cap * D;
   zc* X = (zc*)dsm;   // r * D * D
   for (int idx = tid; idx < r * D * D; idx += nt) {
     const int rr = idx / (D * D), am = idx - rr * D * D;
@@ -199,7 +520,7 @@ __global__ void __launch_bounds__(DYN_THREADS) dyn_deriv_kernel(DynLaunch L) {
     X[idx] = cscale(acc, (double)L.d);
   }
   __syncthreads();
-  zc* out = (zc*)L.deriv + ((long long)h * L.hist_steps + n) * D * D * D;
+  zc* out = (zc*)L.deriv + ((long long)h * L.num_steps + n) * D * D * D;
   for (int idx = tid; idx < D * D * D; idx += nt) {
     const int a = idx / (D * D), me = idx - a * D * D;
     const int m = me / D, e = me - m * D;
@@ -209,24 +530,113 @@ __global__ void __launch_bounds__(DYN_THREADS) dyn_deriv_kernel(DynLaunch L) {
   }
 }
 
-cudaError_t launch_dyn_back_init(const DynLaunch& L, const double* target, cudaStream_t stream) {
-  dyn_back_init_kernel<<<L.nh, 32, 0, stream>>>(L, target);
+// Shape of a sweep: systems per CTA, CTAs per cluster, dynamic shared memory.
+// Many systems: one CTA per SM with its share of them (every load of A serves
+// all of a CTA's systems).  Few: the step's columns are split over up to eight
+// CTAs while a CTA's FP64 work of a step (2 l r D clocks on one SM) is above
+// 3000 clocks: the exchange through the cluster costs about 1000, and below
+// that a step's fixed chain of phases (about 6000 clocks) hides what is saved
+// (8 systems, bond 13: 200 us a sweep on one CTA each, 175 us on eight).
+struct SweepShape {
+  int S, C, max_cols;
+  size_t stage;   // elements of one staging buffer, 0 = columns read from global memory
+  size_t smem;
+};
+
+static SweepShape sweep_shape(const SweepLaunch& L, int max_s) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  sms = sms > 0 ? sms : 1;
+  SweepShape sh;
+  const double clocks = 2.0 * L.max_bond * L.max_bond * L.D;
+  sh.C = 1;
+  while (sh.C < 8 && 2 * sh.C * L.nh <= sms && clocks > 3000.0 * sh.C) sh.C *= 2;
+  sh.S = sh.C > 1 ? 1 : std::min(max_s, (L.nh + sms - 1) / sms);
+  const size_t limit = 200 * 1024;
+  for (;; --sh.S) {
+    sh.max_cols = (L.max_bond + sh.C) / sh.C;
+    sh.smem = ((size_t)2 * sh.S * L.max_bond * L.D + (size_t)sh.S * sh.max_cols * L.D +
+               (size_t)4 * sh.S * L.D * L.D) * sizeof(zc);
+    if (sh.smem <= limit || sh.S == 1) break;
+  }
+  sh.stage = (size_t)L.max_bond * L.D * sh.max_cols;
+  if (sh.smem + 2 * sh.stage * sizeof(zc) <= limit)
+    sh.smem += 2 * sh.stage * sizeof(zc);
+  else
+    sh.stage = 0;
+  return sh;
+}
+
+template <typename K, typename... Args>
+static cudaError_t launch_clusters(K kernel, int ctas, int C, size_t smem, cudaStream_t stream, Args... args) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(SWEEP_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+cudaError_t launch_sweep_prepare(const SweepLaunch& L, cudaStream_t stream) {
+  // enough CTAs per step for its columns; step 0's also form the propagators
+  const int y = std::max(1, std::min(64, std::max((L.cap * L.D * 8) / SWEEP_THREADS / 4,
+                                                  (L.nh * L.D * L.D + SWEEP_THREADS - 1) / SWEEP_THREADS / 2)));
+  sweep_prepare_kernel<<<dim3(L.num_steps, y), SWEEP_THREADS, 0, stream>>>(L);
   return cudaGetLastError();
 }
 
-cudaError_t launch_dyn_back_step(const DynLaunch& L, int l, int r, cudaStream_t stream) {
-  const int chunks = (l + DYN_RB - 1) / DYN_RB;
-  const size_t smem = (size_t)(r * L.D + DYN_RB * L.D) * sizeof(zc);
-  dim3 grid(chunks, L.nh);
-  dyn_back_step_kernel<<<grid, DYN_THREADS, smem, stream>>>(L, l, r);
-  return cudaGetLastError();
+cudaError_t launch_sweep(const SweepLaunch& L0, cudaStream_t stream) {
+  SweepLaunch L = L0;
+  SweepShape sh = sweep_shape(L, L.fwd_hist ? 1 : L.D == 4 ? 8 : 4);
+  if (L.D != 4 && sh.S == 3) sh = sweep_shape(L, 2);   // built for 1, 2 and 4 systems
+  L.max_cols = sh.max_cols;
+  L.stage = (long long)sh.stage;
+  const int ctas = (L.nh + sh.S - 1) / sh.S * sh.C;
+  if (L.D == 4) {
+    if (L.fwd_hist) return launch_clusters(sweep_kernel<1, true, 4>, ctas, sh.C, sh.smem, stream, L);
+    switch (sh.S) {
+      case 1: return launch_clusters(sweep_kernel<1, false, 4>, ctas, sh.C, sh.smem, stream, L);
+      case 2: return launch_clusters(sweep_kernel<2, false, 4>, ctas, sh.C, sh.smem, stream, L);
+      case 3: return launch_clusters(sweep_kernel<3, false, 4>, ctas, sh.C, sh.smem, stream, L);
+      case 4: return launch_clusters(sweep_kernel<4, false, 4>, ctas, sh.C, sh.smem, stream, L);
+      case 5: return launch_clusters(sweep_kernel<5, false, 4>, ctas, sh.C, sh.smem, stream, L);
+      case 6: return launch_clusters(sweep_kernel<6, false, 4>, ctas, sh.C, sh.smem, stream, L);
+      case 7: return launch_clusters(sweep_kernel<7, false, 4>, ctas, sh.C, sh.smem, stream, L);
+      default: return launch_clusters(sweep_kernel<8, false, 4>, ctas, sh.C, sh.smem, stream, L);
+    }
+  }
+  if (L.fwd_hist) return launch_clusters(sweep_kernel<1, true, 0>, ctas, sh.C, sh.smem, stream, L);
+  switch (sh.S) {
+    case 1: return launch_clusters(sweep_kernel<1, false, 0>, ctas, sh.C, sh.smem, stream, L);
+    case 2: return launch_clusters(sweep_kernel<2, false, 0>, ctas, sh.C, sh.smem, stream, L);
+    default: return launch_clusters(sweep_kernel<4, false, 0>, ctas, sh.C, sh.smem, stream, L);
+  }
 }
 
-cudaError_t launch_dyn_deriv(const DynLaunch& L, int num_steps, int max_r, cudaStream_t stream) {
-  const size_t smem = (size_t)max_r * L.D * L.D * sizeof(zc);
+cudaError_t launch_sweep_back(const SweepLaunch& L0, const double* target, cudaStream_t stream) {
+  SweepLaunch L = L0;
+  const SweepShape sh = sweep_shape(L, 1);
+  L.max_cols = sh.max_cols;
+  L.stage = (long long)sh.stage;
+  return L.D == 4 ? launch_clusters(sweep_back_kernel<4>, L.nh * sh.C, sh.C, sh.smem, stream, L, target)
+                  : launch_clusters(sweep_back_kernel<0>, L.nh * sh.C, sh.C, sh.smem, stream, L, target);
+}
+
+cudaError_t launch_dyn_deriv(const SweepLaunch& L, cudaStream_t stream) {
+  const size_t smem = (size_t)L.max_bond * L.D * L.D * sizeof(zc);
   cudaError_t e = cudaFuncSetAttribute(dyn_deriv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  dim3 grid(num_steps, L.nh);
+  dim3 grid(L.num_steps, L.nh);
   dyn_deriv_kernel<<<grid, DYN_THREADS, smem, stream>>>(L);
   return cudaGetLastError();
 }

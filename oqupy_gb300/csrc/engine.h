@@ -150,17 +150,39 @@ struct DynLaunch {
   unsigned int* counter;  // nh counters of finished chunks (zero between steps)
   int max_chunks;
   int k;                // step
-  // gradient sweeps (otb_dyn_gradient; null / unused otherwise)
-  double* fwd_hist;     // nh * hist_steps * cap * D: v_k at the start of step k
-  double* back_hist;    // nh * (hist_steps + 1) * cap * D: adjoint vectors Y_k
-  double* deriv;        // nh * hist_steps * D^3: per-step derivative cores
-  int hist_steps;
+};
+
+// A whole sweep of nh systems over num_steps steps.
+struct SweepLaunch {
+  int nh;
+  int D;
+  int d;
+  int num_steps;
+  int cap;              // bond capacity of the process tensor's slots
+  int max_bond;         // largest bond of the swept steps
+  int max_cols;         // columns of a step per CTA (set at launch)
+  long long stage;      // elements of a staging buffer in shared memory (set at launch; 0: none)
+  const double* sites;  // as in DynLaunch
+  long long slot_elems;
+  const int2* dims;
+  const double* caps;
+  const double* ptab;   // propagator pairs (P1 then P2)
+  const int* pidx;      // nh * num_steps: pair of system h at step k; null: pair h throughout
+  const double* rho0;   // nh * D
+  double* qtab;         // per step (one only when pidx is null) and system: Q, d P2
+  double* bcol;         // num_steps * cap * D: read-out columns
+  double* out;          // (num_steps + 1) * nh * D
+  // gradient sweeps (null otherwise)
+  double* fwd_hist;     // nh * num_steps * cap * D: v_k at the start of step k
+  double* back_hist;    // nh * (num_steps + 1) * cap * D: adjoint vectors Y_k
+  double* deriv;        // nh * num_steps * D^3: per-step derivative cores
 };
 
 cudaError_t launch_dyn_step(const DynLaunch& L, int r, cudaStream_t stream);
 cudaError_t launch_dyn_init(const DynLaunch& L, const double* rho0, cudaStream_t stream);
-cudaError_t launch_dyn_back_init(const DynLaunch& L, const double* target, cudaStream_t stream);
-cudaError_t launch_dyn_back_step(const DynLaunch& L, int l, int r, cudaStream_t stream);
-cudaError_t launch_dyn_deriv(const DynLaunch& L, int num_steps, int max_r, cudaStream_t stream);
+cudaError_t launch_sweep_prepare(const SweepLaunch& L, cudaStream_t stream);
+cudaError_t launch_sweep(const SweepLaunch& L, cudaStream_t stream);
+cudaError_t launch_sweep_back(const SweepLaunch& L, const double* target, cudaStream_t stream);
+cudaError_t launch_dyn_deriv(const SweepLaunch& L, cudaStream_t stream);
 
 }  // namespace otb
