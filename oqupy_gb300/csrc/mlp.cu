@@ -3,8 +3,9 @@
 //
 //   C[M][N] = A[M][K] * B[N][K]^T      A, B bf16, K contiguous ("K-major")
 //
-// One CTA (128 threads) computes a 128 x 128 tile.  Per 64-wide K chunk the
-// CTA stages A and B into shared memory in the canonical no-swizzle K-major
+// Operands with 16-byte aligned rows go through tc_gemm_tma_kernel (below),
+// others through tc_gemm_pipe_kernel: one CTA (128 threads) computes a 128 x
+// 128 tile.  Per 64-wide K chunk the CTA stages A and B into shared memory in the canonical no-swizzle K-major
 // layout of the 5th-generation tensor core -- 8-row x 16-byte core matrices,
 // the two core matrices of a 16-deep K step 128 B apart (leading byte
 // offset), successive 8-row groups 1024 B apart (stride byte offset) -- and
@@ -14,9 +15,12 @@
 // records an error, still frees its TMEM and returns.  The epilogue reads the
 // accumulator with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31 = tile
 // rows) and applies the fused bias / GELU / GELU-gradient step.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "../../include/oqupy_gb300.h"
 #include "capi_util.h"
@@ -57,35 +61,11 @@ __device__ __forceinline__ float gelu_grad_f(float x) {
   return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
-// stage a 128 x 64 bf16 tile (rows r0.., k k0..) of a row-major [R][K]
-// matrix into the core-matrix layout: core (rg, kg) at (rg * 8 + kg) * 128 B
-__device__ __forceinline__ void stage_tile(unsigned char* dst, const __nv_bfloat16* src, int R, int K,
-                                           int r0, int k0) {
-  for (int chunk = threadIdx.x; chunk < TC_BM * (TC_BK / 8); chunk += blockDim.x) {
-    const int rr = chunk / (TC_BK / 8), kc = chunk % (TC_BK / 8);
-    const int row = r0 + rr, kk = k0 + kc * 8;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (row < R) {
-      const __nv_bfloat16* p = src + (size_t)row * K + kk;
-      if (kk + 8 <= K && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
-        v = *reinterpret_cast<const uint4*>(p);
-      } else {
-        union {
-          uint4 u;
-          __nv_bfloat16 h[8];
-        } tmp;
-        for (int e = 0; e < 8; ++e) tmp.h[e] = (kk + e < K) ? p[e] : __float2bfloat16(0.f);
-        v = tmp.u;
-      }
-    }
-    const int rg = rr >> 3, r8 = rr & 7;
-    *reinterpret_cast<uint4*>(dst + (size_t)(rg * (TC_BK / 8) + kc) * 128 + r8 * 16) = v;
-  }
-}
-
-// Same tile as stage_tile, with 16-byte cp.async copies (global -> shared,
-// no register round trip) for every aligned full chunk; ragged or unaligned
-// chunks (K % 8 != 0, tile edges) are zero-padded through registers.
+// Stages a 128 x 64 bf16 tile (rows r0.., k k0..) of a row-major [R][K] matrix
+// into the core-matrix layout, core (rg, kg) at (rg * 8 + kg) * 128 B: 16-byte
+// cp.async copies (no register round trip) for every aligned full chunk;
+// ragged or unaligned chunks (K % 8 != 0, tile edges) are zero-padded through
+// registers.
 __device__ __forceinline__ void stage_tile_async(unsigned char* dst, const __nv_bfloat16* src, int R, int K,
                                                  int r0, int k0) {
   for (int chunk = threadIdx.x; chunk < TC_BM * (TC_BK / 8); chunk += blockDim.x) {
@@ -110,6 +90,86 @@ __device__ __forceinline__ void stage_tile_async(unsigned char* dst, const __nv_
   }
 }
 
+struct GemmOut {
+  const float* bias;
+  const float* zin;
+  float* zout;
+  float* outf;
+  __nv_bfloat16* outb;
+  int ldf;   // row stride of zin, zout and outf
+  int ldb;   // row stride of outb
+  int epi;
+};
+
+// 16 consecutive outputs of one row, in the widest stores the address allows.
+__device__ __forceinline__ void store16(float* p, const float* v, int n) {
+  if (n == 16 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      reinterpret_cast<float4*>(p)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+      if (q < n) p[q] = v[q];
+  }
+}
+__device__ __forceinline__ void store16(__nv_bfloat16* p, const float* v, int n) {
+  if (n == 16 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    union {
+      uint4 u[2];
+      __nv_bfloat162 h[8];
+    } t;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t.h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+    reinterpret_cast<uint4*>(p)[0] = t.u[0];
+    reinterpret_cast<uint4*>(p)[1] = t.u[1];
+  } else {
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+      if (q < n) p[q] = __float2bfloat16(v[q]);
+  }
+}
+
+// 16 accumulators of one row through the fused step.
+__device__ __forceinline__ void epilogue16(const GemmOut& o, const uint32_t* r, size_t row, int col, int n) {
+  float v[16];
+  const size_t at = row * o.ldf + col;
+  if (o.epi == EPI_GELU_GRAD) {
+    const float* z = o.zin + at;
+    float zz[16];
+    if (n == 16 && (reinterpret_cast<uintptr_t>(z) & 15) == 0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 t = reinterpret_cast<const float4*>(z)[q];
+        zz[4 * q] = t.x;
+        zz[4 * q + 1] = t.y;
+        zz[4 * q + 2] = t.z;
+        zz[4 * q + 3] = t.w;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) zz[q] = q < n ? z[q] : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]) * gelu_grad_f(zz[q]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
+    if (o.bias) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q)
+        if (q < n) v[q] += __ldg(o.bias + col + q);
+    }
+    if (o.epi == EPI_GELU) {
+      if (o.zout) store16(o.zout + at, v, n);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) v[q] = gelu_f(v[q]);
+    }
+  }
+  if (o.outf) store16(o.outf + at, v, n);
+  if (o.outb) store16(o.outb + row * o.ldb + col, v, n);
+}
+
 __device__ __forceinline__ bool tc_wait_phase(uint64_t* mbar, int phase) {
   uint32_t done = 0;
   for (long long it = 0; it < TC_WAIT_LIMIT && !done; ++it) {
@@ -122,8 +182,7 @@ __device__ __forceinline__ bool tc_wait_phase(uint64_t* mbar, int phase) {
   return done != 0;
 }
 
-// Two-stage pipeline version of tc_gemm_kernel: while the tensor core runs
-// the four MMAs of chunk k, the CTA's cp.async copies of chunk k+1 land in
+// Two-stage pipeline: while the tensor core runs the four MMAs of chunk k, the CTA's cp.async copies of chunk k+1 land in
 // the other buffer.  A buffer is refilled only after the mbarrier reports
 // the MMAs that read it complete (at most one MMA batch is outstanding at
 // any wait, so the phase parity identifies it).  All waits are bounded.
@@ -214,6 +273,7 @@ __global__ void __launch_bounds__(TC_THREADS)
   asm volatile("tcgen05.fence::after_thread_sync;");
 
   if (!s_err) {
+    const GemmOut o{bias, zin, zout, outf, outb, N, N, epi};
     const int row = m0 + warp * 32 + lane;
     for (int c0 = 0; c0 < TC_BN; c0 += 16) {
       uint32_t r[16];
@@ -224,25 +284,7 @@ __global__ void __launch_bounds__(TC_THREADS)
             "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
           : "r"(taddr));
       asm volatile("tcgen05.wait::ld.sync.aligned;");
-      if (row < M) {
-        for (int j = 0; j < 16; ++j) {
-          const int col = n0 + c0 + j;
-          if (col >= N) break;
-          float v = __uint_as_float(r[j]);
-          const size_t o = (size_t)row * N + col;
-          if (epi == EPI_GELU_GRAD) {
-            v *= gelu_grad_f(zin[o]);
-          } else {
-            if (bias) v += bias[col];
-            if (epi == EPI_GELU) {
-              if (zout) zout[o] = v;
-              v = gelu_f(v);
-            }
-          }
-          if (outf) outf[o] = v;
-          if (outb) outb[o] = __float2bfloat16(v);
-        }
-      }
+      if (row < M && n0 + c0 < N) epilogue16(o, r, (size_t)row, n0 + c0, min(16, N - n0 - c0));
     }
   } else if (tid == 0) {
     atomicExch(err, 1);
@@ -258,120 +300,226 @@ __global__ void __launch_bounds__(TC_THREADS)
   }
 }
 
-__global__ void __launch_bounds__(TC_THREADS)
-    tc_gemm_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, int M,
-                   int N, int K, const float* __restrict__ bias, int epi, const float* __restrict__ zin,
-                   float* __restrict__ zout, float* __restrict__ outf, __nv_bfloat16* __restrict__ outb,
-                   int* __restrict__ err) {
-  __shared__ __align__(1024) unsigned char sA[TC_BM * TC_BK * 2];
-  __shared__ __align__(1024) unsigned char sB[TC_BN * TC_BK * 2];
-  __shared__ __align__(8) uint64_t mbar;
-  __shared__ uint32_t tmem_base;
-  __shared__ int s_err;
-  __shared__ int s_drain;  // phase parity of an MMA batch still in flight after a timed-out wait
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * TC_BM, n0 = blockIdx.x * TC_BN;
+// ---------------------------------------------------------------------------
+// TMA-fed persistent GEMM
+// ---------------------------------------------------------------------------
+//
+// Every CTA (one per SM) walks over 128 x BN tiles: one warp issues the TMA
+// loads of 64-deep K chunks into a ring of shared-memory stages (128-byte
+// swizzle), one thread issues the tcgen05.mma, eight warps run the epilogue
+// from TMEM, where two accumulators let the next tile's products overlap it.
+// Either operand may be stored K-contiguous ([rows][K]) or transposed
+// ([K][rows], the tensor core's MN-major layout), so that weight gradients read
+// activations and their gradients as they lie.
+//
+// What bounds it: for the hidden layers the epilogue's FP32 issue (GELU: about
+// 45 instructions an output, eight warps), for a wide output layer the FP32
+// result's write to memory.  The two-stage kernel above (cp.async staging by
+// the warps that also issue the products and run the epilogue, scalar stores)
+// reached 79 TFLOP/s on a 60001-point inference of a 5-512x4-1500 network
+// (2370 us); with this one the inference takes 492 us.
+//
+// Used when rows are 16-byte aligned; other operands keep the kernel above.
+// Tile width: 256 where that gives every SM a tile, else 128, else 64 (a
+// training step's products have few tiles, and are bound by one tile's chain).
+constexpr int TM_BM = 128, TM_BK = 64;
+constexpr int TM_EPI_WARPS = 8;
+constexpr int TM_THREADS = 64 + 32 * TM_EPI_WARPS;
+constexpr unsigned long long TM_WAIT_NS = 2000000000ull;
 
-  if (warp == 0) {
+template <int BN>
+struct TmShape {
+  static constexpr int stages = BN == 256 ? 4 : 6;
+  static constexpr int a_bytes = TM_BM * TM_BK * 2;
+  static constexpr int b_bytes = BN * TM_BK * 2;
+  static constexpr int smem = stages * (a_bytes + b_bytes) + 1024;   // + alignment
+  static constexpr int tmem_cols = 2 * BN;
+};
+
+// shared-memory matrix descriptor, 128-byte swizzle; K-major: 8-row groups
+// 1024 B apart; MN-major: 64-wide column blocks 8192 B apart (64 K rows of 128
+// B each), 8-row K groups 1024 B apart
+__device__ __forceinline__ uint64_t swizzled_desc(uint32_t saddr, bool mn_major) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)((mn_major ? 8192 : 16) >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
+__device__ __forceinline__ void tma_load(const CUtensorMap* map, uint64_t* bar, uint32_t dst, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+      "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      : "memory");
+}
+
+// Wait bounded to TM_WAIT_NS, which also ends when another role has given up.
+__device__ __forceinline__ bool tm_wait(uint64_t* bar, int parity, volatile int* abort) {
+  unsigned long long t0 = 0, t;
+  for (int it = 0;; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (*abort) return false;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    if (it == 0) t0 = t;
+    if (t - t0 > TM_WAIT_NS) break;
+  }
+  *abort = 1;
+  return false;
+}
+
+// Waits (bounded) for the last use of every stage after `used` uses in turn.
+__device__ __forceinline__ void tm_drain(uint64_t* bars, int stages, int used) {
+  for (int st = 0; st < stages && st < used; ++st) {
+    int never = 0;
+    tm_wait(&bars[st], ((used - st + stages - 1) / stages - 1) & 1, &never);
+  }
+}
+
+__device__ __forceinline__ void tm_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+template <int BN>
+__global__ void __launch_bounds__(TM_THREADS, 1)
+    tc_gemm_tma_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int M, int N,
+                       int K, int ta, int tb, GemmOut out, int* __restrict__ err) {
+  typedef TmShape<BN> Sh;
+  extern __shared__ unsigned char tm_raw[];
+  __shared__ __align__(8) uint64_t full[Sh::stages], empty[Sh::stages], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_base;
+  __shared__ int abort_flag;
+  const uint32_t base = (smem_u32(tm_raw) + 1023u) & ~1023u;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                 "r"(TC_BN));
+                 "r"(Sh::tmem_cols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)));
+    for (int i = 0; i < Sh::stages; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[i])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[i])));
+    }
+    for (int i = 0; i < 2; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_full[i])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acc_empty[i])), "r"(TM_EPI_WARPS));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;");
-    s_err = 0;
-    s_drain = -1;
+    abort_flag = 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base;
-  const uint32_t idesc = make_idesc(TC_BM, TC_BN);
+  volatile int* const stop = &abort_flag;
+  const int nk = (K + TM_BK - 1) / TM_BK;
+  const int tn = (N + BN - 1) / BN, tiles = tn * ((M + TM_BM - 1) / TM_BM);
+  const int mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // this CTA's tiles
 
-  int phase = 0;
-  const int nk = (K + TC_BK - 1) / TC_BK;
-  for (int kc = 0; kc < nk && !s_err; ++kc) {
-    stage_tile(sA, A, M, K, m0, kc * TC_BK);
-    stage_tile(sB, B, N, K, n0, kc * TC_BK);
-    asm volatile("fence.proxy.async.shared::cta;");
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;");
-      for (int ks = 0; ks < TC_BK / 16; ++ks) {
-        // a 16-deep K step spans core-matrix columns 2 ks and 2 ks + 1
-        const uint64_t ad = make_desc(smem_u32(sA) + ks * 2 * 128, 128, (TC_BK / 8) * 128);
-        const uint64_t bd = make_desc(smem_u32(sB) + ks * 2 * 128, 128, (TC_BK / 8) * 128);
-        const uint32_t acc = (kc > 0 || ks > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-            "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(&mbar)));
-    }
-    // bounded wait for the MMAs of this chunk (they read sA / sB)
-    uint32_t done = 0;
-    for (long long it = 0; it < TC_WAIT_LIMIT && !done; ++it) {
-      asm volatile(
-          "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-          " selp.u32 %0, 1, 0, p;\n}\n"
-          : "=r"(done)
-          : "r"(smem_u32(&mbar)), "r"(phase));
-    }
-    if (!done) {
-      s_err = 1;
-      s_drain = phase;
-    }
-    phase ^= 1;
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    __syncthreads();
-  }
-
-  if (!s_err) {
-    // epilogue: warp w reads TMEM lanes 32 w .. 32 w + 31 (tile rows)
-    const int row = m0 + warp * 32 + lane;
-    for (int c0 = 0; c0 < TC_BN; c0 += 16) {
-      uint32_t r[16];
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(taddr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;");
-      if (row < M) {
-        for (int j = 0; j < 16; ++j) {
-          const int col = n0 + c0 + j;
-          if (col >= N) break;
-          float v = __uint_as_float(r[j]);
-          const size_t o = (size_t)row * N + col;
-          if (epi == EPI_GELU_GRAD) {
-            v *= gelu_grad_f(zin[o]);
-          } else {
-            if (bias) v += bias[col];
-            if (epi == EPI_GELU) {
-              if (zout) zout[o] = v;
-              v = gelu_f(v);
-            }
-          }
-          if (outf) outf[o] = v;
-          if (outb) outb[o] = __float2bfloat16(v);
+  if (warp == 0 && lane == 0) {
+    int it = 0;   // chunk counter: stage it % stages, use it / stages
+    for (int t = 0; t < mine && !*stop; ++t) {
+      const int tile = blockIdx.x + t * gridDim.x;
+      const int m0 = tile / tn * TM_BM, n0 = tile % tn * BN;
+      for (int kc = 0; kc < nk; ++kc, ++it) {
+        const int st = it % Sh::stages, use = it / Sh::stages;
+        if (use > 0 && !tm_wait(&empty[st], (use - 1) & 1, stop)) break;
+        const uint32_t sa = base + st * (Sh::a_bytes + Sh::b_bytes), sb = sa + Sh::a_bytes;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full[st])),
+                     "r"(Sh::a_bytes + Sh::b_bytes)
+                     : "memory");
+        if (ta) {
+          for (int j = 0; j < TM_BM / 64; ++j) tma_load(&mapA, &full[st], sa + j * 8192, m0 + 64 * j, kc * TM_BK);
+        } else {
+          tma_load(&mapA, &full[st], sa, kc * TM_BK, m0);
+        }
+        if (tb) {
+          for (int j = 0; j < BN / 64; ++j) tma_load(&mapB, &full[st], sb + j * 8192, n0 + 64 * j, kc * TM_BK);
+        } else {
+          tma_load(&mapB, &full[st], sb, kc * TM_BK, n0);
         }
       }
     }
-  } else if (tid == 0) {
-    atomicExch(err, 1);
-    // one more bounded wait for the batch still in flight, so that it is
-    // not writing the accumulator when the columns are released
-    if (s_drain >= 0) tc_wait_phase(&mbar, s_drain);
+    // after a give-up: no copy may be in flight when the CTA ends
+    if (*stop) tm_drain(full, Sh::stages, it);
+  } else if (warp == 1 && lane == 0) {
+    const uint32_t idesc = make_idesc(TM_BM, BN) | (ta ? 1u << 15 : 0u) | (tb ? 1u << 16 : 0u);
+    const int step_a = ta ? 2048 : 32, step_b = tb ? 2048 : 32;   // bytes of a 16-deep K step
+    int it = 0;
+    for (int t = 0; t < mine && !*stop; ++t) {
+      const int buf = t & 1;
+      if (t >= 2 && !tm_wait(&acc_empty[buf], ((t >> 1) - 1) & 1, stop)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      bool ok = true;
+      for (int kc = 0; kc < nk; ++kc, ++it) {
+        const int st = it % Sh::stages;
+        if (!tm_wait(&full[st], (it / Sh::stages) & 1, stop)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t sa = base + st * (Sh::a_bytes + Sh::b_bytes), sb = sa + Sh::a_bytes;
+#pragma unroll
+        for (int ks = 0; ks < TM_BK / 16; ++ks) {
+          const uint64_t ad = swizzled_desc(sa + ks * step_a, ta), bd = swizzled_desc(sb + ks * step_b, tb);
+          const uint32_t acc = (kc > 0 || ks > 0) ? 1u : 0u;
+          asm volatile(
+              "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+              " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem + buf * BN),
+              "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+            smem_u32(&empty[st])));
+      }
+      if (!ok) break;
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+          smem_u32(&acc_full[buf])));
+    }
+    // after a give-up: no product may be in flight when TMEM is released
+    if (*stop) tm_drain(empty, Sh::stages, it);
+  } else if (warp >= 2) {
+    const int quarter = warp & 3, half = (warp - 2) >> 2;   // TMEM lanes 32 quarter.., columns half
+    for (int t = 0; t < mine; ++t) {
+      const int buf = t & 1;
+      const int tile = blockIdx.x + t * gridDim.x;
+      const int m0 = tile / tn * TM_BM, n0 = tile % tn * BN;
+      if (!__all_sync(0xffffffffu, tm_wait(&acc_full[buf], (t >> 1) & 1, stop))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const int row = m0 + quarter * 32 + lane;
+      for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 16) {
+        if (n0 + c0 >= N) break;
+        uint32_t r[16];
+        const uint32_t taddr = tmem + buf * BN + ((uint32_t)(quarter * 32) << 16) + c0;
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(taddr));
+        asm volatile("tcgen05.wait::ld.sync.aligned;");
+        if (row < M) epilogue16(out, r, (size_t)row, n0 + c0, min(16, N - n0 - c0));
+        __syncwarp();
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      if (lane == 0) tm_arrive(&acc_empty[buf]);
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_BN));
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (tid == 0 && abort_flag) atomicExch(err, 1);
+  __syncwarp();
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Sh::tmem_cols));
   }
 }
 
@@ -463,21 +611,92 @@ __global__ void bloch_free_add_kernel(float* __restrict__ y, const float* __rest
 
 using namespace otb;
 
+namespace {
+
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// The driver's tensor-map encoder (null where the driver has none).
+EncodeTiled tensor_map_encoder() {
+  static EncodeTiled f = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return (EncodeTiled)p;
+  }();
+  return f;
+}
+
+// Map of an operand of `rows` logical rows and depth K: stored [rows][K] (box
+// 64 x box_rows) or, transposed, [K][rows] (box 64 x 64); ld elements per
+// stored row, a multiple of 8.
+bool operand_map(CUtensorMap* map, const void* p, int rows, int K, int ld, bool trans, int box_rows) {
+  EncodeTiled enc = tensor_map_encoder();
+  if (!enc) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)(trans ? rows : K), (cuuint64_t)(trans ? K : rows)};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  const cuuint32_t box[2] = {64, (cuuint32_t)(trans ? 64 : box_rows)};
+  const cuuint32_t ones[2] = {1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, ones,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BN>
+otb_status launch_tma(const void* A, int lda, bool ta, const void* B, int ldb, bool tb, int M, int N, int K,
+                      const GemmOut& out, int sms, int32_t* err, cudaStream_t stream) {
+  CUtensorMap ma, mb;
+  if (!operand_map(&ma, A, M, K, lda, ta, TM_BM) || !operand_map(&mb, B, N, K, ldb, tb, BN))
+    return set_error(OTB_ERR_CUDA, "tensor map");
+  const int tiles = ((M + TM_BM - 1) / TM_BM) * ((N + BN - 1) / BN);
+  if (!check_cuda(cudaFuncSetAttribute(tc_gemm_tma_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       TmShape<BN>::smem),
+                  "tma gemm smem"))
+    return OTB_ERR_CUDA;
+  tc_gemm_tma_kernel<BN><<<std::min(tiles, sms), TM_THREADS, TmShape<BN>::smem, stream>>>(ma, mb, M, N, K, ta, tb, out,
+                                                                                          err);
+  if (!check_cuda(cudaGetLastError(), "tma gemm")) return OTB_ERR_CUDA;
+  return OTB_OK;
+}
+
+bool tma_operand(const void* p, int ld) { return ld % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// Out = A B^T, A [M][K] (lda; transposed: [K][M]) and B [N][K] (ldb; transposed:
+// [K][N]) with 16-byte aligned rows.
+otb_status gemm_tma(const void* A, int lda, bool ta, const void* B, int ldb, bool tb, int M, int N, int K,
+                    const GemmOut& out, int32_t* err, cudaStream_t stream) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  sms = std::max(sms, 1);
+  const int mt = (M + TM_BM - 1) / TM_BM;
+  if (mt * ((N + 255) / 256) >= sms) return launch_tma<256>(A, lda, ta, B, ldb, tb, M, N, K, out, sms, err, stream);
+  if (mt * ((N + 127) / 128) >= sms) return launch_tma<128>(A, lda, ta, B, ldb, tb, M, N, K, out, sms, err, stream);
+  return launch_tma<64>(A, lda, ta, B, ldb, tb, M, N, K, out, sms, err, stream);
+}
+
+}  // namespace
+
 extern "C" otb_status otb_mlp_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K,
                                    const float* bias, int32_t epilogue, const float* z_in, float* z_out,
                                    float* out_f32, void* out_bf16, int32_t* err, void* stream) {
   if (!A || !B || !err || M <= 0 || N <= 0 || K <= 0 || epilogue < 0 || epilogue > 2)
     return set_error(OTB_ERR_INVALID_ARG, "bad gemm arguments");
   if (epilogue == EPI_GELU_GRAD && !z_in) return set_error(OTB_ERR_INVALID_ARG, "gelu-grad needs z_in");
+  if (tma_operand(A, K) && tma_operand(B, K) && tensor_map_encoder()) {
+    const GemmOut out{bias, z_in, z_out, out_f32, (__nv_bfloat16*)out_bf16, N, N, epilogue};
+    return gemm_tma(A, K, false, B, K, false, M, N, K, out, err, (cudaStream_t)stream);
+  }
   dim3 grid((N + TC_BN - 1) / TC_BN, (M + TC_BM - 1) / TC_BM);
   constexpr int smem = 2 * (TC_BM + TC_BN) * TC_BK * 2;   // two A + B stages, 64 KiB
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (!check_cuda(cudaFuncSetAttribute(tc_gemm_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                    "tc gemm smem"))
-      return OTB_ERR_CUDA;
-    attr_set = true;
-  }
+  if (!check_cuda(cudaFuncSetAttribute(tc_gemm_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                  "tc gemm smem"))
+    return OTB_ERR_CUDA;
   tc_gemm_pipe_kernel<<<grid, TC_THREADS, smem, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, M, N, K, bias, epilogue, z_in, z_out, out_f32,
       (__nv_bfloat16*)out_bf16, err);
