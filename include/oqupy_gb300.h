@@ -368,6 +368,39 @@ otb_status otb_mlp_adamw(float* w, const float* g, float* m, float* v, void* w_b
                          int64_t n, float lr, float beta1, float beta2, float eps,
                          float weight_decay, int32_t step, void* stream);
 
+/* otb_mlp_gemm on operands with row strides (elements, multiples of 8; bases
+ * 16-byte aligned): A is [M][K], or with trans_a [K][M]; B is [N][K], or with
+ * trans_b [K][N].  z_in, z_out and out_f32 are [M][N]; out_bf16 has row stride
+ * ld_bf16. */
+otb_status otb_mlp_gemm_strided(const void* A, int32_t lda, int32_t trans_a, const void* B,
+                                int32_t ldb, int32_t trans_b, int32_t M, int32_t N, int32_t K,
+                                const float* bias, int32_t epilogue, const float* z_in,
+                                float* z_out, float* out_f32, void* out_bf16, int32_t ld_bf16,
+                                int32_t* err, void* stream);
+/* otb_mlp_mse_grad of a [rows][cols] matrix, the bf16 gradient with row stride
+ * ld_bf16 */
+otb_status otb_mlp_mse_grad_rows(const float* y, const float* t, float* g_f32, void* g_bf16,
+                                 int32_t rows, int32_t cols, int32_t ld_bf16, double* loss,
+                                 void* stream);
+/* otb_mlp_colsum of n <= 32 matrices of `rows` rows in one launch (host arrays
+ * of device pointers and column counts) */
+otb_status otb_mlp_colsums(int32_t n, const float* const* in, float* const* out, int32_t rows,
+                           const int32_t* cols, void* stream);
+/* One layer of a network: FP32 weights [fout][fin] and bias [fout] with their
+ * gradients and AdamW moments, the weights' bf16 copy (row stride ld_w) and its
+ * transpose [fin][fout] (row stride ld_wt).  Device pointers. */
+typedef struct {
+  int32_t fout, fin, ld_w, ld_wt;
+  float *w, *mw, *vw, *b, *mb, *vb;
+  const float *gw, *gb;
+  void *w_bf16, *wt_bf16;
+} otb_mlp_layer;
+/* AdamW step on every layer (n <= 32) in one launch: weight decay on the
+ * weights, none on the biases; refreshes both bf16 copies. */
+otb_status otb_mlp_adamw_net(int32_t n, const otb_mlp_layer* layers, float lr, float beta1,
+                             float beta2, float eps, float weight_decay, int32_t step,
+                             void* stream);
+
 /* Surrogate output baseline (no reference counterpart): adds to y[B][3][nsteps]
  * the Bloch vector of the bath-free system H = Omega/2 sx + eps/2 sz started
  * in (0, 0, 1) at times dt, 2 dt, ..., nsteps dt; omega_eps[B][2] holds

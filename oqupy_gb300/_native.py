@@ -84,6 +84,12 @@ class PtInfo(ctypes.Structure):
                 ("flops_alg", ctypes.c_double)]
 
 
+class MlpLayer(ctypes.Structure):
+    _fields_ = ([(k, ctypes.c_int32) for k in ("fout", "fin", "ld_w", "ld_wt")]
+                + [(k, ctypes.c_void_p) for k in ("w", "mw", "vw", "b", "mb", "vb", "gw", "gb",
+                                                  "w_bf16", "wt_bf16")])
+
+
 class DeviceError(RuntimeError):
     """A status code returned by the CUDA library."""
 
@@ -135,6 +141,12 @@ def _declare(lib):
         "otb_mlp_transpose_bf16": (i32, [P, P, i32, i32, P]),
         "otb_mlp_f32_to_bf16": (i32, [P, P, ctypes.c_int64, P]),
         "otb_mlp_colsum": (i32, [P, P, i32, i32, P]),
+        "otb_mlp_gemm_strided": (i32, [P, i32, i32, P, i32, i32, i32, i32, i32, P, i32, P, P, P, P,
+                                       i32, P, P]),
+        "otb_mlp_mse_grad_rows": (i32, [P, P, P, P, i32, i32, i32, P, P]),
+        "otb_mlp_colsums": (i32, [i32, ctypes.POINTER(P), ctypes.POINTER(P), i32, c_int32_p, P]),
+        "otb_mlp_adamw_net": (i32, [i32, ctypes.POINTER(MlpLayer), ctypes.c_float, ctypes.c_float,
+                                    ctypes.c_float, ctypes.c_float, ctypes.c_float, i32, P]),
         "otb_mlp_bloch_free_add": (i32, [P, P, i32, i32, ctypes.c_float, P]),
         "otb_mlp_mse_grad": (i32, [P, P, P, P, ctypes.c_int64, P, P]),
         "otb_mlp_adamw": (i32, [P, P, P, P, P, ctypes.c_int64, ctypes.c_float,
@@ -163,7 +175,8 @@ def exported_symbols():
         "otb_pt_get_tensor", "otb_pt_get_cap", "otb_dyn_run", "otb_dyn_run_steps", "otb_dyn_gradient", "otb_dyn_session_create",
         "otb_dyn_session_step", "otb_dyn_session_state", "otb_dyn_session_destroy", "otb_mlp_gemm",
         "otb_mlp_transpose_bf16", "otb_mlp_f32_to_bf16", "otb_mlp_colsum",
-        "otb_mlp_mse_grad", "otb_mlp_adamw", "otb_mlp_bloch_free_add",
+        "otb_mlp_mse_grad", "otb_mlp_adamw", "otb_mlp_gemm_strided", "otb_mlp_mse_grad_rows",
+        "otb_mlp_colsums", "otb_mlp_adamw_net", "otb_mlp_bloch_free_add",
         "otb_measure_fma_peak", "otb_last_error", "otb_version"]
 
 

@@ -101,7 +101,7 @@ struct GemmOut {
   int epi;
 };
 
-// 16 consecutive outputs of one row, in the widest stores the address allows.
+// n <= 16 consecutive outputs of one row, in the widest stores the address allows.
 __device__ __forceinline__ void store16(float* p, const float* v, int n) {
   if (n == 16 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
 #pragma unroll
@@ -130,44 +130,82 @@ __device__ __forceinline__ void store16(__nv_bfloat16* p, const float* v, int n)
   }
 }
 
-// 16 accumulators of one row through the fused step.
-__device__ __forceinline__ void epilogue16(const GemmOut& o, const uint32_t* r, size_t row, int col, int n) {
-  float v[16];
-  const size_t at = row * o.ldf + col;
-  if (o.epi == EPI_GELU_GRAD) {
-    const float* z = o.zin + at;
-    float zz[16];
-    if (n == 16 && (reinterpret_cast<uintptr_t>(z) & 15) == 0) {
+// The fused step on CH accumulators of one row (n of them inside the matrix):
+// v = the outputs; with EPI_GELU z = the pre-activations.
+template <int CH>
+__device__ __forceinline__ void fused_step(const GemmOut& o, const uint32_t* r, size_t at, int col, int n, float* v,
+                                           float* z) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 t = reinterpret_cast<const float4*>(z)[q];
-        zz[4 * q] = t.x;
-        zz[4 * q + 1] = t.y;
-        zz[4 * q + 2] = t.z;
-        zz[4 * q + 3] = t.w;
+  for (int q = 0; q < CH; ++q) v[q] = __uint_as_float(r[q]);
+  if (o.epi == EPI_GELU_GRAD) {
+    const float* zi = o.zin + at;
+    if (n == CH && (reinterpret_cast<uintptr_t>(zi) & 15) == 0) {
+#pragma unroll
+      for (int q = 0; q < CH / 4; ++q) {
+        const float4 t = reinterpret_cast<const float4*>(zi)[q];
+        v[4 * q] *= gelu_grad_f(t.x);
+        v[4 * q + 1] *= gelu_grad_f(t.y);
+        v[4 * q + 2] *= gelu_grad_f(t.z);
+        v[4 * q + 3] *= gelu_grad_f(t.w);
       }
     } else {
 #pragma unroll
-      for (int q = 0; q < 16; ++q) zz[q] = q < n ? z[q] : 0.f;
+      for (int q = 0; q < CH; ++q)
+        if (q < n) v[q] *= gelu_grad_f(zi[q]);
     }
+    return;
+  }
+  if (o.bias) {
 #pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]) * gelu_grad_f(zz[q]);
-  } else {
+    for (int q = 0; q < CH; ++q)
+      if (q < n) v[q] += __ldg(o.bias + col + q);
+  }
+  if (o.epi == EPI_GELU) {
 #pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
-    if (o.bias) {
-#pragma unroll
-      for (int q = 0; q < 16; ++q)
-        if (q < n) v[q] += __ldg(o.bias + col + q);
-    }
-    if (o.epi == EPI_GELU) {
-      if (o.zout) store16(o.zout + at, v, n);
-#pragma unroll
-      for (int q = 0; q < 16; ++q) v[q] = gelu_f(v[q]);
+    for (int q = 0; q < CH; ++q) {
+      z[q] = v[q];
+      v[q] = gelu_f(v[q]);
     }
   }
+}
+
+// 16 accumulators of one row through the fused step and to memory.
+__device__ __forceinline__ void epilogue16(const GemmOut& o, const uint32_t* r, size_t row, int col, int n) {
+  float v[16], z[16];
+  const size_t at = row * o.ldf + col;
+  fused_step<16>(o, r, at, col, n, v, z);
+  if (o.epi == EPI_GELU && o.zout) store16(o.zout + at, z, n);
   if (o.outf) store16(o.outf + at, v, n);
   if (o.outb) store16(o.outb + row * o.ldb + col, v, n);
+}
+
+// A warp's 32 x 32 block (lane = row, v = its 32 columns) to row-major memory
+// through its shared buffer (rows 33 words apart), so that a store writes whole
+// 128-byte row segments instead of 32 scattered pieces.
+__device__ __forceinline__ void store_block(float* buf, const float* v, float* dst, int ld, int rows) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < 32; ++q) buf[lane * 33 + q] = v[q];
+  __syncwarp();
+  for (int i = 0; i < rows; ++i) dst[(size_t)i * ld + lane] = buf[i * 33 + lane];
+  __syncwarp();
+}
+__device__ __forceinline__ void store_block(float* buf, const float* v, __nv_bfloat16* dst, int ld, int rows) {
+  const int lane = threadIdx.x & 31;
+  uint32_t* b = reinterpret_cast<uint32_t*>(buf);   // rows 17 words apart
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    union {
+      uint32_t u;
+      __nv_bfloat162 h;
+    } t;
+    t.h = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+    b[lane * 17 + q] = t.u;
+  }
+  __syncwarp();
+  for (int i = lane >> 4; i < rows; i += 2)   // two rows of 64 bytes a store
+    *reinterpret_cast<uint32_t*>(dst + (size_t)i * ld + 2 * (lane & 15)) = b[i * 17 + (lane & 15)];
+  __syncwarp();
 }
 
 __device__ __forceinline__ bool tc_wait_phase(uint64_t* mbar, int phase) {
@@ -317,7 +355,10 @@ __global__ void __launch_bounds__(TC_THREADS)
 // result's write to memory.  The two-stage kernel above (cp.async staging by
 // the warps that also issue the products and run the epilogue, scalar stores)
 // reached 79 TFLOP/s on a 60001-point inference of a 5-512x4-1500 network
-// (2370 us); with this one the inference takes 492 us.
+// (2370 us); with this one the inference takes 453 us (492 us with every lane
+// storing pieces of its own row).  A training step of 256 points, where the
+// 1500-column operands were staged element by element and both operands of
+// every weight gradient transposed first: 1020 -> 327 us, launches 45 -> 19.
 //
 // Used when rows are 16-byte aligned; other operands keep the kernel above.
 // Tile width: 256 where that gives every SM a tile, else 128, else 64 (a
@@ -327,12 +368,15 @@ constexpr int TM_EPI_WARPS = 8;
 constexpr int TM_THREADS = 64 + 32 * TM_EPI_WARPS;
 constexpr unsigned long long TM_WAIT_NS = 2000000000ull;
 
+constexpr int TM_XPOSE = 32 * 33 * 4;   // an epilogue warp's transposition buffer
+
 template <int BN>
 struct TmShape {
-  static constexpr int stages = BN == 256 ? 4 : 6;
+  static constexpr int stages = BN == 256 ? 3 : 5;
   static constexpr int a_bytes = TM_BM * TM_BK * 2;
   static constexpr int b_bytes = BN * TM_BK * 2;
-  static constexpr int smem = stages * (a_bytes + b_bytes) + 1024;   // + alignment
+  static constexpr int ring = stages * (a_bytes + b_bytes);
+  static constexpr int smem = ring + TM_EPI_WARPS * TM_XPOSE + 1024;   // + alignment
   static constexpr int tmem_cols = 2 * BN;
 };
 
@@ -495,18 +539,45 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
       const int m0 = tile / tn * TM_BM, n0 = tile % tn * BN;
       if (!__all_sync(0xffffffffu, tm_wait(&acc_full[buf], (t >> 1) & 1, stop))) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
-      const int row = m0 + quarter * 32 + lane;
-      for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 16) {
+      const int row0 = m0 + quarter * 32, row = row0 + lane;
+      const int rows = min(32, M - row0);
+      float* const xbuf = reinterpret_cast<float*>(tm_raw + (base - smem_u32(tm_raw)) + Sh::ring) + (warp - 2) * (TM_XPOSE / 4);
+      for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
         if (n0 + c0 >= N) break;
-        uint32_t r[16];
+        uint32_t r[32];
         const uint32_t taddr = tmem + buf * BN + ((uint32_t)(quarter * 32) << 16) + c0;
         asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+              "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
             : "r"(taddr));
         asm volatile("tcgen05.wait::ld.sync.aligned;");
-        if (row < M) epilogue16(out, r, (size_t)row, n0 + c0, min(16, N - n0 - c0));
+        if (rows <= 0) continue;
+        const int col = n0 + c0;
+        if (col + 32 <= N) {
+          // rows past the matrix read row 0's pre-activations and are not stored
+          float v[32], z[32];
+          fused_step<32>(out, r, (size_t)(row < M ? row : row0) * out.ldf + col, col, 32, v, z);
+          const size_t at = (size_t)row0 * out.ldf + col;
+          if (out.epi == EPI_GELU && out.zout) store_block(xbuf, z, out.zout + at, out.ldf, rows);
+          if (out.outf) store_block(xbuf, v, out.outf + at, out.ldf, rows);
+          if (out.outb) {
+            if ((out.ldb & 1) || (reinterpret_cast<uintptr_t>(out.outb) & 3)) {
+              if (row < M) {
+                store16(out.outb + (size_t)row * out.ldb + col, v, 16);
+                store16(out.outb + (size_t)row * out.ldb + col + 16, v + 16, 16);
+              }
+            } else {
+              store_block(xbuf, v, out.outb + (size_t)row0 * out.ldb + col, out.ldb, rows);
+            }
+          }
+        } else if (row < M) {
+          epilogue16(out, r, (size_t)row, col, min(16, N - col));
+          if (col + 16 < N) epilogue16(out, r + 16, (size_t)row, col + 16, N - col - 16);
+        }
         __syncwarp();
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
@@ -553,20 +624,124 @@ __global__ void colsum_kernel(const float* __restrict__ in, float* __restrict__ 
   out[c] = s;
 }
 
-// mean-squared-error gradient dY = 2 (Y - T) / (R C) (FP32 and bf16); loss
-// partial sums accumulated into *loss
-__global__ void mse_grad_kernel(const float* __restrict__ y, const float* __restrict__ t, float* __restrict__ gf,
-                                __nv_bfloat16* __restrict__ gb, long long n, float scale, double* loss) {
+// Bias gradients of every layer in one launch: column sums of row-major FP32
+// matrices.  A CTA takes 32 columns of one matrix: 8 warps sum every eighth row
+// (coalesced), then the eight partial sums in order.  (One thread per column on
+// a handful of CTAs, one launch a layer: 17 us each for 256 rows; all of them
+// now: 5 us.)
+constexpr int MLP_MAX_LAYERS = 32;
+struct ColsumJobs {
+  int n, rows;
+  int first[MLP_MAX_LAYERS + 1];   // first CTA of every matrix
+  int cols[MLP_MAX_LAYERS];
+  const float* in[MLP_MAX_LAYERS];
+  float* out[MLP_MAX_LAYERS];
+};
+
+__global__ void __launch_bounds__(256) colsum_multi_kernel(const __grid_constant__ ColsumJobs j) {
+  __shared__ float part[8][33];
+  int q = 0;
+  while (q + 1 < j.n && (int)blockIdx.x >= j.first[q + 1]) ++q;
+  const int C = j.cols[q];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = ((int)blockIdx.x - j.first[q]) * 32 + lane;
+  float s = 0.f;
+  if (c < C) {
+    const float* p = j.in[q] + c;
+#pragma unroll 4
+    for (int r = warp; r < j.rows; r += 8) s += p[(size_t)r * C];
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && c < C) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) s += part[w][lane];
+    j.out[q][c] = s;
+  }
+}
+
+// AdamW on every tensor of a network in one launch, 32 x 32 tiles; weights also
+// refresh their bf16 copy (row stride ldw) and its transpose (row stride ldt).
+// (Two updates and a transposition per layer, 15 launches of 3 to 8 us for five
+// layers, before.)
+struct AdamTensor {
+  float *w, *m, *v;
+  const float* g;
+  __nv_bfloat16 *wb, *wt;   // null: a bias
+  int rows, cols, ldw, ldt, first;
+  float wd;
+};
+struct AdamJobs {
+  int n;
+  float lr, b1, b2, eps, c1, c2;
+  AdamTensor t[2 * MLP_MAX_LAYERS];
+};
+
+__device__ __forceinline__ float adamw_update(float& w, float g, float& m, float& v, float lr, float b1, float b2,
+                                              float eps, float wd, float c1, float c2) {
+  m = b1 * m + (1.f - b1) * g;
+  v = b2 * v + (1.f - b2) * g * g;
+  float wi = w * (1.f - lr * wd);
+  wi -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+  w = wi;
+  return wi;
+}
+
+__global__ void __launch_bounds__(256) adamw_multi_kernel(const __grid_constant__ AdamJobs j) {
+  __shared__ float tile[32][33];
+  int q = 0;
+  while (q + 1 < j.n && (int)blockIdx.x >= j.t[q + 1].first) ++q;
+  const AdamTensor& t = j.t[q];
+  const int tiles_c = (t.cols + 31) / 32, b = (int)blockIdx.x - t.first;
+  const int r0 = b / tiles_c * 32, c0 = b % tiles_c * 32;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < 32; i += 8) {
+    const int r = r0 + y + i, c = c0 + x;
+    if (r < t.rows && c < t.cols) {
+      const size_t e = (size_t)r * t.cols + c;
+      float w = t.w[e], m = t.m[e], v = t.v[e];
+      adamw_update(w, t.g[e], m, v, j.lr, j.b1, j.b2, j.eps, t.wd, j.c1, j.c2);
+      t.w[e] = w;
+      t.m[e] = m;
+      t.v[e] = v;
+      if (t.wb) t.wb[(size_t)r * t.ldw + c] = __float2bfloat16(w);
+      tile[y + i][x] = w;
+    }
+  }
+  if (!t.wt) return;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 32; i += 8) {
+    const int c = c0 + y + i, r = r0 + x;
+    if (c < t.cols && r < t.rows) t.wt[(size_t)c * t.ldt + r] = __float2bfloat16(tile[x][y + i]);
+  }
+}
+
+// mean-squared-error gradient dY = 2 (Y - T) / (R C) (FP32, and bf16 with row
+// stride ldb); loss partial sums accumulated into *loss, one atomic per CTA
+__global__ void __launch_bounds__(256)
+    mse_grad_kernel(const float* __restrict__ y, const float* __restrict__ t, float* __restrict__ gf,
+                    __nv_bfloat16* __restrict__ gb, int rows, int cols, int ldb, float scale, double* loss) {
+  __shared__ double part[8];
   double acc = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float d = y[i] - t[i];
-    acc += (double)d * d;
-    const float g = 2.f * d * scale;
-    gf[i] = g;
-    gb[i] = __float2bfloat16(g);
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+      const size_t i = (size_t)r * cols + c;
+      const float d = y[i] - t[i];
+      acc += (double)d * d;
+      const float g = 2.f * d * scale;
+      gf[i] = g;
+      gb[(size_t)r * ldb + c] = __float2bfloat16(g);
+    }
   }
   for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) acc += part[w];
+    atomicAdd(loss, acc);
+  }
 }
 
 // AdamW on FP32 master weights; refreshes the bf16 copy
@@ -574,14 +749,7 @@ __global__ void adamw_kernel(float* __restrict__ w, const float* __restrict__ g,
                              float* __restrict__ v, __nv_bfloat16* __restrict__ wb, long long n, float lr, float b1,
                              float b2, float eps, float wd, float c1, float c2) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    float wi = w[i] * (1.f - lr * wd);
-    wi -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
+    const float wi = adamw_update(w[i], g[i], m[i], v[i], lr, b1, b2, eps, wd, c1, c2);
     if (wb) wb[i] = __float2bfloat16(wi);
   }
 }
@@ -664,6 +832,12 @@ otb_status launch_tma(const void* A, int lda, bool ta, const void* B, int ldb, b
   return OTB_OK;
 }
 
+// a few rows per CTA, four CTAs per SM
+void launch_mse(const float* y, const float* t, float* gf, __nv_bfloat16* gb, int rows, int cols, int ldb, float scale,
+                double* loss, cudaStream_t s) {
+  mse_grad_kernel<<<std::min(rows, 608), 256, 0, s>>>(y, t, gf, gb, rows, cols, ldb, scale, loss);
+}
+
 bool tma_operand(const void* p, int ld) { return ld % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Out = A B^T, A [M][K] (lda; transposed: [K][M]) and B [N][K] (ldb; transposed:
@@ -731,9 +905,91 @@ extern "C" otb_status otb_mlp_colsum(const float* in, float* out, int32_t R, int
 extern "C" otb_status otb_mlp_mse_grad(const float* y, const float* t, float* g_f32, void* g_bf16, int64_t n,
                                        double* loss, void* stream) {
   if (!y || !t || !g_f32 || !g_bf16 || !loss || n <= 0) return set_error(OTB_ERR_INVALID_ARG, "bad mse arguments");
-  mse_grad_kernel<<<1024, 256, 0, (cudaStream_t)stream>>>(y, t, g_f32, (__nv_bfloat16*)g_bf16, n,
-                                                          1.f / (float)n, loss);
+  // flat: rows of 1024 values and a remainder row
+  const int64_t rows = n / 1024, rest = n % 1024;
+  if (rows > INT32_MAX) return set_error(OTB_ERR_INVALID_ARG, "bad mse arguments");
+  cudaStream_t s = (cudaStream_t)stream;
+  __nv_bfloat16* gb = (__nv_bfloat16*)g_bf16;
+  if (rows) launch_mse(y, t, g_f32, gb, (int)rows, 1024, 1024, 1.f / (float)n, loss, s);
+  if (rest) {
+    const int64_t o = rows * 1024;
+    launch_mse(y + o, t + o, g_f32 + o, gb + o, 1, (int)rest, (int)rest, 1.f / (float)n, loss, s);
+  }
   if (!check_cuda(cudaGetLastError(), "mse")) return OTB_ERR_CUDA;
+  return OTB_OK;
+}
+
+extern "C" otb_status otb_mlp_mse_grad_rows(const float* y, const float* t, float* g_f32, void* g_bf16, int32_t rows,
+                                            int32_t cols, int32_t ld_bf16, double* loss, void* stream) {
+  if (!y || !t || !g_f32 || !g_bf16 || !loss || rows <= 0 || cols <= 0 || ld_bf16 < cols)
+    return set_error(OTB_ERR_INVALID_ARG, "bad mse arguments");
+  launch_mse(y, t, g_f32, (__nv_bfloat16*)g_bf16, rows, cols, ld_bf16, 1.f / (float)((int64_t)rows * cols), loss,
+             (cudaStream_t)stream);
+  if (!check_cuda(cudaGetLastError(), "mse")) return OTB_ERR_CUDA;
+  return OTB_OK;
+}
+
+extern "C" otb_status otb_mlp_gemm_strided(const void* A, int32_t lda, int32_t trans_a, const void* B, int32_t ldb,
+                                           int32_t trans_b, int32_t M, int32_t N, int32_t K, const float* bias,
+                                           int32_t epilogue, const float* z_in, float* z_out, float* out_f32,
+                                           void* out_bf16, int32_t ld_bf16, int32_t* err, void* stream) {
+  if (!A || !B || !err || M <= 0 || N <= 0 || K <= 0 || epilogue < 0 || epilogue > 2 ||
+      lda < (trans_a ? M : K) || ldb < (trans_b ? N : K) || (out_bf16 && ld_bf16 < N))
+    return set_error(OTB_ERR_INVALID_ARG, "bad gemm arguments");
+  if (epilogue == EPI_GELU_GRAD && !z_in) return set_error(OTB_ERR_INVALID_ARG, "gelu-grad needs z_in");
+  if (!tma_operand(A, lda) || !tma_operand(B, ldb))
+    return set_error(OTB_ERR_INVALID_ARG, "operand rows must be 16-byte aligned");
+  const GemmOut out{bias, z_in, z_out, out_f32, (__nv_bfloat16*)out_bf16, N, out_bf16 ? ld_bf16 : N, epilogue};
+  return gemm_tma(A, lda, trans_a != 0, B, ldb, trans_b != 0, M, N, K, out, err, (cudaStream_t)stream);
+}
+
+extern "C" otb_status otb_mlp_colsums(int32_t n, const float* const* in, float* const* out, int32_t rows,
+                                      const int32_t* cols, void* stream) {
+  if (n < 1 || n > MLP_MAX_LAYERS || !in || !out || !cols || rows <= 0)
+    return set_error(OTB_ERR_INVALID_ARG, "bad colsum arguments");
+  ColsumJobs j;
+  j.n = n;
+  j.rows = rows;
+  int first = 0;
+  for (int i = 0; i < n; ++i) {
+    if (!in[i] || !out[i] || cols[i] <= 0) return set_error(OTB_ERR_INVALID_ARG, "bad colsum arguments");
+    j.first[i] = first;
+    j.cols[i] = cols[i];
+    j.in[i] = in[i];
+    j.out[i] = out[i];
+    first += (cols[i] + 31) / 32;
+  }
+  j.first[n] = first;
+  colsum_multi_kernel<<<first, 256, 0, (cudaStream_t)stream>>>(j);
+  if (!check_cuda(cudaGetLastError(), "colsums")) return OTB_ERR_CUDA;
+  return OTB_OK;
+}
+
+extern "C" otb_status otb_mlp_adamw_net(int32_t n, const otb_mlp_layer* layers, float lr, float beta1, float beta2,
+                                        float eps, float weight_decay, int32_t step, void* stream) {
+  if (n < 1 || n > MLP_MAX_LAYERS || !layers || step < 1) return set_error(OTB_ERR_INVALID_ARG, "bad adamw arguments");
+  AdamJobs j;
+  j.n = 2 * n;
+  j.lr = lr;
+  j.b1 = beta1;
+  j.b2 = beta2;
+  j.eps = eps;
+  j.c1 = 1.f - powf(beta1, (float)step);
+  j.c2 = 1.f - powf(beta2, (float)step);
+  int first = 0;
+  for (int i = 0; i < n; ++i) {
+    const otb_mlp_layer& l = layers[i];
+    if (l.fout <= 0 || l.fin <= 0 || !l.w || !l.gw || !l.mw || !l.vw || !l.b || !l.gb || !l.mb || !l.vb || !l.w_bf16 ||
+        !l.wt_bf16 || l.ld_w < l.fin || l.ld_wt < l.fout)
+      return set_error(OTB_ERR_INVALID_ARG, "bad adamw arguments");
+    j.t[2 * i] = AdamTensor{l.w, l.mw, l.vw, l.gw, (__nv_bfloat16*)l.w_bf16, (__nv_bfloat16*)l.wt_bf16,
+                            l.fout, l.fin, l.ld_w, l.ld_wt, first, weight_decay};
+    first += ((l.fout + 31) / 32) * ((l.fin + 31) / 32);
+    j.t[2 * i + 1] = AdamTensor{l.b, l.mb, l.vb, l.gb, nullptr, nullptr, 1, l.fout, 0, 0, first, 0.f};
+    first += (l.fout + 31) / 32;
+  }
+  adamw_multi_kernel<<<first, 256, 0, (cudaStream_t)stream>>>(j);
+  if (!check_cuda(cudaGetLastError(), "adamw")) return OTB_ERR_CUDA;
   return OTB_OK;
 }
 

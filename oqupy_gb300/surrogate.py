@@ -15,6 +15,7 @@ space whose validation error exceeds the stated budget, falls back to the
 TEMPO solve; the surrogate answers the rest.
 """
 
+import ctypes
 import time
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -53,35 +54,29 @@ class Mlp:
             self.v.append(torch.zeros(fout, fin, device=self.dev))
             self.mb.append(torch.zeros(fout, device=self.dev))
             self.vb.append(torch.zeros(fout, device=self.dev))
-        self.Wb = [torch.empty(w.shape, dtype=torch.bfloat16, device=self.dev) for w in self.W]
-        self.WbT = [torch.empty((w.shape[1], w.shape[0]), dtype=torch.bfloat16, device=self.dev)
-                    for w in self.W]
+        # bf16 copies, rows padded to 16 bytes (what the tensor-core kernel's loads need)
+        self.Wb = [self._rows(*w.shape) for w in self.W]
+        self.WbT = [self._rows(w.shape[1], w.shape[0]) for w in self.W]
         self.err = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self.steps = 0
-        for l in range(len(self.W)):
-            self._refresh(l)
+        for l, w in enumerate(self.W):
+            self.Wb[l].copy_(w)
+            self.WbT[l].copy_(w.T)
 
     # -- primitives -------------------------------------------------------
     def _p(self, t):
         return None if t is None else t.data_ptr()
 
-    def _gemm(self, A, B, M, N, K, bias=None, epi=0, zin=None, zout=None, outf=None, outb=None):
-        nat.check(nat.lib().otb_mlp_gemm(self._p(A), self._p(B), M, N, K, self._p(bias), epi,
-                                         self._p(zin), self._p(zout), self._p(outf), self._p(outb),
-                                         self._p(self.err), None))
+    def _rows(self, rows, cols):
+        """An uninitialised bf16 matrix with rows padded to a multiple of 8."""
+        return self.torch.empty((rows, (cols + 7) // 8 * 8), dtype=self.torch.bfloat16,
+                                device=self.dev)[:, :cols]
 
-    def _transpose(self, x):
-        R, C = x.shape
-        out = self.torch.empty((C, R), dtype=self.torch.bfloat16, device=self.dev)
-        nat.check(nat.lib().otb_mlp_transpose_bf16(x.data_ptr(), out.data_ptr(), R, C, None))
-        return out
-
-    def _refresh(self, l):
-        nat.check(nat.lib().otb_mlp_f32_to_bf16(self.W[l].data_ptr(), self.Wb[l].data_ptr(),
-                                                self.W[l].numel(), None))
-        w = self.Wb[l]
-        nat.check(nat.lib().otb_mlp_transpose_bf16(w.data_ptr(), self.WbT[l].data_ptr(),
-                                                   w.shape[0], w.shape[1], None))
+    def _gemm(self, A, ta, B, tb, M, N, K, bias=None, epi=0, zin=None, zout=None, outf=None, outb=None):
+        nat.check(nat.lib().otb_mlp_gemm_strided(
+            A.data_ptr(), A.stride(0), ta, B.data_ptr(), B.stride(0), tb, M, N, K, self._p(bias), epi,
+            self._p(zin), self._p(zout), self._p(outf), self._p(outb),
+            0 if outb is None else outb.stride(0), self._p(self.err), None))
 
     # -- passes -----------------------------------------------------------
     def forward(self, X, keep: bool = False):
@@ -89,23 +84,24 @@ class Mlp:
         FP32; with ``keep`` the pre-activations and activations are kept for
         ``backward``."""
         torch = self.torch
-        H = X.to(torch.bfloat16).contiguous()
-        Bn = H.shape[0]
+        Bn = X.shape[0]
+        H = self._rows(Bn, X.shape[1])
+        H.copy_(X)
         Hs, Zs = [H], []
         L = len(self.W)
         for l in range(L):
             fout, fin = self.W[l].shape
             if l < L - 1:
                 Z = torch.empty((Bn, fout), device=self.dev) if keep else None
-                Hn = torch.empty((Bn, fout), dtype=torch.bfloat16, device=self.dev)
-                self._gemm(H, self.Wb[l], Bn, fout, fin, bias=self.b[l], epi=1, zout=Z, outb=Hn)
+                Hn = self._rows(Bn, fout)
+                self._gemm(H, 0, self.Wb[l], 0, Bn, fout, fin, bias=self.b[l], epi=1, zout=Z, outb=Hn)
                 H = Hn
                 if keep:
                     Zs.append(Z)
                     Hs.append(H)
             else:
                 Y = torch.empty((Bn, fout), device=self.dev)
-                self._gemm(H, self.Wb[l], Bn, fout, fin, bias=self.b[l], epi=0, outf=Y)
+                self._gemm(H, 0, self.Wb[l], 0, Bn, fout, fin, bias=self.b[l], epi=0, outf=Y)
         if keep:
             self._cache = (Zs, Hs)
         return Y
@@ -118,42 +114,50 @@ class Mlp:
         torch = self.torch
         Y = self.forward(X, keep=True)
         Zs, Hs = self._cache
-        n = Y.numel()
+        Bn = Y.shape[0]
         dZf = torch.empty_like(Y)
-        dZb = torch.empty(Y.shape, dtype=torch.bfloat16, device=self.dev)
+        dZb = self._rows(Bn, Y.shape[1])
         if loss is None:
             loss = torch.zeros(1, dtype=torch.float64, device=self.dev)
-        nat.check(nat.lib().otb_mlp_mse_grad(Y.data_ptr(), T.contiguous().data_ptr(), dZf.data_ptr(),
-                                             dZb.data_ptr(), n, loss.data_ptr(), None))
-        Bn = Y.shape[0]
-        gW, gb = [None] * len(self.W), [None] * len(self.W)
-        for l in reversed(range(len(self.W))):
+        nat.check(nat.lib().otb_mlp_mse_grad_rows(Y.data_ptr(), T.contiguous().data_ptr(), dZf.data_ptr(),
+                                                  dZb.data_ptr(), Bn, Y.shape[1], dZb.stride(0),
+                                                  loss.data_ptr(), None))
+        n = len(self.W)
+        gW, gb, dZ = [None] * n, [None] * n, [None] * n
+        for l in reversed(range(n)):
             fout, fin = self.W[l].shape
+            dZ[l] = dZf
+            # the weight gradient reads both operands as they lie ([batch][features])
             gW[l] = torch.empty((fout, fin), device=self.dev)
-            self._gemm(self._transpose(dZb), self._transpose(Hs[l]), fout, fin, Bn, outf=gW[l])
+            self._gemm(dZb, 1, Hs[l], 1, fout, fin, Bn, outf=gW[l])
             gb[l] = torch.empty(fout, device=self.dev)
-            nat.check(nat.lib().otb_mlp_colsum(dZf.data_ptr(), gb[l].data_ptr(), Bn, fout, None))
             if l > 0:
                 nf = torch.empty((Bn, fin), device=self.dev)
-                nb = torch.empty((Bn, fin), dtype=torch.bfloat16, device=self.dev)
-                self._gemm(dZb, self.WbT[l], Bn, fin, fout, epi=2, zin=Zs[l - 1], outf=nf, outb=nb)
+                nb = self._rows(Bn, fin)
+                self._gemm(dZb, 0, self.WbT[l], 0, Bn, fin, fout, epi=2, zin=Zs[l - 1], outf=nf, outb=nb)
                 dZf, dZb = nf, nb
+        for k in range(0, n, 32):              # up to 32 layers a launch
+            part = range(k, min(k + 32, n))
+            P = ctypes.c_void_p * len(part)
+            nat.check(nat.lib().otb_mlp_colsums(
+                len(part), P(*[dZ[l].data_ptr() for l in part]), P(*[gb[l].data_ptr() for l in part]), Bn,
+                (ctypes.c_int32 * len(part))(*[self.W[l].shape[0] for l in part]), None))
         self._cache = None
         return loss, gW, gb
 
     def step(self, gW, gb, lr=1e-3, weight_decay=0.0, beta1=0.9, beta2=0.999, eps=1e-8):
         self.steps += 1
-        L = nat.lib()
-        for l in range(len(self.W)):
-            nat.check(L.otb_mlp_adamw(self.W[l].data_ptr(), gW[l].data_ptr(), self.m[l].data_ptr(),
-                                      self.v[l].data_ptr(), self.Wb[l].data_ptr(), self.W[l].numel(),
-                                      lr, beta1, beta2, eps, weight_decay, self.steps, None))
-            nat.check(L.otb_mlp_adamw(self.b[l].data_ptr(), gb[l].data_ptr(), self.mb[l].data_ptr(),
-                                      self.vb[l].data_ptr(), None, self.b[l].numel(), lr, beta1, beta2,
-                                      eps, 0.0, self.steps, None))
-            w = self.Wb[l]
-            nat.check(L.otb_mlp_transpose_bf16(w.data_ptr(), self.WbT[l].data_ptr(), w.shape[0],
-                                               w.shape[1], None))
+        n = len(self.W)
+        layers = (nat.MlpLayer * n)()
+        for l in range(n):
+            fout, fin = self.W[l].shape
+            layers[l] = nat.MlpLayer(
+                fout, fin, self.Wb[l].stride(0), self.WbT[l].stride(0), self.W[l].data_ptr(), self.m[l].data_ptr(),
+                self.v[l].data_ptr(), self.b[l].data_ptr(), self.mb[l].data_ptr(), self.vb[l].data_ptr(),
+                gW[l].data_ptr(), gb[l].data_ptr(), self.Wb[l].data_ptr(), self.WbT[l].data_ptr())
+        for k in range(0, n, 32):              # up to 32 layers a launch
+            nat.check(nat.lib().otb_mlp_adamw_net(min(32, n - k), ctypes.byref(layers[k]), lr, beta1, beta2, eps,
+                                                  weight_decay, self.steps, None))
 
     def check_errors(self):
         if int(self.err.item()) != 0:
