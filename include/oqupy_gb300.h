@@ -288,7 +288,7 @@ otb_status otb_dyn_gradient(otb_pt* h, int32_t inst, int32_t n_systems,
  * every device allocation, or code running where cudaMalloc is not allowed:
  * the caller allocates all device buffers below, and the TEMPO step's
  * working memory comes from a fixed device array inside the library
- * (1 MiB, present on every GPU that loads the library until exit), which
+ * (1.5 MiB, present on every GPU that loads the library until exit), which
  * limits bonds to chi_cap * D <= OTB_TEMPO_STATIC_MAX_CHI_D.
  *
  * One instance, one CTA.  Every call looks up the array's device address

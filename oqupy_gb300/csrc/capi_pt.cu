@@ -149,7 +149,7 @@ extern "C" otb_status otb_pt_create(const otb_pt_config* cfg, int32_t n, const o
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   h->grid = cfg->grid > 0 ? cfg->grid : std::max(1, std::min(n, 2 * std::max(sms, 1)));
   h->wcap = (long long)(h->cap * h->Dmax) * (h->cap * h->Dmax);
-  h->work_stride = pt_work_bytes(h->wcap);
+  h->work_stride = pt_work_bytes(h->wcap, h->precision == 1);
   if (!h->d_work.alloc((size_t)h->grid * h->work_stride)) return OTB_ERR_OOM;
   *out = h.release();
   return OTB_OK;

@@ -297,7 +297,7 @@ extern "C" otb_status otb_tempo_create(const otb_tempo_config* cfg, int32_t n,
   // switch shapes later (an explicit grid fixes it)
   h->grid_alloc = cfg->grid > 0 ? cfg->grid : std::max(h->grid, std::min(n, 2 * h->sms));
   h->wcap = (long long)(h->cap * h->Dmax) * (h->cap * h->Dmax);
-  h->work_stride = tempo_work_bytes(h->wcap);
+  h->work_stride = tempo_work_bytes(h->wcap, h->precision == OTB_PRECISION_MIXED);
   if (!h->d_work.alloc((size_t)h->grid_alloc * h->work_stride)) return OTB_ERR_OOM;
   *out = h.release();
   return OTB_OK;

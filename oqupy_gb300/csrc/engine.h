@@ -65,8 +65,10 @@ struct TempoLaunch {
 constexpr long long QR_BOOK_BYTES = 48 * 1024;
 
 // Per-CTA workspace: four matrices of wcap 16-byte elements (the QR's row
-// factor, theta / temporaries, carry, the split's working matrix).
-inline long long tempo_work_bytes(long long wcap) { return wcap * (4 * 16) + QR_BOOK_BYTES; }
+// factor, theta / temporaries, carry, the split's working matrix) and, in FP64,
+// two for the split's orthogonalisation.
+constexpr long long tempo_mat_bytes(long long wcap, bool mixed) { return wcap * 16 * (mixed ? 4 : 6); }
+inline long long tempo_work_bytes(long long wcap, bool mixed) { return tempo_mat_bytes(wcap, mixed) + QR_BOOK_BYTES; }
 
 // precision: 0 = complex128 (FP64), 1 = mixed (double-float on the FP32 pipe;
 // FP64 rank decisions and read-out)
@@ -124,8 +126,10 @@ struct PtLaunch {
 };
 
 // Per-CTA PT workspace: five matrices of wcap 16-byte elements (U, carry,
-// theta, the QR's row factor, the split's working matrix).
-inline long long pt_work_bytes(long long wcap) { return wcap * (5 * 16) + QR_BOOK_BYTES; }
+// theta, the QR's row factor, the split's working matrix) and, in FP64, two for
+// the split's orthogonalisation.
+constexpr long long pt_mat_bytes(long long wcap, bool mixed) { return wcap * 16 * (mixed ? 5 : 7); }
+inline long long pt_work_bytes(long long wcap, bool mixed) { return pt_mat_bytes(wcap, mixed) + QR_BOOK_BYTES; }
 
 cudaError_t launch_pt(const PtLaunch& L, int precision, int grid, int block, cudaStream_t stream);
 

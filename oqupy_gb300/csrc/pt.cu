@@ -128,6 +128,7 @@ __device__ int split_generic(const Acc& X, int m, int n, double epsrel, float qr
       const int pj = perm[j];
       const zc* u = W + (size_t)pj * m;
       zc acc = mk<double>(0, 0);
+#pragma unroll 4
       for (int row = 0; row < m; ++row) cjfma(acc, u[row], X(row, col));
       b.Cg[idx] = cscale(acc, sinv[pj]);
     }
@@ -137,6 +138,7 @@ __device__ int split_generic(const Acc& X, int m, int n, double epsrel, float qr
       const int pj = perm[j];
       const zc* w = W + (size_t)pj * n;
       zc acc = mk<double>(0, 0);
+#pragma unroll 4
       for (int col = 0; col < n; ++col) cfma(acc, X(row, col), w[col]);
       b.Tg[idx] = cscale(acc, sinv[pj]);
     }
@@ -185,6 +187,7 @@ __device__ void sweep_rl(PtCtx<MIXED>& c, PtShared& sh, int k) {
     const zc* brow = B + (size_t)la * n;
     const zc* crow = c.b.Cg + (size_t)j * n;
     zc acc = mk<double>(0, 0);
+#pragma unroll 4
     for (int q = 0; q < n; ++q) cfma(acc, brow[q], crow[q]);
     c.Xg[idx] = acc;
   }
@@ -223,6 +226,7 @@ __device__ void sweep_lr(PtCtx<MIXED>& c, PtShared& sh, int k) {
     const int j = idx / (Db * r2), ar = idx - j * (Db * r2);
     const zc* crow = c.b.Cg + (size_t)j * n;
     zc acc = mk<double>(0, 0);
+#pragma unroll 4
     for (int q = 0; q < n; ++q) cfma(acc, crow[q], B[(size_t)q * (Db * r2) + ar]);
     c.Xg[idx] = acc;
   }
@@ -339,6 +343,7 @@ __device__ void pt_step(PtCtx<MIXED>& c, PtShared& sh) {
         default: coef = Im[a * D + a]; mc = 0; break;
       }
       zc acc = mk<double>(0, 0);
+#pragma unroll 4
       for (int rr = 0; rr < r; ++rr)
         cfma(acc, A[((size_t)ll * Da + ain) * r + rr], C[(size_t)x * (crd * cmd) + rr * cmd + mc]);
       c.Xg[idx] = cmul(coef, acc);
@@ -398,6 +403,7 @@ __device__ void pt_caps(PtCtx<MIXED>& c, PtShared& sh) {
       zc acc = mk<double>(0, 0);
       for (int i = 0; i < dd; ++i) {
         const int a = i * (dd + 1);  // diagonal Liouville index (i, i)
+#pragma unroll 4
         for (int rr = 0; rr < r; ++rr) cfma(acc, A[((size_t)ll * D + a) * r + rr], nxt[rr]);
       }
       // d * (1/d) from the rank-3 factor and trace_square
@@ -436,7 +442,8 @@ __global__ void __launch_bounds__(PT_THREADS) pt_kernel(PtLaunch L) {
     c.Xg = c.b.Cg + L.wcap;
     c.b.sb.Wg = c.Xg + L.wcap;
     c.b.sb.Xg = c.Xg + 2 * L.wcap;
-    c.b.sb.bkg = work + L.wcap * 80;
+    c.b.sb.Mg = c.Xg + 3 * L.wcap;
+    c.b.sb.bkg = work + pt_mat_bytes(L.wcap, MIXED);
     c.b.sb.smem = dsm;
     c.b.sb.smem_bytes = L.smem_bytes;
     if (threadIdx.x == 0) sh.st = L.state[i];

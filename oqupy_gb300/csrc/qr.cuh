@@ -29,7 +29,7 @@
 
 #include <climits>
 
-#include "jacobi.cuh"
+#include "orthogonal.cuh"
 
 namespace otb {
 
@@ -350,7 +350,7 @@ __device__ int jacobi_norms(typename QA<T>::E* W, int m, int n, int ld, double s
 }
 
 // The split driver on X (R x N, ld R, the oriented matrix over `scale`, a
-// power of two; destroyed), with Zg (R x N elements) as spare global storage,
+// power of two; destroyed), with Zg (R x N elements; FP64: and Mg, 2 N^2) as spare global storage,
 // zs / zs_bytes spare shared memory and bkg spare global bookkeeping of
 // qr_book_bytes(N).  x_shared says whether X itself is in shared memory.
 // delta <= 0 selects the default cut.  Returns the kept rank; *Wout holds
@@ -358,9 +358,9 @@ __device__ int jacobi_norms(typename QA<T>::E* W, int m, int n, int ld, double s
 // units of A) / book->perm describing its columns in descending order.
 template <typename T>
 __device__ int qr_jacobi_truncate(typename QA<T>::E* X, bool x_shared, int R, int N, double scale,
-                                  typename QA<T>::E* Zg, unsigned char* zs, size_t zs_bytes, unsigned char* bkg,
-                                  double epsrel, float delta, SplitBook* book, JacobiShared* sh,
-                                  typename QA<T>::E** Wout) {
+                                  typename QA<T>::E* Zg, typename QA<T>::E* Mg, unsigned char* zs,
+                                  size_t zs_bytes, unsigned char* bkg, double epsrel, float delta, SplitBook* book,
+                                  JacobiShared* sh, typename QA<T>::E** Wout) {
   typedef QA<T> Q;
   typedef typename Q::E E;
   typedef typename Q::S S;
@@ -405,6 +405,15 @@ __device__ int qr_jacobi_truncate(typename QA<T>::E* X, bool x_shared, int R, in
     E* Y = X + (size_t)k * k;
     S* rinv = bk.rinv<S>();
     plain_qr<T>(Z, N, k, R2, rinv, bk.n2<S>(0));
+    if constexpr (!Q::kFF) {
+      if (k >= PRESWEEP_MIN_COLS) {   // 4 k^2 <= R N
+        E* W2 = presweep(R2, k, k, R2 + (size_t)k * k, R2 + (size_t)2 * k * k, reinterpret_cast<float*>(norm));
+        if (W2 != R2) {
+          for (int idx = tid; idx < k * k; idx += nt) R2[idx] = W2[idx];
+          __syncthreads();
+        }
+      }
+    }
     const int sw64 = jacobi_norms<T>(R2, k, k, k, scale, norm, sh);
     const int kk = jacobi_rank(k, epsrel, norm, perm, sh, sw64, t2);
     for (int idx = tid; idx < k * kk; idx += nt) {
@@ -417,6 +426,7 @@ __device__ int qr_jacobi_truncate(typename QA<T>::E* X, bool x_shared, int R, in
       const int j = idx / N, r = idx - j * N;
       const E* y = R2 + (size_t)perm[j] * k;
       typename Q::Acc acc = Q::acc_zero();
+#pragma unroll 4
       for (int i = 0; i < k; ++i) Q::acc_fma(acc, Z[(size_t)i * N + r], y[i]);
       Y[idx] = Q::acc_value(acc);
     }
@@ -430,6 +440,26 @@ __device__ int qr_jacobi_truncate(typename QA<T>::E* X, bool x_shared, int R, in
     __syncthreads();
     *Wout = Y;
     return kk;
+  }
+  if constexpr (!Q::kFF) {
+    if (k >= PRESWEEP_MIN_COLS) {
+      // scratch in X's storage (behind Z, when Z moved there) where it fits,
+      // else in spare shared or global memory
+      const size_t xfree = (size_t)R * N;
+      size_t off = Z == X ? (size_t)N * k : 0;
+      E* tmp = Zg;   // Z is in X: its global home is free
+      if (off + (size_t)N * k <= xfree) {
+        tmp = X + off;
+        off += (size_t)N * k;
+      }
+      E* mats = Mg;
+      if (off + presweep_mats(k) <= xfree)
+        mats = X + off;
+      else if (reinterpret_cast<unsigned char*>(Z) == zs &&
+               ((size_t)N * k + presweep_mats(k)) * sizeof(E) <= zs_bytes)
+        mats = reinterpret_cast<E*>(zs) + (size_t)N * k;
+      Z = presweep(Z, N, k, tmp, mats, reinterpret_cast<float*>(norm));
+    }
   }
   const int sw64 = jacobi_norms<T>(Z, N, k, N, scale, norm, sh);
   const int kk = jacobi_rank(k, epsrel, norm, perm, sh, sw64, t2);

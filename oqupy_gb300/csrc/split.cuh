@@ -37,6 +37,7 @@ struct SplitShared {
 struct SplitBufs {
   void* Wg;             // spare matrix (the QR's row factor when it does not fit in shared memory)
   void* Xg;             // working matrix when it does not fit in shared memory
+  void* Mg;             // FP64: two more, for the orthogonalisation's products
   unsigned char* bkg;   // QR bookkeeping of more than 383 columns when shared memory is too small
   unsigned char* smem;
   int smem_bytes;
@@ -82,8 +83,9 @@ __device__ __forceinline__ SplitOut<T> oriented_split(const Acc& A, int R, int N
   o.flip = N >= QR_MIN_COLS;
   if (o.flip) {
     const size_t used = x_shared ? xbytes : 0;
-    o.kk = qr_jacobi_truncate<T>(X, x_shared, R, N, scale, reinterpret_cast<E*>(b.Wg), b.smem + used,
-                                 (size_t)b.smem_bytes - used, b.bkg, epsrel, qr_delta, &sh.book, &sh.jsh, &o.W);
+    o.kk = qr_jacobi_truncate<T>(X, x_shared, R, N, scale, reinterpret_cast<E*>(b.Wg), reinterpret_cast<E*>(b.Mg),
+                                 b.smem + used, (size_t)b.smem_bytes - used, b.bkg, epsrel, qr_delta, &sh.book,
+                                 &sh.jsh, &o.W);
     return o;
   }
   const int sw64 = jacobi_norms<T>(X, R, N, R, scale, sh.book.norm, &sh.jsh);

@@ -163,6 +163,7 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, const 
     for (int idx = tid; idx < D * r1; idx += nt) {
       const int a = idx / r1, rr = idx - a * r1;
       Acc f = Q::acc_zero();
+#pragma unroll 4
       for (int c = 0; c < r0; ++c) Q::acc_fma(f, Cf[c], A1[((long long)c * D + a) * r1 + rr]);
       Tf[idx] = Q::acc_value(f);
     }
@@ -208,6 +209,7 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, const 
         Q::acc_fma(f, sh.pf[2][a * D + mr], A[a * r + rr]);
       } else {
         Acc g = Q::acc_zero();
+#pragma unroll 4
         for (int c = 0; c < ccd; ++c)
           Q::acc_fma(g, Cf[(long long)x * (ccd * D) + c * D + mr], A[((long long)c * D + a) * r + rr]);
         Q::acc_fma(f, sh.pf[2][a * D + mr], Q::acc_value(g));
@@ -254,6 +256,7 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, const 
         const E* u = W + (long long)pj * m;
         const E* th = Tf + (long long)col * m;
         Acc f = Q::acc_zero();
+#pragma unroll 4
         for (int row = 0; row < m; ++row) Q::acc_fmaj(f, u[row], th[row]);
         Cf[idx] = Q::scaleE(Q::acc_value(f), sinv[pj]);
       }
@@ -265,6 +268,7 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, const 
         const int pj = sh.ss.book.perm[j];
         const E* w = W + (long long)pj * n;
         Acc f = Q::acc_zero();
+#pragma unroll 4
         for (int col = 0; col < n; ++col) Q::acc_fma(f, Tf[(long long)col * m + row], w[col]);
         A[idx] = Q::scaleE(Q::acc_value(f), sinv[pj]);
       }
@@ -313,6 +317,7 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, const 
           const E* u = W + (long long)pj * m;
           const E* y = A + (long long)col * m;
           Acc f = Q::acc_zero();
+#pragma unroll 4
           for (int row = 0; row < m; ++row) Q::acc_fmaj(f, u[row], y[row]);
           Cf[idx] = Q::scaleE(Q::acc_value(f), sinv[pj]);
         }
@@ -330,6 +335,7 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, const 
           const int pj = sh.ss.book.perm[j];
           const E* w = W + (long long)pj * n;
           Acc f = Q::acc_zero();
+#pragma unroll 4
           for (int col = 0; col < n; ++col) Q::acc_fma(f, A[(long long)col * m + row], w[col]);
           Tf[idx] = Q::scaleE(Q::acc_value(f), sinv[pj]);
         }
@@ -350,6 +356,7 @@ __device__ void tempo_step(const TempoLaunch& L, const InstDev& I, int i, const 
         const E* brow = B + (long long)la * n;
         const E* crow = Cf + (long long)j * n;
         Acc f = Q::acc_zero();
+#pragma unroll 4
         for (int c = 0; c < n; ++c) Q::acc_fma(f, brow[c], crow[c]);
         Tf[idx] = Q::acc_value(f);
       }
@@ -442,7 +449,8 @@ __global__ void __launch_bounds__(TEMPO_THREADS, 1) tempo_kernel(TempoLaunch L) 
   b.Tg = work + L.wcap * 16;
   b.Cg = work + L.wcap * 32;
   b.sb.Xg = work + L.wcap * 48;
-  b.sb.bkg = work + L.wcap * 64;
+  b.sb.Mg = work + L.wcap * 64;
+  b.sb.bkg = work + tempo_mat_bytes(L.wcap, MIXED);
   b.sb.smem = dsm;
   b.sb.smem_bytes = L.smem_bytes;
   for (;;) {
@@ -558,12 +566,12 @@ cudaError_t launch_tempo(const TempoLaunch& L, int precision, int grid, int bloc
 // or code running where cudaMalloc is not allowed) pass all device buffers in
 // and get the TEMPO step's working memory from this file-scope array.  It is
 // one CTA's workspace for splits of at most (chi_cap * D) columns with
-// chi_cap * D <= 128: 128 * 128 * 64 bytes = 1 MiB, held by every GPU that
+// chi_cap * D <= 128: 128 * 128 * 96 bytes = 1.5 MiB, held by every GPU that
 // loads the library until the process exits.  No part of it has to start at
 // zero: every workspace matrix is written before it is read.
 constexpr int STATIC_MAX_CHI_D = 128;
 constexpr long long STATIC_WCAP = (long long)STATIC_MAX_CHI_D * STATIC_MAX_CHI_D;
-constexpr long long STATIC_SCRATCH_BYTES = STATIC_WCAP * (3 * 16 + 16);
+constexpr long long STATIC_SCRATCH_BYTES = tempo_mat_bytes(STATIC_WCAP, false);
 static __device__ __align__(256) unsigned char g_tempo_static_scratch[STATIC_SCRATCH_BYTES];
 
 template <bool MIXED>
@@ -583,6 +591,7 @@ __global__ void __launch_bounds__(STATIC_THREADS)
   b.Tg = work + L.wcap * 16;
   b.Cg = work + L.wcap * 32;
   b.sb.Xg = work + L.wcap * 48;
+  b.sb.Mg = work + L.wcap * 64;
   b.sb.bkg = nullptr;   // chi_cap * D <= 128: the bookkeeping always fits in shared memory
   b.sb.smem = dsm;
   b.sb.smem_bytes = L.smem_bytes;

@@ -1,7 +1,8 @@
 """The truncated bond split on the GPU at the shapes where it can go wrong:
 rank-deficient operands (a bath of zero coupling leaves product states, so
-every split has exactly zero columns), and rounding that must not depend on the
-launch shape or on the rest of the batch."""
+every split has exactly zero columns), operands from below the width at which
+they are orthogonalised by products up to the widest register form, and rounding
+that must not depend on the launch shape or on the rest of the batch."""
 import numpy as np
 import pytest
 
@@ -54,3 +55,38 @@ def test_rounding_is_independent_of_launch_shape_and_batch(precision):
         np.testing.assert_array_equal(states(insts, 16, precision, **kw), ref)
     for i in range(3):
         np.testing.assert_array_equal(states([insts[i]], 16, precision)[0], ref[i])
+
+
+def qutrit(dkmax, epsrel):
+    from oqupy_gb300 import bath
+    infl, _ = bath.influences(0.15, 3.0, 3.0, "exponential", 1.0, 0.05, dkmax, np.diag([1.0, 0.0, -1.0]))
+    rng = np.random.default_rng(5)
+    g = rng.normal(size=(3, 3)) + 1j * rng.normal(size=(3, 3))
+    h = 0.5 * (g + g.conj().T)
+    p1, p2 = bath.half_step_propagators(h / np.linalg.norm(h, 2), 0.05)
+    return dict(hs_dim=3, dkmax=dkmax, epsrel=epsrel, influences=infl, prop1=p1, prop2=p2,
+                rho0=np.diag([1.0, 0.0, 0.0]).astype(complex))
+
+
+@pytest.mark.parametrize("shape", [dict(), dict(block=512, smem_kb=200), dict(block=256, smem_kb=8)])
+@pytest.mark.parametrize("make, steps", [(lambda: spin_boson(0.05, 2, 1e-12), 12),   # narrow: up to 12 columns
+                                         (lambda: spin_boson(0.3, 7, 1e-12), 12),
+                                         (lambda: spin_boson(0.3, 7, 1e-12, eps=0.0), 12),   # symmetric: equal pairs
+                                         (lambda: qutrit(4, 1e-12), 5)])
+def test_complex128_split_matches_the_oracle(make, steps, shape):
+    """Operands on either side of the width for the product form, with working
+    matrices in shared and in global memory.  Both sides drop at most
+    epsrel s_0 = 1e-12 per split, at most 16 splits a step: 192 splits and a
+    factor of 2 for the two sides give 4e-10."""
+    from oracle import tempo_oracle as to
+    from oqupy_gb300.tempo import TempoBatch
+    inst = make()
+    infl = inst["influences"]
+    want, _ = to.tempo_dynamics(inst["rho0"].reshape(-1), lambda dk: infl[dk] if 0 <= dk < len(infl) else None,
+                                np.eye(inst["hs_dim"]), lambda s: (inst["prop1"], inst["prop2"]),
+                                inst["dkmax"], inst["epsrel"], steps)
+    b = TempoBatch([inst], precision="complex128", chi_cap=128, out_cap=steps + 1, **shape)
+    b.advance(steps)
+    got = b.states(0, steps + 1)[0]
+    b.close()
+    np.testing.assert_allclose(got, want, atol=4e-10)
