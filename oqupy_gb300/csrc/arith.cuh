@@ -29,6 +29,20 @@ __device__ __forceinline__ float rcp_est(float x) {
   return y;
 }
 
+// FP64 -> FP32 by integer instructions: a conversion takes the FP64 pipe like
+// any FP64 instruction.  Truncated (*rest: the cut bits); values below 2^-126
+// are 0, those above the range infinite or NaN.
+__device__ __forceinline__ float trunc32(double d, unsigned* rest = nullptr) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  const unsigned e = (hi >> 20) & 0x7ffu;
+  const unsigned f =
+      (hi & 0x80000000u) | (min(e - 896u, 255u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+  const bool normal = e > 896u;
+  if (rest) *rest = normal ? lo & 0x1fffffffu : 0u;
+  return __uint_as_float(normal ? f : 0u);
+}
+__device__ __forceinline__ cx<float> trunc32(const cx<double>& a) { return mk<float>(trunc32(a.x), trunc32(a.y)); }
+
 template <>
 struct QA<double> {
   typedef cx<double> E;
@@ -55,6 +69,10 @@ struct QA<double> {
     return v;
   }
   static __device__ __forceinline__ S abs2_acc(const E& x, S acc) { return fma(x.x, x.x, fma(x.y, x.y, acc)); }
+  static __device__ __forceinline__ float abs2_32(const E& x, float acc) {
+    const cx<float> y = trunc32(x);
+    return fmaf(y.x, y.x, fmaf(y.y, y.y, acc));
+  }
   // (wr, wi) += conj(a) x
   static __device__ __forceinline__ void dotj(S& wr, S& wi, const E& a, const E& x) {
     wr = fma(a.x, x.x, fma(a.y, x.y, wr));
@@ -179,6 +197,9 @@ struct QA<ff> {
       v = ff_make(s.hi, __fadd_rn(__fadd_rn(v.lo, o.lo), s.lo));
     }
     return v;
+  }
+  static __device__ __forceinline__ float abs2_32(const E& x, float acc) {
+    return fmaf(x.x.hi, x.x.hi, fmaf(x.y.hi, x.y.hi, acc));
   }
   static __device__ __forceinline__ S abs2_acc(const E& x, S acc) {
     ffp_acc(x.x.hi, x.x.lo, x.x.hi, x.x.lo, acc.hi, acc.lo);

@@ -40,7 +40,7 @@ namespace otb {
 // (95 instances, splits of ~77 x 35: the 12 steps take 196 instead of 174 ms).
 constexpr int PRESWEEP_MIN_COLS = 8;
 constexpr int PRESWEEP_CORRECTIONS = 2;
-constexpr float PRESWEEP_MAX_TAN = 4e-6f;
+constexpr float PRESWEEP_MAX_TAN = 4e-6f;   // larger tangents are left to the sweeps
 
 // FP32 one-sided Jacobi sweeps on F (m + k rows, k columns, ld m + k): the
 // inner products run over the first m rows, the rotations over all (the last k
@@ -208,17 +208,7 @@ __device__ __forceinline__ cx<float> product32(const cx<float>* a, int lda, cons
   return mk<float>(sx, sy);
 }
 
-// FP64 -> FP32 and double-float by integer instructions: a conversion takes the
-// FP64 pipe like any FP64 instruction.  Truncated; values below 2^-126 are 0.
-__device__ __forceinline__ float trunc32(double d, unsigned* rest = nullptr) {
-  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
-  const unsigned e = (hi >> 20) & 0x7ffu;
-  const unsigned f = (hi & 0x80000000u) | ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
-  const bool normal = e > 896u;
-  if (rest) *rest = normal ? lo & 0x1fffffffu : 0u;
-  return __uint_as_float(normal ? f : 0u);
-}
-__device__ __forceinline__ cx<float> trunc32(const cx<double>& a) { return mk<float>(trunc32(a.x), trunc32(a.y)); }
+// FP64 -> double-float by integer instructions (trunc32).
 __device__ __forceinline__ ff split32(double d) {
   unsigned rest;
   const float h = trunc32(d, &rest);

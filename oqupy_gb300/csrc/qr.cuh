@@ -147,6 +147,125 @@ __device__ __forceinline__ void project(const typename QA<T>::E* v, typename QA<
   }
 }
 
+// The FP64 form of a step on the columns of X (R rows): with v the pivot column,
+// c <- c - v (v^H c) / |v|^2 for the `nrest` columns list[t] (list[t + 1] from
+// t = pos on), by a group of G lanes each.  out[j ostride] receives column j's
+// inner product v^H c, nkey[t] / nlist[t] its new FP32 squared norm and index.
+// In between, the last warp forms |v|^2 in full: *diag and *rinv receive
+// |v|^2 and 1 / |v|, all others 1 / |v|^2 through *beta_sh.  Ends with a
+// barrier.
+//
+// The columns' own squared norms only rank them and decide the stop, so FP32
+// is enough for all but the pivot's: against project(), which keeps them in the
+// columns' arithmetic and has every warp form the pivot's reciprocal, a column
+// takes 8 instead of 10 multiply-adds an element, a group two reductions less,
+// for one barrier more.  48 instances of splits ~77 x 31: 25100 instead of
+// 35300 clocks a step, bound by the FP64 pipe in both.  Double-float columns
+// keep project(): with one instruction a clock the barrier and the reloads cost
+// what the norms save (splits of ~77 x 35: 16600 and 15600 clocks a step).
+struct GsStep {
+  cx<double>* X;
+  const cx<double>* v;
+  cx<double>*out, *diag;
+  double *rinv, *beta_sh;
+  const float* key;
+  const short* list;
+  float* nkey;
+  short* nlist;
+  size_t ostride;
+  int R, nrest, pos;
+  float v2;
+};
+
+// RC rows a lane at a time.  Both halves read the columns (an element's loads
+// are hidden behind its multiply-adds, 64 clocks each); the inner products wait
+// in `out`.
+template <int G, int RC>
+__device__ __forceinline__ void gs_columns(const GsStep& g) {
+  typedef QA<double> Q;
+  typedef cx<double> E;
+  const int gl = threadIdx.x & (G - 1), group = threadIdx.x / G, ngroups = blockDim.x / G;
+  const int first = (int)(threadIdx.x & ~31u) / G;   // the warp's first group
+  for (int tb = 0; tb + first < g.nrest; tb += ngroups) {
+    const int t = tb + group;
+    const bool act = t < g.nrest;
+    const int p = act ? t + (t >= g.pos ? 1 : 0) : 0;
+    const int j = g.list[p];
+    const E* c = g.X + (size_t)j * g.R;
+    double wr = 0.0, wi = 0.0;
+    for (int r0 = gl; r0 < g.R; r0 += RC * G) {
+      E a[RC], x[RC];
+#pragma unroll
+      for (int q = 0; q < RC; ++q) {
+        const bool in = act && r0 + q * G < g.R;
+        a[q] = in ? g.v[r0 + q * G] : Q::zeroE();
+        x[q] = in ? c[r0 + q * G] : Q::zeroE();
+      }
+#pragma unroll
+      for (int q = 0; q < RC; ++q) Q::dotj(wr, wi, a[q], x[q]);
+    }
+    __syncwarp();
+    Q::dot_sum<G>(wr, wi, inverse_bound(g.v2, g.key[p]));
+    if (act && gl == 0) g.out[j * g.ostride] = mk<double>(wr, wi);
+  }
+  __syncthreads();
+  const double beta = *g.beta_sh;
+  for (int tb = 0; tb + first < g.nrest; tb += ngroups) {
+    const int t = tb + group;
+    const bool act = t < g.nrest;
+    const int j = g.list[act ? t + (t >= g.pos ? 1 : 0) : 0];
+    E* c = g.X + (size_t)j * g.R;
+    float s2 = 0.f;
+    if (act) {
+      const E w = g.out[j * g.ostride];
+      const double bx = Q::mul(beta, w.x), by = Q::mul(beta, w.y);
+      for (int r0 = gl; r0 < g.R; r0 += RC * G) {
+        E x[RC];
+#pragma unroll
+        for (int q = 0; q < RC; ++q) {
+          const bool in = r0 + q * G < g.R;
+          x[q] = in ? Q::sub_scaled(c[r0 + q * G], g.v[r0 + q * G], bx, by) : Q::zeroE();
+          s2 = Q::abs2_32(x[q], s2);
+        }
+#pragma unroll
+        for (int q = 0; q < RC; ++q)
+          if (r0 + q * G < g.R) c[r0 + q * G] = x[q];
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int off = G >> 1; off > 0; off >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, off, 32);
+    if (act && gl == 0) {
+      g.nkey[t] = s2;
+      g.nlist[t] = (short)j;
+    }
+  }
+}
+
+__device__ __forceinline__ void gs_step(const GsStep& g) {
+  typedef QA<double> Q;
+  if (threadIdx.x >> 5 == (blockDim.x >> 5) - 1) {
+    double acc = 0.0;
+    for (int r = threadIdx.x & 31; r < g.R; r += 32) acc = Q::abs2_acc(g.v[r], acc);
+    __syncwarp();
+    acc = Q::group_sum<32>(acc);
+    const double ri = Q::rsqrt(acc);
+    if ((threadIdx.x & 31) == 0) {
+      *g.beta_sh = Q::mul(ri, ri);
+      *g.rinv = ri;
+      *g.diag = Q::realE(acc);
+    }
+  }
+  const int G = qr_group(g.R, g.nrest);
+  if (G == 8)
+    gs_columns<8, 3>(g);
+  else if (G == 16)
+    gs_columns<16, 3>(g);
+  else
+    gs_columns<32, 3>(g);
+  __syncthreads();
+}
+
 // Pivoted Gram-Schmidt QR of X (R x N, column-major ld R; destroyed).
 // Returns k and writes Z (N x k, ld N): Z[q, i] = conj(R[i, q]), zero where
 // column q was chosen before step i; Z's storage holds N x N.  *tail2 is the
@@ -211,38 +330,58 @@ __device__ int pivoted_qr(typename QA<T>::E* X, int R, int N, float delta, const
       break;
     }
     const int p = list[pos];
-    const S np = bk.n2<S>(cur)[pos];
-    const S ri = Q::rsqrt(np);
-    const S beta = Q::mul(ri, ri);
-    if (tid == 0) {
-      bk.rinv<S>()[i] = ri;
-      Z[(size_t)i * N + p] = Q::realE(np);
-    }
-    const E* v = X + (size_t)p * R;
-    const int nrest = n - 1;
-    const int G = qr_group(R, nrest);
-    const int gl = tid & (G - 1), group = tid / G, ngroups = nt / G;
-    for (int tb = 0; tb < nrest; tb += ngroups) {
-      if (tb + (warp * 32) / G >= nrest) break;   // no column left for this warp
-      const int t = tb + group;
-      const bool act = t < nrest;
-      const int q = act ? t + (t >= pos ? 1 : 0) : pos;
-      const int j = list[q];
-      const float rb = inverse_bound(__uint_as_float(best), key[q]);
-      E* cj = X + (size_t)j * R;
-      S wr, wi, s2;
-      project<T>(v, cj, R, G, gl, act, beta, rb, wr, wi, s2);
-      if (act && gl == 0) {
-        bk.n2<S>(nxt)[t] = s2;
-        bk.key(nxt)[t] = Q::tof(s2);
-        bk.list(nxt)[t] = (short)j;
-        E z;
-        z.x = wr;
-        z.y = wi;
-        Z[(size_t)i * N + j] = z;
+    if constexpr (!Q::kFF) {
+      GsStep g;
+      g.X = X;
+      g.v = X + (size_t)p * R;
+      g.out = Z + (size_t)i * N;
+      g.ostride = 1;
+      g.diag = g.out + p;
+      g.rinv = bk.rinv<S>() + i;
+      g.beta_sh = bk.n2<S>(0);
+      g.key = key;
+      g.list = list;
+      g.nkey = bk.key(nxt);
+      g.nlist = bk.list(nxt);
+      g.R = R;
+      g.nrest = n - 1;
+      g.pos = pos;
+      g.v2 = __uint_as_float(best);
+      gs_step(g);
+    } else {
+      const S np = bk.n2<S>(cur)[pos];
+      const S ri = Q::rsqrt(np);
+      const S beta = Q::mul(ri, ri);
+      if (tid == 0) {
+        bk.rinv<S>()[i] = ri;
+        Z[(size_t)i * N + p] = Q::realE(np);
       }
+      const E* v = X + (size_t)p * R;
+      const int nrest = n - 1;
+      const int G = qr_group(R, nrest);
+      const int gl = tid & (G - 1), group = tid / G, ngroups = nt / G;
+      for (int tb = 0; tb < nrest; tb += ngroups) {
+        if (tb + (warp * 32) / G >= nrest) break;   // no column left for this warp
+        const int t = tb + group;
+        const bool act = t < nrest;
+        const int q = act ? t + (t >= pos ? 1 : 0) : pos;
+        const int j = list[q];
+        const float rb = inverse_bound(__uint_as_float(best), key[q]);
+        E* cj = X + (size_t)j * R;
+        S wr, wi, s2;
+        project<T>(v, cj, R, G, gl, act, beta, rb, wr, wi, s2);
+        if (act && gl == 0) {
+          bk.n2<S>(nxt)[t] = s2;
+          bk.key(nxt)[t] = Q::tof(s2);
+          bk.list(nxt)[t] = (short)j;
+          E z;
+          z.x = wr;
+          z.y = wi;
+          Z[(size_t)i * N + j] = z;
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
   __syncthreads();   // a stop at step k leaves warps that may still be reading the keys
   // rows of R: conj(inner products) over the pivot norms
@@ -253,16 +392,16 @@ __device__ int pivoted_qr(typename QA<T>::E* X, int R, int N, float delta, const
 }
 
 // Unpivoted Gram-Schmidt QR of Z (M x K, M >= K, column-major ld M), in place:
-// on return column i of Z is 1 / rinv[i] times the i-th column of Q and R2
+// on return column i of Z is 1 / bk.rinv()[i] times the i-th column of Q and R2
 // (K x K, ld K) holds R.  Like pivoted_qr without the search.  Q is not used
 // as an orthogonal matrix: Z V = Q (R2 V) holds to rounding whatever its
 // orthogonality, and R2 is backward stable.
 template <typename T>
-__device__ void plain_qr(typename QA<T>::E* Z, int M, int K, typename QA<T>::E* R2, typename QA<T>::S* rinv,
-                         typename QA<T>::S* n2) {
+__device__ void plain_qr(typename QA<T>::E* Z, int M, int K, typename QA<T>::E* R2, const QrBook& bk) {
   typedef QA<T> Q;
   typedef typename Q::E E;
   typedef typename Q::S S;
+  S *rinv = bk.rinv<S>(), *n2 = bk.n2<S>(0);
   const int tid = threadIdx.x, nt = blockDim.x, lane32 = tid & 31;
   for (int j = tid >> 5; j < K; j += nt >> 5) {
     S acc = Q::zero();
@@ -272,36 +411,65 @@ __device__ void plain_qr(typename QA<T>::E* Z, int M, int K, typename QA<T>::E* 
   }
   for (int idx = tid; idx < K * K; idx += nt) R2[idx] = Q::zeroE();
   __syncthreads();
-  for (int i = 0; i < K; ++i) {
-    const S np = n2[i];
-    const S ri = Q::rsqrt(np);
-    const S beta = Q::mul(ri, ri);
-    if (tid == 0) {
-      rinv[i] = ri;
-      R2[(size_t)i * K + i] = Q::realE(np);
-    }
-    const E* v = Z + (size_t)i * M;
-    const int nrest = K - i - 1;
-    const int G = qr_group(M, nrest);
-    const int gl = tid & (G - 1), group = tid / G, ngroups = nt / G;
-    for (int tb = 0; tb < nrest; tb += ngroups) {
-      if (tb + (tid >> 5) * 32 / G >= nrest) break;
-      const int t = tb + group;
-      const bool act = t < nrest;
-      E* cj = Z + (size_t)(act ? i + 1 + t : i) * M;
-      S wr, wi, s2;
-      const int j = act ? i + 1 + t : i;
-      const float rb = inverse_bound(Q::tof(np), Q::tof(n2[j]));
-      project<T>(v, cj, M, G, gl, act, beta, rb, wr, wi, s2);
-      if (act && gl == 0) n2[j] = s2;
-      if (act && gl == 0) {
-        E z;
-        z.x = wr;
-        z.y = wi;
-        R2[(size_t)(i + 1 + t) * K + i] = z;
-      }
+  if constexpr (!Q::kFF) {
+    float* key = bk.key(0);
+    short* list = bk.list(0);
+    for (int j = tid; j < K; j += nt) {
+      key[j] = (float)n2[j];
+      list[j] = (short)j;
     }
     __syncthreads();
+    for (int i = 0; i < K; ++i) {
+      GsStep g;
+      g.X = Z;
+      g.v = Z + (size_t)i * M;
+      g.out = R2 + i;
+      g.ostride = K;
+      g.diag = g.out + (size_t)i * K;
+      g.rinv = rinv + i;
+      g.beta_sh = n2;
+      g.key = key + i + 1;
+      g.nkey = key + i + 1;
+      g.list = list + i + 1;
+      g.nlist = list + i + 1;
+      g.R = M;
+      g.nrest = K - i - 1;
+      g.pos = INT_MAX;
+      g.v2 = key[i];
+      gs_step(g);
+    }
+  } else {
+    for (int i = 0; i < K; ++i) {
+      const S np = n2[i];
+      const S ri = Q::rsqrt(np);
+      const S beta = Q::mul(ri, ri);
+      if (tid == 0) {
+        rinv[i] = ri;
+        R2[(size_t)i * K + i] = Q::realE(np);
+      }
+      const E* v = Z + (size_t)i * M;
+      const int nrest = K - i - 1;
+      const int G = qr_group(M, nrest);
+      const int gl = tid & (G - 1), group = tid / G, ngroups = nt / G;
+      for (int tb = 0; tb < nrest; tb += ngroups) {
+        if (tb + (tid >> 5) * 32 / G >= nrest) break;
+        const int t = tb + group;
+        const bool act = t < nrest;
+        E* cj = Z + (size_t)(act ? i + 1 + t : i) * M;
+        S wr, wi, s2;
+        const int j = act ? i + 1 + t : i;
+        const float rb = inverse_bound(Q::tof(np), Q::tof(n2[j]));
+        project<T>(v, cj, M, G, gl, act, beta, rb, wr, wi, s2);
+        if (act && gl == 0) n2[j] = s2;
+        if (act && gl == 0) {
+          E z;
+          z.x = wr;
+          z.y = wi;
+          R2[(size_t)(i + 1 + t) * K + i] = z;
+        }
+      }
+      __syncthreads();
+    }
   }
   for (int idx = tid; idx < K * K; idx += nt) R2[idx] = Q::scaleE(R2[idx], rinv[idx % K]);
   __syncthreads();
@@ -404,7 +572,7 @@ __device__ int qr_jacobi_truncate(typename QA<T>::E* X, bool x_shared, int R, in
     E* R2 = X;
     E* Y = X + (size_t)k * k;
     S* rinv = bk.rinv<S>();
-    plain_qr<T>(Z, N, k, R2, rinv, bk.n2<S>(0));
+    plain_qr<T>(Z, N, k, R2, bk);
     if constexpr (!Q::kFF) {
       if (k >= PRESWEEP_MIN_COLS) {   // 4 k^2 <= R N
         E* W2 = presweep(R2, k, k, R2 + (size_t)k * k, R2 + (size_t)2 * k * k, reinterpret_cast<float*>(norm));
