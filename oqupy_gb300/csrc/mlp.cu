@@ -179,35 +179,6 @@ __device__ __forceinline__ void epilogue16(const GemmOut& o, const uint32_t* r, 
   if (o.outb) store16(o.outb + row * o.ldb + col, v, n);
 }
 
-// A warp's 32 x 32 block (lane = row, v = its 32 columns) to row-major memory
-// through its shared buffer (rows 33 words apart), so that a store writes whole
-// 128-byte row segments instead of 32 scattered pieces.
-__device__ __forceinline__ void store_block(float* buf, const float* v, float* dst, int ld, int rows) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int q = 0; q < 32; ++q) buf[lane * 33 + q] = v[q];
-  __syncwarp();
-  for (int i = 0; i < rows; ++i) dst[(size_t)i * ld + lane] = buf[i * 33 + lane];
-  __syncwarp();
-}
-__device__ __forceinline__ void store_block(float* buf, const float* v, __nv_bfloat16* dst, int ld, int rows) {
-  const int lane = threadIdx.x & 31;
-  uint32_t* b = reinterpret_cast<uint32_t*>(buf);   // rows 17 words apart
-#pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    union {
-      uint32_t u;
-      __nv_bfloat162 h;
-    } t;
-    t.h = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-    b[lane * 17 + q] = t.u;
-  }
-  __syncwarp();
-  for (int i = lane >> 4; i < rows; i += 2)   // two rows of 64 bytes a store
-    *reinterpret_cast<uint32_t*>(dst + (size_t)i * ld + 2 * (lane & 15)) = b[i * 17 + (lane & 15)];
-  __syncwarp();
-}
-
 __device__ __forceinline__ bool tc_wait_phase(uint64_t* mbar, int phase) {
   uint32_t done = 0;
   for (long long it = 0; it < TC_WAIT_LIMIT && !done; ++it) {
@@ -355,10 +326,13 @@ __global__ void __launch_bounds__(TC_THREADS)
 // result's write to memory.  The two-stage kernel above (cp.async staging by
 // the warps that also issue the products and run the epilogue, scalar stores)
 // reached 79 TFLOP/s on a 60001-point inference of a 5-512x4-1500 network
-// (2370 us); with this one the inference takes 453 us (492 us with every lane
-// storing pieces of its own row).  A training step of 256 points, where the
-// 1500-column operands were staged element by element and both operands of
-// every weight gradient transposed first: 1020 -> 327 us, launches 45 -> 19.
+// (2370 us); with this one the inference takes 438 us.  bf16 rows and
+// pre-activations are stored by the lane that holds them (a 512-wide hidden
+// layer takes 72 us, 78 through shared memory), FP32 results through shared
+// memory as whole row segments (output layer 144 us, 190 without).  A training
+// step of 256 points, where the 1500-column operands were staged element by
+// element and both operands of every weight gradient transposed first: 1020 ->
+// 312 us, launches 45 -> 19.
 //
 // Used when rows are 16-byte aligned; other operands keep the kernel above.
 // Tile width: 256 where that gives every SM a tile, else 128, else 64 (a
@@ -368,7 +342,7 @@ constexpr int TM_EPI_WARPS = 8;
 constexpr int TM_THREADS = 64 + 32 * TM_EPI_WARPS;
 constexpr unsigned long long TM_WAIT_NS = 2000000000ull;
 
-constexpr int TM_XPOSE = 32 * 33 * 4;   // an epilogue warp's transposition buffer
+constexpr int TM_XPOSE = 32 * 33 * 4;   // an epilogue warp's transposition buffer (rows 33 words apart)
 
 template <int BN>
 struct TmShape {
@@ -558,21 +532,26 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
         if (rows <= 0) continue;
         const int col = n0 + c0;
         if (col + 32 <= N) {
-          // rows past the matrix read row 0's pre-activations and are not stored
-          float v[32], z[32];
-          fused_step<32>(out, r, (size_t)(row < M ? row : row0) * out.ldf + col, col, 32, v, z);
-          const size_t at = (size_t)row0 * out.ldf + col;
-          if (out.epi == EPI_GELU && out.zout) store_block(xbuf, z, out.zout + at, out.ldf, rows);
-          if (out.outf) store_block(xbuf, v, out.outf + at, out.ldf, rows);
-          if (out.outb) {
-            if ((out.ldb & 1) || (reinterpret_cast<uintptr_t>(out.outb) & 3)) {
-              if (row < M) {
-                store16(out.outb + (size_t)row * out.ldb + col, v, 16);
-                store16(out.outb + (size_t)row * out.ldb + col + 16, v + 16, 16);
-              }
-            } else {
-              store_block(xbuf, v, out.outb + (size_t)row0 * out.ldb + col, out.ldb, rows);
+          // bf16 rows and pre-activations as 32- and 64-byte pieces of the lane's
+          // own row; FP32 results, twice the bytes, as whole row segments
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            float v[16], z[16];
+            // rows past the matrix read row 0's pre-activations and are not stored
+            fused_step<16>(out, r + 16 * hf, (size_t)(row < M ? row : row0) * out.ldf + col + 16 * hf, col + 16 * hf, 16, v, z);
+            if (row < M) {
+              if (out.epi == EPI_GELU && out.zout) store16(out.zout + (size_t)row * out.ldf + col + 16 * hf, z, 16);
+              if (out.outb) store16(out.outb + (size_t)row * out.ldb + col + 16 * hf, v, 16);
             }
+            if (out.outf) {
+#pragma unroll
+              for (int q = 0; q < 16; ++q) xbuf[lane * 33 + 16 * hf + q] = v[q];
+            }
+          }
+          if (out.outf) {
+            __syncwarp();
+            float* dst = out.outf + (size_t)row0 * out.ldf + col + lane;
+            for (int i = 0; i < rows; ++i) dst[(size_t)i * out.ldf] = xbuf[i * 33 + lane];
           }
         } else if (row < M) {
           epilogue16(out, r, (size_t)row, col, min(16, N - col));
