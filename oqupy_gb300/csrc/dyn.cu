@@ -13,13 +13,14 @@
 // time-dependent system has one pair per step, and control operations
 // (system_dynamics.py:131-160) are folded into the pairs of their steps on
 // the host -- a post-measurement control of step k into P1_hk (P1 post_k),
-// a pre-measurement control of step k+1 into P2_hk (pre_{k+1} P2).  One
-// launch per step (grid: bond chunks x systems); the host replays the
-// launches of a whole sweep as a CUDA graph.  A transform_in / transform_out
-// of the process tensor is folded into P1 / P2 on the host.  The read-out
-// sum is reproducible bit for bit: a CTA adds its bond chunk's terms in a
-// fixed order, and the last CTA of a system to finish (counted after a
-// memory fence) adds the chunks' partial sums in chunk order.
+// a pre-measurement control of step k+1 into P2_hk (pre_{k+1} P2).  A
+// transform_in / transform_out of the process tensor is folded into P1 / P2 on
+// the host.  Whole sweeps run in one launch (sweep_kernel, below);
+// dyn_step_kernel does one step at a time for callers that decide the next
+// propagators from the states in between (grid: bond chunks x systems).  Both
+// are reproducible bit for bit.  dyn_step_kernel's read-out: a CTA adds its
+// bond chunk's terms in a fixed order, and the last CTA of a system to finish
+// (counted after a memory fence) adds the chunks' partial sums in chunk order.
 #include <cooperative_groups.h>
 
 #include <algorithm>
