@@ -23,6 +23,7 @@ constexpr int JACOBI_MAX_SWEEPS = 60;
 struct JacobiShared {
   double red[33];
   unsigned worst;   // largest relative off-diagonal rotated in the last allowed sweep (float bits)
+  unsigned c2max[2], t2max[2];   // largest rotated squared cosine and scaled tangent of a sweep (float bits)
   int noise_converged;
   int kept;
   int status;
@@ -68,6 +69,16 @@ __device__ __forceinline__ int jacobi_group(int pairs, int rows) { return (pairs
 // double-float, norms and gamma reduced by error-free additions) -> 1340
 // clocks; a 27 x 20 FP64 one: 16100 -> 4970.
 //
+// The last sweep is known without another one to check it.  A rotation leaves
+// 1e-6 of its pair's cosine (the FP32 angle), and changes the cosine of column u
+// with any third column w by |tau| |v| / |u| cos(v, w); over the rest of the
+// sweep a pair sees at most 2 n of these.  When the largest cosine rotated in a
+// sweep times (2e-6 + 2 n times the largest |tau| |v| / |u|) is below half the
+// rotation threshold, the next sweep would rotate nothing, and only the norms
+// are formed anew.  253 double-float instances, 40 steps: 265 -> 260 ms; 48
+// complex128 ones, 12 steps (two sweeps after the products' rotations, now
+// mostly one): 221 -> 210 ms.
+//
 // Numerical-zero floor: a column whose squared norm is below (16 sqrt(m) eps)^2
 // (double-float: (32 sqrt(m) eps)^2) times the largest squared column norm
 // holds only rounding noise of the other columns; pairs involving such a
@@ -94,8 +105,10 @@ __device__ int jacobi_sweeps_rc(typename QA<T>::E* W, int m, int n, int ld, type
   if (tid == 0) {
     sh->noise_converged = 0;
     sh->worst = 0u;
+    sh->c2max[0] = sh->t2max[0] = 0u;
   }
   int sweep;
+  bool done = false;
   for (sweep = 0; sweep < JACOBI_MAX_SWEEPS; ++sweep) {
     // squared column norms, and the largest (a lower bound of s_max^2)
     for (int j = warp; j < n; j += nw) {
@@ -106,6 +119,10 @@ __device__ int jacobi_sweeps_rc(typename QA<T>::E* W, int m, int n, int ld, type
       if (lane32 == 0) nrm2[j] = Q::fin(acc);
     }
     __syncthreads();
+    if (done) break;
+    const int par = sweep & 1;
+    if (tid == 0) sh->c2max[par ^ 1] = sh->t2max[par ^ 1] = 0u;
+    float c2m = 0.f, t2m = 0.f;
     unsigned mxb = 0u;
     for (int j = lane32; j < n; j += 32) mxb = max(mxb, __float_as_uint(Q::tof(nrm2[j])));
     const float zfloor = zf * zf * __uint_as_float(__reduce_max_sync(0xffffffffu, mxb));
@@ -158,6 +175,9 @@ __device__ int jacobi_sweeps_rc(typename QA<T>::E* W, int m, int n, int ld, type
           float q0 = rcp_est(fabsf(d) + hh * rsqrt_est(hh));
           q0 = d < 0.f ? -q0 : q0;
           const float tx = x * q0, ty = y * q0;
+          const float ratio = fmaxf(A, B) * rr;
+          c2m = fmaxf(c2m, c2);
+          t2m = fmaxf(t2m, fmaf(tx, tx, ty * ty) * (ratio * ratio));
           const typename Q::Rot rot = Q::rotation(tx, ty);
           for (int r0 = lane; r0 < (ALL ? lane + 1 : m); r0 += RC * G) {
 #pragma unroll
@@ -187,7 +207,17 @@ __device__ int jacobi_sweeps_rc(typename QA<T>::E* W, int m, int n, int ld, type
       }
       if (round < nr - 1) __syncthreads();
     }
+    {
+      const unsigned cb = __reduce_max_sync(0xffffffffu, __float_as_uint(c2m));
+      const unsigned tb = __reduce_max_sync(0xffffffffu, __float_as_uint(t2m));
+      if (lane32 == 0 && cb) {
+        atomicMax(&sh->c2max[par], cb);
+        atomicMax(&sh->t2max[par], tb);
+      }
+    }
     if (!__syncthreads_or(rotated)) break;
+    const float left = 2e-6f + 4.f * (float)np * sqrtf(__uint_as_float(sh->t2max[par]));
+    done = __uint_as_float(sh->c2max[par]) * (left * left) < 0.25f * tol2;
   }
   // at the sweep cap, rotations below 1e-10 relative are rounding noise
   if (sweep == JACOBI_MAX_SWEEPS && tid == 0 && __uint_as_float(sh->worst) < 1e-10f) sh->noise_converged = 1;

@@ -68,6 +68,20 @@ def qutrit(dkmax, epsrel):
                 rho0=np.diag([1.0, 0.0, 0.0]).astype(complex))
 
 
+def check_against_oracle(inst, steps, precision, atol, **shape):
+    from oracle import tempo_oracle as to
+    infl = inst["influences"]
+    want, _ = to.tempo_dynamics(inst["rho0"].reshape(-1), lambda dk: infl[dk] if 0 <= dk < len(infl) else None,
+                                np.eye(inst["hs_dim"]), lambda s: (inst["prop1"], inst["prop2"]),
+                                inst["dkmax"], inst["epsrel"], steps)
+    from oqupy_gb300.tempo import TempoBatch
+    b = TempoBatch([inst], precision=precision, chi_cap=128, out_cap=steps + 1, **shape)
+    b.advance(steps)
+    got = b.states(0, steps + 1)[0]
+    b.close()
+    np.testing.assert_allclose(got, want, rtol=0, atol=atol)
+
+
 @pytest.mark.parametrize("shape", [dict(), dict(block=512, smem_kb=200), dict(block=256, smem_kb=8)])
 @pytest.mark.parametrize("make, steps", [(lambda: spin_boson(0.05, 2, 1e-12), 12),   # narrow: up to 12 columns
                                          (lambda: spin_boson(0.3, 7, 1e-12), 12),
@@ -78,15 +92,12 @@ def test_complex128_split_matches_the_oracle(make, steps, shape):
     matrices in shared and in global memory.  Both sides drop at most
     epsrel s_0 = 1e-12 per split, at most 16 splits a step: 192 splits and a
     factor of 2 for the two sides give 4e-10."""
-    from oracle import tempo_oracle as to
-    from oqupy_gb300.tempo import TempoBatch
-    inst = make()
-    infl = inst["influences"]
-    want, _ = to.tempo_dynamics(inst["rho0"].reshape(-1), lambda dk: infl[dk] if 0 <= dk < len(infl) else None,
-                                np.eye(inst["hs_dim"]), lambda s: (inst["prop1"], inst["prop2"]),
-                                inst["dkmax"], inst["epsrel"], steps)
-    b = TempoBatch([inst], precision="complex128", chi_cap=128, out_cap=steps + 1, **shape)
-    b.advance(steps)
-    got = b.states(0, steps + 1)[0]
-    b.close()
-    np.testing.assert_allclose(got, want, atol=4e-10)
+    check_against_oracle(make(), steps, "complex128", 4e-10, **shape)
+
+
+@pytest.mark.parametrize("make, steps", [(lambda: spin_boson(0.3, 7, 1e-9), 12),
+                                         (lambda: spin_boson(0.3, 7, 1e-9, eps=0.0), 12),
+                                         (lambda: qutrit(4, 1e-9), 5)])
+def test_mixed_split_matches_the_oracle(make, steps):
+    """As above with epsrel 1e-9: 4e-7."""
+    check_against_oracle(make(), steps, "mixed", 4e-7)
