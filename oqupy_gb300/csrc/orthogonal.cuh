@@ -34,11 +34,16 @@
 
 namespace otb {
 
-// Splits of fewer columns go straight to the sweeps (at 8 columns the products
-// already save more than half, and smaller splits have no QR).  Double-float
-// splits always do: their products run on the pipe that the sweeps are bound by
-// (95 instances, splits of ~77 x 35: the 12 steps take 196 instead of 174 ms).
-constexpr int PRESWEEP_MIN_COLS = 8;
+// Splits of fewer columns go straight to the sweeps.  From 8 columns on the
+// products are faster (three builds of 14 steps: 18.2 ms, 19.3 ms with 10, 22.2
+// with 16), but sweeps keep a small column to its own rounding and products only
+// to that of the largest one, which decides exactly tied pairs otherwise: in a
+// mean-field model with such a pair the states' distance from the reference at
+// step 13 is 6e-11 with 10, 12, 16 or no products, 1.1e-10 with 8.
+// Double-float splits never take this way: their products run on the pipe that
+// the sweeps are bound by (95 instances, splits of ~77 x 35: the 12 steps take
+// 196 instead of 174 ms).
+constexpr int PRESWEEP_MIN_COLS = 10;
 constexpr int PRESWEEP_CORRECTIONS = 2;
 constexpr float PRESWEEP_MAX_TAN = 4e-6f;   // larger tangents are left to the sweeps
 
