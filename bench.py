@@ -934,7 +934,8 @@ def run_tempo(args, rank, world):
                     "steps_per_launch": ls,
                     "warmup": f"{args.warmup} bench steps on a separate batch (seed {BATCH_SEED + 7919})",
                     "launch": ({"autotuned_per_bond_bucket": tuner.table()} if tuner is not None
-                               else {"block": args.block or 256, "smem_kb": args.smem_kb or 56})},
+                               else {"block": args.block or "library default",
+                                     "smem_kb": args.smem_kb or "library default"})},
             "roofline": roofline, "cpu_baseline": cpu,
             "e2e": {"value": len(insts) * frac_traj / e2e_all, "unit": "trajectories/s",
                     "h2d_bytes_per_step": int(h2d // max(1, args.steps)),

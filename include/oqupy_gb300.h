@@ -65,14 +65,18 @@ typedef struct {
   int32_t precision;   /* OTB_PRECISION_* */
   int32_t chi_cap;     /* bond-dimension capacity of every site, chi_cap * D <= 1152 */
   int32_t out_cap;     /* states kept per instance (ring), >= 2 */
-  int32_t grid;        /* CTAs per launch, 0 = 2 per SM for blocks up
-                          to 256 threads, 1 per SM above */
-  int32_t block;       /* threads per CTA (64..512, multiple of 32), 0 =
-                          512 for batches of up to one instance per SM,
-                          256 for larger ones */
+  int32_t grid;        /* CTAs per launch, 0 = as many as are resident: one
+                          per SM for blocks above 256 threads and batches of
+                          up to one instance per SM, else up to three by the
+                          block's registers and smem_kb */
+  int32_t block;       /* threads per CTA (64..512, multiple of 32), 0 = 512;
+                          for more instances than SMs 256 with memories of up
+                          to 7 two-level steps, two CTAs per SM up to 5 */
   int32_t smem_kb;     /* dynamic shared memory per CTA for working matrices
-                          (KiB, <= 200), 0 = 200 for one CTA per SM, 100
-                          for two */
+                          (KiB, <= 200), 0 = an equal share of the SM's for
+                          its CTAs (200, 95 or 57 for one, two or three; 100
+                          for one of up to 256 threads in batches of more
+                          instances than SMs) */
   double qr_cut;       /* relative cut of the rank-revealing QR that precedes
                           the Jacobi SVD of every split of >= 8 columns: the
                           factorisation stops once the remaining block's
@@ -123,8 +127,9 @@ otb_status otb_tempo_advance(otb_tempo* h, int32_t nsteps, void* stream);
 /* Launch shape of the next advances (no reference counterpart: the
  * reference has no launch): block threads per CTA (64..512), smem_kb
  * dynamic shared memory per CTA (<= 200), grid CTAs (capped at the grid the
- * handle's workspace was allocated for); 0 = otb_tempo_config's defaults.  Used by the per-bond-bucket
- * launch-shape tuner. */
+ * handle's workspace was allocated for); 0 = otb_tempo_config's defaults (a
+ * default grid wider than that workspace waits for the device and allocates
+ * more).  Used by the per-bond-bucket launch-shape tuner. */
 otb_status otb_tempo_set_launch(otb_tempo* h, int32_t block, int32_t smem_kb, int32_t grid);
 /* States of steps [first_step, first_step+count) of one instance, each D
  * complex; steps must still be held by the output ring (step 0 = rho0). */

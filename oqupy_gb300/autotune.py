@@ -25,12 +25,13 @@ from typing import Dict, List, Optional, Sequence, Tuple
 
 from .tempo import TempoBatch
 
-# (threads per CTA, CTAs per SM, dynamic smem KiB)
+# (threads per CTA, CTAs per SM, dynamic smem KiB); all of a shape's CTAs fit:
+# 128 registers a thread, 18 KiB of static and 1 KiB of reserved shared memory a CTA
 CANDIDATES: List[Tuple[int, int, int]] = [
-    (256, 3, 56), (256, 2, 88), (256, 1, 200), (192, 3, 56), (128, 4, 48)]
+    (512, 1, 200), (256, 2, 95), (256, 2, 56), (256, 1, 200), (160, 3, 56), (128, 4, 37)]
 
 
-# (threads per CTA, dynamic smem KiB): narrow CTAs, three per SM / one wide CTA per SM
+# (threads per CTA, dynamic smem KiB): one wide CTA per SM / two narrow ones
 BUCKET_CANDIDATES: List[Tuple[int, int]] = [(512, 200), (256, 56)]
 
 

@@ -20,6 +20,8 @@ struct otb_tempo {
   int out_cap = 0;
   int grid = 0;
   int grid_alloc = 0;   // CTAs the per-CTA workspace is allocated for
+  bool grid_fixed = false;   // the caller gave the grid at creation
+  double memory = 0.0;       // longest memory of the instances, in two-level steps
   int sms = 0;
   int block = 256;
   int smem_bytes = 0;
@@ -122,18 +124,48 @@ otb_status upload_inst(otb_tempo* h) {
   return OTB_OK;
 }
 
-// Launch shape where the caller gives none (block / smem_bytes / grid 0).
-// A kernel's registers allow 512 threads per SM.  A batch of at most one
-// instance per SM runs one 512-thread CTA with the largest shared-memory share
-// on each; more instances share an SM two by two (256 threads, 100 KiB): 253
-// spin-boson instances, 40 steps, 242 ms that way and 266 ms one by one; 95
-// converged ones (splits of ~75 x 34 columns), 12 steps, 212 and 176 ms.
-// CTAs of more than 256 threads (128 registers each) fill an SM alone.
+// Launch shape where the caller gives none (block / smem_bytes / grid 0).  A
+// kernel's registers allow 512 threads per SM.
+//  * One 512-thread CTA with the largest shared-memory share has an SM for
+//    itself, in batches of up to one instance per SM and in larger ones with a
+//    memory of more than NARROW_MEMORY steps: a launch ends with its longest
+//    instance, which two CTAs on an SM slow down.  Milliseconds a step of 304
+//    spin-boson instances (epsrel 1e-6, steps 12-24 and 24-36 in double-float |
+//    complex128), one CTA of 512 threads, one of 256, two of 256 with 95 KiB each:
+//    memory of 8 steps 5.6 6.2 | 10.2 11.5, 5.6 6.2 | 10.7 12.2, 8.2 8.4 | 12.6
+//    15.6; of 24 steps 20.8 82 | 34 160, 21.6 102 | 37 174, 29.3 132 | 44 206.
+//  * One of 256 threads with 100 KiB (what is left of the SM's memory is the L1
+//    cache) up to that memory: memory of 6 steps 2.83 3.04 | 4.90 5.31, 2.69 2.89 |
+//    5.01 5.50, 3.26 3.62 | 4.92 5.74; of 7 steps 4.11 | 7.48 (steps 12-24), 4.06 |
+//    7.80 (4.17 | 7.87 with 200 KiB), 5.53 | 8.89.
+//  * Two of 256 threads for a memory of SHORT_MEMORY steps at most, whose splits
+//    leave most of a wide CTA idle: memory of 5 steps 1.64 1.72 | 2.75 3.05, 1.53
+//    1.63 | 2.70 3.07, 1.54 1.65 | 2.28 2.49 (1216 instances 6.25 6.40 | 10.5 10.7,
+//    5.84 6.12 | 10.3 10.5, 4.90 4.75 | 7.1 7.3); of 4 steps 0.95 0.95 | 1.52 1.52,
+//    0.87 0.86 | 1.44 1.43, 0.70 0.71 | 0.99 1.01.
+//  The memory counts in two-level steps (a step's bond grows by up to D = 4):
+//  304 qutrits, epsrel 1e-8, memory of 3 steps (4.8): 8.7 | 16.3, 10.0 | 17.2, 8.6 |
+//  15.8; epsrel 1e-6, of 5 steps (7.9): 34 | 96, 41 | 104, 43 | 106.
+//  * A block of up to 256 threads that the caller chooses gets as many CTAs per
+//    SM as its registers allow, up to three, with an equal share of the memory.
+// Everything follows from what really fits, so that the grid's CTAs are all
+// resident.
+constexpr double SHORT_MEMORY = 5.0, NARROW_MEMORY = 7.0;
+
 void launch_shape(otb_tempo* h, int block, int smem_bytes, int grid) {
+  const int prec = h->precision;
   const bool alone = h->n <= h->sms;
-  h->block = block > 0 ? block : (alone ? 512 : 256);
-  const int per_sm = h->block > 256 ? 1 : 2;
-  h->smem_bytes = smem_bytes > 0 ? smem_bytes : (per_sm == 1 || alone ? 200 : 100) * 1024;
+  h->block = block > 0 ? block : alone || h->memory > NARROW_MEMORY ? 512 : 256;
+  const bool one = alone || h->block > 256 || (block <= 0 && h->memory > SHORT_MEMORY);
+  int per_sm = one ? 1 : std::min(3, tempo_residency(prec, h->block, 1024));
+  per_sm = std::max(1, per_sm);
+  h->smem_bytes = smem_bytes;
+  if (smem_bytes <= 0) {
+    const int share = tempo_shared_share(prec, per_sm);
+    h->smem_bytes = share <= 0 ? 56 * 1024 : alone || h->block > 256 ? share : std::min(share, 100 * 1024);
+  } else if (!one) {
+    per_sm = std::max(1, std::min(3, tempo_residency(prec, h->block, smem_bytes)));
+  }
   h->grid = grid > 0 ? grid : std::max(1, std::min(h->n, per_sm * h->sms));
 }
 
@@ -292,10 +324,13 @@ extern "C" otb_status otb_tempo_create(const otb_tempo_config* cfg, int32_t n,
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   h->sms = std::max(sms, 1);
+  for (const InstDev& I : h->inst)
+    h->memory = std::max(h->memory, I.dkmax * (std::log((double)I.D) / std::log(4.0)));
   launch_shape(h.get(), cfg->block, cfg->smem_kb * 1024, cfg->grid);
-  // workspace for the widest default grid, so otb_tempo_set_launch can
-  // switch shapes later (an explicit grid fixes it)
-  h->grid_alloc = cfg->grid > 0 ? cfg->grid : std::max(h->grid, std::min(n, 2 * h->sms));
+  // workspace for two CTAs per SM, so that otb_tempo_set_launch can mostly
+  // switch shapes without another allocation (an explicit grid fixes it)
+  h->grid_fixed = cfg->grid > 0;
+  h->grid_alloc = h->grid_fixed ? cfg->grid : std::max(h->grid, std::min(n, 2 * h->sms));
   h->wcap = (long long)(h->cap * h->Dmax) * (h->cap * h->Dmax);
   h->work_stride = tempo_work_bytes(h->wcap, h->precision == OTB_PRECISION_MIXED);
   if (!h->d_work.alloc((size_t)h->grid_alloc * h->work_stride)) return OTB_ERR_OOM;
@@ -356,6 +391,14 @@ extern "C" otb_status otb_tempo_set_launch(otb_tempo* h, int32_t block, int32_t 
   if (smem_kb < 0 || smem_kb > 200) return set_error(OTB_ERR_INVALID_ARG, "smem_kb must be in [0, 200]");
   if (grid < 0) return set_error(OTB_ERR_INVALID_ARG, "grid must be >= 0");
   launch_shape(h, block, smem_kb * 1024, grid);
+  if (grid == 0 && !h->grid_fixed && h->grid > h->grid_alloc) {
+    // a narrow block's CTAs: more workspace, once no launch uses the present one
+    DevBuf more;
+    if (more.alloc((size_t)h->grid * h->work_stride) && check_cuda(cudaDeviceSynchronize(), "launch shape")) {
+      h->d_work = std::move(more);
+      h->grid_alloc = h->grid;
+    }
+  }
   h->grid = std::max(1, std::min(h->grid, h->grid_alloc));
   return OTB_OK;
 }

@@ -76,6 +76,11 @@ cudaError_t launch_tempo_order(InstState* state, int* order, int n, cudaStream_t
 cudaError_t launch_tempo(const TempoLaunch& L, int precision, int grid, int block,
                          int smem_bytes, cudaStream_t stream);
 int tempo_smem_bytes(int precision);
+// CTAs of the batched kernel that one SM holds at a block size and a dynamic
+// shared-memory size (0 if none fits), and the largest dynamic size (bytes, in
+// whole KiB) with which `ctas` CTAs share an SM.
+int tempo_residency(int precision, int block, int smem_bytes);
+int tempo_shared_share(int precision, int ctas);
 
 // ---------------------------------------------------------------- PT-TEMPO
 

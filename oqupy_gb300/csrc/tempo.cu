@@ -32,6 +32,7 @@
 // no reshuffle.
 #include <math.h>
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 
@@ -44,6 +45,7 @@
 namespace otb {
 
 constexpr int TEMPO_THREADS = 512;   // largest CTA of the batched kernel (launch bound)
+constexpr int TEMPO_MAX_SMEM = 200 * 1024;   // largest dynamic shared memory of a launch
 constexpr int STATIC_THREADS = 256;  // CTA of the allocation-free single-instance kernel
 
 struct Bufs {
@@ -474,12 +476,45 @@ __global__ void __launch_bounds__(TEMPO_THREADS, 1) tempo_kernel(TempoLaunch L) 
   }
 }
 
+// Dynamic shared memory for the working matrices of the allocation-free entry
+// point and of launches that give none.
 int tempo_smem_bytes(int precision) {
-  // dynamic shared memory for the working matrices when the caller gives
-  // none (the C ABI passes its own default, 56 KiB: three CTAs per SM with
-  // the static SharedStep block)
   (void)precision;
   return 88 * 1024;
+}
+
+static const void* tempo_entry(int precision) {
+  return precision == 0 ? (const void*)tempo_kernel<false> : (const void*)tempo_kernel<true>;
+}
+
+// The largest dynamic share, whatever a launch takes: the limit belongs to the
+// function, and threads with other sizes may be launching it at the same time.
+static cudaError_t allow_shared(int precision) {
+  return cudaFuncSetAttribute(tempo_entry(precision), cudaFuncAttributeMaxDynamicSharedMemorySize, TEMPO_MAX_SMEM);
+}
+
+int tempo_residency(int precision, int block, int smem_bytes) {
+  int ctas = 0;
+  if (allow_shared(precision) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, tempo_entry(precision), block, smem_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return ctas;
+}
+
+int tempo_shared_share(int precision, int ctas) {
+  int dev = 0, sm = 0, reserved = 0;
+  cudaFuncAttributes at;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
+      cudaFuncGetAttributes(&at, tempo_entry(precision)) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  const int share = sm / ctas - reserved - (int)at.sharedSizeBytes;
+  return std::max(0, std::min(share, TEMPO_MAX_SMEM)) / 1024 * 1024;
 }
 
 // Work-queue order for the next launch: instances by the device time they
@@ -543,17 +578,12 @@ cudaError_t launch_tempo(const TempoLaunch& L, int precision, int grid, int bloc
   const int smem = smem_bytes > 0 ? smem_bytes : tempo_smem_bytes(precision);
   TempoLaunch l2 = L;
   l2.smem_bytes = smem;
-  if (precision == 0) {
-    cudaError_t e = cudaFuncSetAttribute(tempo_kernel<false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
+  const cudaError_t e = allow_shared(precision);
+  if (e != cudaSuccess) return e;
+  if (precision == 0)
     tempo_kernel<false><<<grid, block, smem, stream>>>(l2);
-  } else {
-    cudaError_t e = cudaFuncSetAttribute(tempo_kernel<true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
+  else
     tempo_kernel<true><<<grid, block, smem, stream>>>(l2);
-  }
   return cudaGetLastError();
 }
 
