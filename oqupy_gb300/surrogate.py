@@ -293,7 +293,9 @@ class Surrogate:
             oe = torch.tensor(p[:, 3:5], dtype=torch.float32, device=self.net.dev)
             nat.check(nat.lib().otb_mlp_bloch_free_add(Y.data_ptr(), oe.data_ptr(), len(p), self.nsteps,
                                                        float(self.dt), None))
-        return Y.cpu().numpy().reshape(len(p), 3, self.nsteps)
+        out = Y.cpu().numpy().reshape(len(p), 3, self.nsteps)
+        self.net.check_errors()      # a product that gave up leaves rows unwritten
+        return out
 
     def _bin(self, params):
         p = np.asarray(params)
