@@ -328,6 +328,7 @@ SweepLaunch sweep_launch(otb_pt* h, int32_t inst, int nh, int num_steps, const s
   L.cap = I.cap;
   L.max_bond = 1;
   for (int k = 0; k < num_steps; ++k) L.max_bond = std::max(L.max_bond, std::max(dims[k].x, dims[k].y));
+  L.wide = sweep_is_wide(I.D, num_steps, dims.data());
   L.sites = (const double*)h->d_sites.p + 2 * I.site_base;
   L.slot_elems = (long long)I.cap * I.D * I.cap;
   L.dims = (const int2*)h->d_dims.p + I.dims_base;

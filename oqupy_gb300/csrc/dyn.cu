@@ -141,8 +141,8 @@ __global__ void dyn_init_kernel(DynLaunch L, const double* rho0) {
 // sum over l is split over G lanes where a CTA has fewer columns than threads.
 // One launch replaces a graph of N kernel nodes that had to be captured and
 // instantiated per call. Whole calls, 60 steps, bond 13, before and now: 8
-// systems 760 and 290 us, 1024 systems 1750 and 930 us, gradient of 24 driven
-// systems 1610 and 560 us.
+// systems 760 and 240 us, 1024 systems 1750 and 920 us, gradient of 24 driven
+// systems 1610 and 500 us.
 constexpr int SWEEP_THREADS = 256;
 
 __global__ void __launch_bounds__(SWEEP_THREADS) sweep_prepare_kernel(SweepLaunch L) {
@@ -201,13 +201,53 @@ __device__ __forceinline__ void lane_sum(zc& v, int G) {
   }
 }
 
-// sum_a M[a ms] x[a] over D terms, the terms lane, lane + lg, ...; summed over
-// the lg lanes (1 or 4).
-__device__ __forceinline__ zc row_product(const zc* M, int ms, const zc* x, int D, int lane, int lg, bool act) {
+// A column's sum over `len` terms is split into V partial sums (terms v, v + V,
+// ...; added by halves, as lane_sum adds lanes), whatever the number of systems
+// and of CTAs that share a step, so that a system's states are the same bits in
+// any batch.  V is the number of lanes a column gets where one CTA holds all
+// `outs` columns of the step, and at least 4 for steps wide enough to be split
+// over a cluster, whose CTAs have lanes left over (bonds from 20 on with D = 4);
+// a CTA with too many columns for V lanes each adds the rest one after the
+// other (WIDE kernels; without such a step every column has its V lanes).  The
+// parts cost a wide sweep that has a CTA or more per SM up to 5 % (bond 85: 77
+// systems 2115 -> 2225 us, 1024 systems 12.3 -> 12.5 ms; with G after the CTA's own
+// columns, but other bits in every batch).
+__host__ __device__ __forceinline__ int sum_parts(int len, int outs) {
+  int V = 1;
+  while (V < 8 && 4 * V <= len && (2 * V * outs <= SWEEP_THREADS || (V < 4 && len * outs > 1500))) V <<= 1;
+  return V;
+}
+__host__ __device__ __forceinline__ int part_lanes(int V, int outs) {
+  int G = 1;
+  while (G < V && 2 * G * outs <= SWEEP_THREADS) G <<= 1;
+  return G;
+}
+// The j-th part of V / G that lane g adds up, in the order in which halves are
+// added: 0 2 1 3 of four.
+__device__ __forceinline__ int part_index(int j, int g, int G, int parts) {
+  return g + G * (parts == 4 ? ((j & 1) << 1) | (j >> 1) : j);
+}
+__device__ __forceinline__ void add_part(int j, const zc& part, zc& sum, zc& hold) {
+  if (j == 0)
+    sum = part;
+  else if (j == 1)
+    sum = sum + part;
+  else if (j == 2)
+    hold = part;
+  else
+    sum = sum + (hold + part);
+}
+
+// CTAs per SM that the register allocation aims at: one CTA's chain of phases is
+// what counts (168 registers for four systems), but with one system's partial
+// sums after each other the compiler's longer unrolling costs more than it hides
+// (77 systems, bond 85: 2350 us a sweep without a bound, 2225 with).
+__host__ __device__ constexpr int sweep_ctas(bool lean, int dt) { return !lean ? 1 : dt == 4 ? 3 : 2; }
+
+// sum_a M[a ms] x[a] over D terms.
+__device__ __forceinline__ zc row_product(const zc* M, int ms, const zc* x, int D) {
   zc acc = mk<double>(0, 0);
-  if (act)
-    for (int a = lane; a < D; a += lg) cfma(acc, M[a * ms], x[a]);
-  lane_sum(acc, lg);
+  for (int a = 0; a < D; ++a) cfma(acc, M[a * ms], x[a]);
   return acc;
 }
 
@@ -226,8 +266,8 @@ __device__ __forceinline__ void stage_columns(const SweepLaunch& L, int k, int2 
 // S systems per CTA; RECORD keeps v_k (gradient sweeps); DT as below.  With L.stage the next
 // step's columns (and propagators) are copied to shared memory while a step
 // computes: a step waits for no global load.
-template <int S, bool RECORD, int DT>
-__global__ void __launch_bounds__(SWEEP_THREADS) sweep_kernel(SweepLaunch L) {
+template <int S, bool RECORD, int DT, bool WIDE>
+__global__ void __launch_bounds__(SWEEP_THREADS, sweep_ctas(WIDE && S == 1, DT)) sweep_kernel(SweepLaunch L) {
   extern __shared__ __align__(16) unsigned char dsm[];
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
@@ -288,70 +328,76 @@ __global__ void __launch_bounds__(SWEEP_THREADS) sweep_kernel(SweepLaunch L) {
       if (k + 2 < N) dnn = L.dims[k + 2];
     }
     const int outs = nc * D;
-    // G lanes share a column's sum over l where threads are left over
-    int G = 1;
-    while (G < 8 && 2 * G * outs <= nt && 4 * G <= l) G <<= 1;
+    const int V = sum_parts(l, (r + 1) * D), G = WIDE ? part_lanes(V, outs) : V, parts = V / G;
     const int g = tid & (G - 1);
     for (int o0 = 0; o0 < outs; o0 += nt / G) {
       const int o = o0 + tid / G;
       const bool act = o < outs;
       const int cc = act ? o / D : 0, a = act ? o - cc * D : 0;
-      zc acc[S];
+      zc sum[S];
 #pragma unroll
-      for (int s = 0; s < S; ++s) acc[s] = mk<double>(0, 0);
+      for (int s = 0; s < S; ++s) sum[s] = mk<double>(0, 0);
       if (act) {
         const bool last = c0 + cc == r;
         const zc* col = L.stage ? as + a * nc + cc
                         : last  ? (const zc*)L.bcol + (long long)k * L.cap * D + a
                                 : (const zc*)L.sites + (long long)k * L.slot_elems + (size_t)a * r + c0 + cc;
         const size_t step = (size_t)D * (L.stage ? nc : last ? 1 : r);
-        for (int l0 = g; l0 < l; l0 += 4 * G) {
-          zc x[4];
+        zc hold[WIDE ? S : 1];
+#pragma unroll 1
+        for (int j = 0; j < (WIDE ? parts : 1); ++j) {
+          zc acc[S];
 #pragma unroll
-          for (int t = 0; t < 4; ++t)
-            if (l0 + t * G < l) x[t] = col[(l0 + t * G) * step];
+          for (int s = 0; s < S; ++s) acc[s] = mk<double>(0, 0);
+          for (int l0 = WIDE ? part_index(j, g, G, parts) : g; l0 < l; l0 += 4 * V) {
+            zc x[4];
 #pragma unroll
-          for (int t = 0; t < 4; ++t)
-            if (l0 + t * G < l) {
+            for (int t = 0; t < 4; ++t)
+              if (l0 + t * V < l) x[t] = col[(l0 + t * V) * step];
 #pragma unroll
-              for (int s = 0; s < S; ++s) cfma(acc[s], u[(size_t)s * ustride + (l0 + t * G) * D + a], x[t]);
-            }
+            for (int t = 0; t < 4; ++t)
+              if (l0 + t * V < l) {
+#pragma unroll
+                for (int s = 0; s < S; ++s) cfma(acc[s], u[(size_t)s * ustride + (l0 + t * V) * D + a], x[t]);
+              }
+          }
+#pragma unroll
+          for (int s = 0; s < S; ++s)
+            if (WIDE)
+              add_part(j, acc[s], sum[s], hold[s]);
+            else
+              sum[s] = acc[s];
         }
       }
-      for (int s = 0; s < S; ++s) lane_sum(acc[s], G);
+#pragma unroll
+      for (int s = 0; s < S; ++s) lane_sum(sum[s], G);
       if (act && g == 0)
 #pragma unroll
-        for (int s = 0; s < S; ++s) w[(size_t)s * wstride + cc * D + a] = acc[s];
+        for (int s = 0; s < S; ++s) w[(size_t)s * wstride + cc * D + a] = sum[s];
     }
     __syncthreads();
     // the next states (to every CTA of the cluster) and the read-out
-    const int n2 = ns * outs;
-    const int lg = (D == 4 && 4 * n2 <= nt) ? 4 : 1, lane = tid & (lg - 1);
-    for (int i0 = 0; i0 < n2; i0 += nt / lg) {
-      const int i = i0 + tid / lg;
-      const bool act = i < n2;
-      const int s = act && S > 1 ? i / outs : 0, o = act ? i - s * outs : 0;
+    for (int i = tid; i < (RECORD ? 2 : ns) * outs; i += nt) {
+      const int s = RECORD || S > 1 ? i / outs : 0, o = i - s * outs;   // RECORD: s = 1 for v_{k+1}
       const int cc = o / D, a = o - cc * D;
-      const bool last = c0 + cc == r;
-      const zc* M = q + (size_t)s * 2 * DD + a * D;
-      const zc* x = w + (size_t)s * wstride + cc * D;
-      const zc y = row_product(last ? M + DD : M, 1, x, D, lane, lg, act);
-      zc vr = y;
-      if (RECORD) vr = row_product(M + DD, 1, x, D, lane, lg, act);   // v_{k+1} = d P2_k w
-      if (act) {
-        if (last) {
-          if (lane == 0) ((zc*)L.out)[((long long)(k + 1) * L.nh + h0 + s) * D + a] = y;
-        } else {
-          zc* dst = un + (size_t)s * ustride + (size_t)(c0 + cc) * D + a;
-          if (C == 1) {
-            if (lane == 0) *dst = y;
-          } else {
-            for (int t = lane; t < C; t += lg) *cluster.map_shared_rank(dst, t) = y;
-          }
-          if (RECORD && lane == 0 && k + 1 < N)
-            ((zc*)L.fwd_hist)[(((long long)(h0 + s) * N + k + 1) * L.cap + c0 + cc) * D + a] = vr;
-        }
+      const bool last = c0 + cc == r, keep = RECORD && s == 1;
+      if (keep && (last || k + 1 == N)) continue;
+      const zc* M = q + (RECORD ? 0 : (size_t)s * 2 * DD) + a * D;
+      const zc* x = w + (RECORD ? 0 : (size_t)s * wstride) + cc * D;
+      const zc y = row_product(last || keep ? M + DD : M, 1, x, D);
+      if (last) {
+        ((zc*)L.out)[((long long)(k + 1) * L.nh + h0 + s) * D + a] = y;
+        continue;
       }
+      if (keep) {   // v_{k+1} = d P2_k w
+        ((zc*)L.fwd_hist)[(((long long)h0 * N + k + 1) * L.cap + c0 + cc) * D + a] = y;
+        continue;
+      }
+      zc* dst = un + (size_t)s * ustride + (size_t)(c0 + cc) * D + a;
+      if (C == 1)
+        *dst = y;
+      else
+        for (int t = 0; t < C; ++t) *cluster.map_shared_rank(dst, t) = y;
     }
     copies_done();
     if (C == 1)
@@ -373,8 +419,8 @@ __global__ void __launch_bounds__(SWEEP_THREADS) sweep_kernel(SweepLaunch L) {
 // transforms folded in), so Y_k equals the reference's backward node before
 // the pre-measurement control of step k.  As sweep_kernel, one system per
 // cluster; the next z is (Q_{k-1})^T w.
-template <int DT>
-__global__ void __launch_bounds__(SWEEP_THREADS) sweep_back_kernel(SweepLaunch L, const double* target) {
+template <int DT, bool WIDE>
+__global__ void __launch_bounds__(SWEEP_THREADS, sweep_ctas(WIDE, DT)) sweep_back_kernel(SweepLaunch L, const double* target) {
   extern __shared__ __align__(16) unsigned char dsm[];
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
@@ -439,47 +485,52 @@ __global__ void __launch_bounds__(SWEEP_THREADS) sweep_back_kernel(SweepLaunch L
     const zc* base = L.stage ? ab + (size_t)(k & 1) * L.stage
                              : (const zc*)L.sites + (long long)k * L.slot_elems + (size_t)l0 * D * r;
     const int outs = nl * D;
-    int G = 1;
-    while (G < 8 && 2 * G * outs <= nt && 4 * G <= r) G <<= 1;
+    const int V = sum_parts(r, dm.x * D), G = WIDE ? part_lanes(V, outs) : V, parts = V / G;
     const int g = tid & (G - 1);
     for (int o0 = 0; o0 < outs; o0 += nt / G) {
       const int o = o0 + tid / G;
       const bool act = o < outs;
-      zc acc = mk<double>(0, 0);
+      zc sum = mk<double>(0, 0);
       if (act) {
         const int b = o % D;
         const zc* row = base + (size_t)o * r;
-        for (int r0 = g; r0 < r; r0 += 4 * G) {
-          zc x[4];
+        zc hold;
+#pragma unroll 1
+        for (int j = 0; j < (WIDE ? parts : 1); ++j) {
+          zc acc = mk<double>(0, 0);
+          for (int r0 = WIDE ? part_index(j, g, G, parts) : g; r0 < r; r0 += 4 * V) {
+            zc x[4];
 #pragma unroll
-          for (int t = 0; t < 4; ++t)
-            if (r0 + t * G < r) x[t] = row[r0 + t * G];
+            for (int t = 0; t < 4; ++t)
+              if (r0 + t * V < r) x[t] = row[r0 + t * V];
 #pragma unroll
-          for (int t = 0; t < 4; ++t)
-            if (r0 + t * G < r) cfma(acc, x[t], z[(r0 + t * G) * D + b]);
+            for (int t = 0; t < 4; ++t)
+              if (r0 + t * V < r) cfma(acc, x[t], z[(r0 + t * V) * D + b]);
+          }
+          if (WIDE)
+            add_part(j, acc, sum, hold);
+          else
+            sum = acc;
         }
       }
-      lane_sum(acc, G);
-      if (act && g == 0) w[o] = acc;
+      lane_sum(sum, G);
+      if (act && g == 0) w[o] = sum;
     }
     __syncthreads();
-    const int lg = (D == 4 && 8 * outs <= nt) ? 4 : 1, lane = tid & (lg - 1);
-    for (int o0 = 0; o0 < 2 * outs; o0 += nt / lg) {
-      const int o = o0 + tid / lg;
-      const bool act = o < 2 * outs, next = o >= outs;
-      const int i = act ? (next ? o - outs : o) : 0;
+    for (int o = tid; o < 2 * outs; o += nt) {
+      const bool next = o >= outs;
+      const int i = next ? o - outs : o;
       const int li = i / D, a = i - li * D;
-      const zc acc = row_product(q + (next ? DD : 0) + a, D, w + li * D, D, lane, lg, act);
-      if (act && next) {
-        zc* dst = zn + (size_t)(l0 + li) * D + a;
-        if (C == 1) {
-          if (lane == 0) *dst = acc;
-        } else {
-          for (int t = lane; t < C; t += lg) *cluster.map_shared_rank(dst, t) = acc;
-        }
-      } else if (act && lane == 0) {
+      const zc acc = row_product(q + (next ? DD : 0) + a, D, w + li * D, D);
+      if (!next) {
         Y[((long long)k * L.cap + l0 + li) * D + a] = acc;
+        continue;
       }
+      zc* dst = zn + (size_t)(l0 + li) * D + a;
+      if (C == 1)
+        *dst = acc;
+      else
+        for (int t = 0; t < C; ++t) *cluster.map_shared_rank(dst, t) = acc;
     }
     copies_done();
     if (C == 1)
@@ -596,32 +647,45 @@ cudaError_t launch_sweep_prepare(const SweepLaunch& L, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
+// Has any step more columns than lanes for its partial sums (WIDE)?
+bool sweep_is_wide(int D, int num_steps, const int2* dims) {
+  for (int k = 0; k < num_steps; ++k) {
+    const int fwd = (dims[k].y + 1) * D, back = dims[k].x * D;
+    const int vf = sum_parts(dims[k].x, fwd), vb = sum_parts(dims[k].y, back);
+    if (part_lanes(vf, fwd) < vf || part_lanes(vb, back) < vb) return true;
+  }
+  return false;
+}
+
+template <int DT, bool WIDE>
+static cudaError_t launch_sweep_shape(const SweepLaunch& L, const SweepShape& sh, cudaStream_t stream) {
+  const int ctas = (L.nh + sh.S - 1) / sh.S * sh.C;
+  if (L.fwd_hist) return launch_clusters(sweep_kernel<1, true, DT, WIDE>, ctas, sh.C, sh.smem, stream, L);
+  switch (sh.S) {
+    case 1: return launch_clusters(sweep_kernel<1, false, DT, WIDE>, ctas, sh.C, sh.smem, stream, L);
+    case 2: return launch_clusters(sweep_kernel<2, false, DT, WIDE>, ctas, sh.C, sh.smem, stream, L);
+    case 4: return launch_clusters(sweep_kernel<4, false, DT, WIDE>, ctas, sh.C, sh.smem, stream, L);
+  }
+  if constexpr (DT == 4) {
+    switch (sh.S) {
+      case 3: return launch_clusters(sweep_kernel<3, false, 4, WIDE>, ctas, sh.C, sh.smem, stream, L);
+      case 5: return launch_clusters(sweep_kernel<5, false, 4, WIDE>, ctas, sh.C, sh.smem, stream, L);
+      case 6: return launch_clusters(sweep_kernel<6, false, 4, WIDE>, ctas, sh.C, sh.smem, stream, L);
+      case 7: return launch_clusters(sweep_kernel<7, false, 4, WIDE>, ctas, sh.C, sh.smem, stream, L);
+      case 8: return launch_clusters(sweep_kernel<8, false, 4, WIDE>, ctas, sh.C, sh.smem, stream, L);
+    }
+  }
+  return cudaErrorInvalidValue;
+}
+
 cudaError_t launch_sweep(const SweepLaunch& L0, cudaStream_t stream) {
   SweepLaunch L = L0;
   SweepShape sh = sweep_shape(L, L.fwd_hist ? 1 : L.D == 4 ? 8 : 4);
   if (L.D != 4 && sh.S == 3) sh = sweep_shape(L, 2);   // built for 1, 2 and 4 systems
   L.max_cols = sh.max_cols;
   L.stage = (long long)sh.stage;
-  const int ctas = (L.nh + sh.S - 1) / sh.S * sh.C;
-  if (L.D == 4) {
-    if (L.fwd_hist) return launch_clusters(sweep_kernel<1, true, 4>, ctas, sh.C, sh.smem, stream, L);
-    switch (sh.S) {
-      case 1: return launch_clusters(sweep_kernel<1, false, 4>, ctas, sh.C, sh.smem, stream, L);
-      case 2: return launch_clusters(sweep_kernel<2, false, 4>, ctas, sh.C, sh.smem, stream, L);
-      case 3: return launch_clusters(sweep_kernel<3, false, 4>, ctas, sh.C, sh.smem, stream, L);
-      case 4: return launch_clusters(sweep_kernel<4, false, 4>, ctas, sh.C, sh.smem, stream, L);
-      case 5: return launch_clusters(sweep_kernel<5, false, 4>, ctas, sh.C, sh.smem, stream, L);
-      case 6: return launch_clusters(sweep_kernel<6, false, 4>, ctas, sh.C, sh.smem, stream, L);
-      case 7: return launch_clusters(sweep_kernel<7, false, 4>, ctas, sh.C, sh.smem, stream, L);
-      default: return launch_clusters(sweep_kernel<8, false, 4>, ctas, sh.C, sh.smem, stream, L);
-    }
-  }
-  if (L.fwd_hist) return launch_clusters(sweep_kernel<1, true, 0>, ctas, sh.C, sh.smem, stream, L);
-  switch (sh.S) {
-    case 1: return launch_clusters(sweep_kernel<1, false, 0>, ctas, sh.C, sh.smem, stream, L);
-    case 2: return launch_clusters(sweep_kernel<2, false, 0>, ctas, sh.C, sh.smem, stream, L);
-    default: return launch_clusters(sweep_kernel<4, false, 0>, ctas, sh.C, sh.smem, stream, L);
-  }
+  if (L.D == 4) return L.wide ? launch_sweep_shape<4, true>(L, sh, stream) : launch_sweep_shape<4, false>(L, sh, stream);
+  return L.wide ? launch_sweep_shape<0, true>(L, sh, stream) : launch_sweep_shape<0, false>(L, sh, stream);
 }
 
 cudaError_t launch_sweep_back(const SweepLaunch& L0, const double* target, cudaStream_t stream) {
@@ -629,8 +693,12 @@ cudaError_t launch_sweep_back(const SweepLaunch& L0, const double* target, cudaS
   const SweepShape sh = sweep_shape(L, 1);
   L.max_cols = sh.max_cols;
   L.stage = (long long)sh.stage;
-  return L.D == 4 ? launch_clusters(sweep_back_kernel<4>, L.nh * sh.C, sh.C, sh.smem, stream, L, target)
-                  : launch_clusters(sweep_back_kernel<0>, L.nh * sh.C, sh.C, sh.smem, stream, L, target);
+  const int ctas = L.nh * sh.C;
+  if (L.D == 4)
+    return L.wide ? launch_clusters(sweep_back_kernel<4, true>, ctas, sh.C, sh.smem, stream, L, target)
+                  : launch_clusters(sweep_back_kernel<4, false>, ctas, sh.C, sh.smem, stream, L, target);
+  return L.wide ? launch_clusters(sweep_back_kernel<0, true>, ctas, sh.C, sh.smem, stream, L, target)
+                : launch_clusters(sweep_back_kernel<0, false>, ctas, sh.C, sh.smem, stream, L, target);
 }
 
 cudaError_t launch_dyn_deriv(const SweepLaunch& L, cudaStream_t stream) {

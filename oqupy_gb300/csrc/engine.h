@@ -169,6 +169,7 @@ struct SweepLaunch {
   int num_steps;
   int cap;              // bond capacity of the process tensor's slots
   int max_bond;         // largest bond of the swept steps
+  int wide;             // sweep_is_wide of the swept steps
   int max_cols;         // columns of a step per CTA (set at launch)
   long long stage;      // elements of a staging buffer in shared memory (set at launch; 0: none)
   const double* sites;  // as in DynLaunch
@@ -189,6 +190,7 @@ struct SweepLaunch {
 
 cudaError_t launch_dyn_step(const DynLaunch& L, int r, cudaStream_t stream);
 cudaError_t launch_dyn_init(const DynLaunch& L, const double* rho0, cudaStream_t stream);
+bool sweep_is_wide(int D, int num_steps, const int2* dims);
 cudaError_t launch_sweep_prepare(const SweepLaunch& L, cudaStream_t stream);
 cudaError_t launch_sweep(const SweepLaunch& L, cudaStream_t stream);
 cudaError_t launch_sweep_back(const SweepLaunch& L, const double* target, cudaStream_t stream);
