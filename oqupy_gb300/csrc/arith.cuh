@@ -17,7 +17,7 @@ template <typename T>
 struct QA;
 
 // FP32 estimates without denormal handling (half the latency of the library
-// forms); their arguments are normal here
+// forms): a denormal argument counts as zero, so callers keep to normal ones
 __device__ __forceinline__ float rsqrt_est(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -42,6 +42,8 @@ __device__ __forceinline__ float trunc32(double d, unsigned* rest = nullptr) {
   return __uint_as_float(normal ? f : 0u);
 }
 __device__ __forceinline__ cx<float> trunc32(const cx<double>& a) { return mk<float>(trunc32(a.x), trunc32(a.y)); }
+
+constexpr float FP32_NORMAL = 1.17549435e-38f;   // smallest normal number
 
 template <>
 struct QA<double> {
@@ -105,12 +107,18 @@ struct QA<double> {
   static __device__ __forceinline__ void acc_fma(Acc& f, const E& a, const E& b) { cfma(f, a, b); }
   static __device__ __forceinline__ void acc_fmaj(Acc& f, const E& a, const E& b) { cjfma(f, a, b); }
   static __device__ __forceinline__ E acc_value(const Acc& f) { return f; }
-  // 1 / sqrt(u), 0 for u <= 0: the FP32 estimate refined to second order in
-  // FP64 (remaining relative error below 2^-64 before the final rounding),
-  // five FP64 instructions instead of the library's square root and division
+  // 1 / sqrt(u), 0 for u <= 0: the FP32 estimate y with the first two terms of
+  // the binomial series of (1 - r)^-1/2, r = 1 - u y^2, in FP64 (what is left out
+  // is below 2^-64 before the final rounding), five FP64 instructions instead of
+  // the library's square root and division.  Values below FP32's normal range
+  // are scaled into it, those below 2^-326 count as zero.
   static __device__ __forceinline__ S rsqrt(S u) {
+    if ((float)u < FP32_NORMAL && u > 0.0) return 0x1p+100 * rsqrt_normal(u * 0x1p+200);
+    return rsqrt_normal(u);
+  }
+  static __device__ __forceinline__ S rsqrt_normal(S u) {
     const float uf = (float)u;
-    if (!(uf > 0.f)) return u * 0.0;   // 0 (NaN stays NaN)
+    if (!(uf >= FP32_NORMAL)) return u * 0.0;   // 0 (NaN stays NaN)
     const double y = (double)rsqrt_est(uf);
     const double r = fma(-u, y * y, 1.0);
     return fma(y * r, fma(0.375, r, 0.5), y);
@@ -152,7 +160,7 @@ struct QA<double> {
     Rot q;
     q.tx = (double)tx;
     q.ty = (double)ty;
-    q.c = rsqrt(fma(q.tx, q.tx, fma(q.ty, q.ty, 1.0)));
+    q.c = rsqrt_normal(fma(q.tx, q.tx, fma(q.ty, q.ty, 1.0)));
     return q;
   }
   static __device__ __forceinline__ void rotate(const Rot& q, E& u, E& v) {
@@ -248,10 +256,11 @@ struct QA<ff> {
   static __device__ __forceinline__ void acc_fma(Acc& f, const E& a, const E& b) { ccacc_fma(f, a, b); }
   static __device__ __forceinline__ void acc_fmaj(Acc& f, const E& a, const E& b) { ccacc_fmaj(f, a, b); }
   static __device__ __forceinline__ E acc_value(const Acc& f) { return ccacc_cff(f); }
-  // 1 / sqrt(u), 0 for u <= 0: the FP32 estimate y refined to second order,
-  // the residual 1 - u y^2 formed from exact products
+  // 1 / sqrt(u), 0 for u <= 0: as in FP64, the residual 1 - u y^2 formed from
+  // exact products.  A squared norm below the normal range has no digits left
+  // and counts as zero (a column 1e-19 of the largest, 2^-48 being rounding).
   static __device__ __forceinline__ S rsqrt(S u) {
-    if (!(u.hi > 0.f)) return ff_make(u.hi * 0.f, 0.f);
+    if (!(u.hi >= FP32_NORMAL)) return ff_make(u.hi * 0.f, 0.f);
     const float y = rsqrt_est(u.hi);
     const float p = __fmul_rn(y, y), pe = __fmaf_rn(y, y, -p);
     float r = __fmaf_rn(-u.hi, p, 1.f);

@@ -45,6 +45,7 @@ namespace otb {
 // 196 instead of 174 ms).
 constexpr int PRESWEEP_MIN_COLS = 10;
 constexpr int PRESWEEP_CORRECTIONS = 2;
+constexpr float PRESWEEP_MIN_NORM2 = 1e-33f;   // B / A stays below 1e37 for norms of up to 1152 columns
 constexpr float PRESWEEP_MAX_TAN = 4e-6f;   // larger tangents are left to the sweeps
 
 // FP32 one-sided Jacobi sweeps on F (m + k rows, k columns, ld m + k): the
@@ -123,7 +124,9 @@ __device__ void presweeps32_rc(cx<float>* F, int m, int k, float* nrm2) {
         const float rr = rsqrt_est(A) * rsqrt_est(B);
         const float x = (up ? o : s) * rr, y = (up ? s : o) * rr;
         const float c2 = fmaf(x, x, y * y);
-        if (active && c2 > tol2) {   // false for NaN (zero columns)
+        // columns at the end of FP32's range are left to the FP64 sweeps: above it
+        // all of the angle's factors are finite (c2 is NaN for zero columns)
+        if (active && c2 > tol2 && c2 < 1e30f && fminf(A, B) > PRESWEEP_MIN_NORM2) {
           large |= c2 > 1e-6f;
           const float d = 0.5f * ((B - A) * rr);
           const float hh = fmaf(d, d, c2);
