@@ -242,10 +242,13 @@ __device__ int jacobi_sweeps(typename QA<T>::E* W, int m, int n, int ld, typenam
   return jacobi_sweeps_rc<T, 16, 4, false>(W, m, n, ld, nrm2, sh);
 }
 
-// Descending order of the n values norm[] and the kept rank (>= 1): the
-// second half of jacobi_finish, for callers that computed the norms.
+// Descending order of the n values norm[] and the kept rank (>= 1).  tail2 is the
+// squared norm, over scale^2, of a block dropped before the sweeps.  Where the
+// largest value is below 2^-400 or above 2^400, squares are summed in units of a
+// power of two next to it, so that their sum stays in range; a largest value
+// whose own square does not is refused.
 __device__ inline int jacobi_rank(int n, double epsrel, double* norm, int* perm, JacobiShared* sh,
-                                  int sweeps, double tail2) {
+                                  int sweeps, double tail2, double scale) {
   const int tid = threadIdx.x;
   const int nthreads = blockDim.x;
   // norms are >= 0: their bit patterns order like the values (no FP64 compare)
@@ -260,15 +263,30 @@ __device__ inline int jacobi_rank(int n, double epsrel, double* norm, int* perm,
   }
   __syncthreads();
   if (tid == 0) {
-    const double thr = epsrel * norm[perm[0]];
-    const double thr2 = thr * thr;
-    double cum = tail2;  // squared norm of a block dropped before the sweeps (all in the tail)
+    const double s0 = norm[perm[0]];
+    const int e = (__double2hiint(s0) >> 20) & 0x7ff;
+    double cum;
     int kept = 0;
+    // (the units cost an FP64 multiplication a value: 1 % of small splits)
+    if (e > 623 && e < 1423) {
+      const double thr = epsrel * s0, thr2 = thr * thr;
+      cum = tail2 * scale * scale;  // a block dropped before the sweeps is all in the tail
 #pragma unroll 4
-    for (int r = n - 1; r >= 0; --r) {
-      const double s = norm[perm[r]];
-      cum = fma(s, s, cum);
-      kept += (cum > thr2) ? 1 : 0;
+      for (int r = n - 1; r >= 0; --r) {
+        const double s = norm[perm[r]];
+        cum = fma(s, s, cum);
+        kept += (cum > thr2) ? 1 : 0;
+      }
+    } else {
+      const double unit = __hiloint2double((e > 1 && e < 2045 ? 2046 - e : 1023) << 20, 0);   // about 1 / s0
+      const double thr = epsrel * (s0 * unit), thr2 = thr * thr;
+      cum = tail2 * (scale * unit) * (scale * unit);
+      for (int r = n - 1; r >= 0; --r) {
+        const double s = norm[perm[r]] * unit;
+        cum = fma(s, s, cum);
+        kept += (cum > thr2) ? 1 : 0;
+      }
+      if (!isfinite(s0 * s0)) cum = s0 * s0;
     }
     if (kept < 1) kept = 1;
     sh->kept = kept;

@@ -554,7 +554,6 @@ __device__ int qr_jacobi_truncate(typename QA<T>::E* X, bool x_shared, int R, in
   E* Z = ((size_t)N * N * sizeof(E) <= zs_bytes) ? reinterpret_cast<E*>(zs) : Zg;
   float tail2;
   const int k = pivoted_qr<T>(X, R, N, delta, bk, Z, &tail2);
-  const double t2 = (double)tail2 * scale * scale;
   const bool second = k >= 8 && 2 * k <= N;
   if (Z == Zg) {
     E* to = (size_t)N * k * sizeof(E) <= zs_bytes ? reinterpret_cast<E*>(zs) : (x_shared && !second ? X : Zg);
@@ -583,7 +582,7 @@ __device__ int qr_jacobi_truncate(typename QA<T>::E* X, bool x_shared, int R, in
       }
     }
     const int sw64 = jacobi_norms<T>(R2, k, k, k, scale, norm, sh);
-    const int kk = jacobi_rank(k, epsrel, norm, perm, sh, sw64, t2);
+    const int kk = jacobi_rank(k, epsrel, norm, perm, sh, sw64, tail2, scale);
     for (int idx = tid; idx < k * kk; idx += nt) {
       const int j = idx / k, i = idx - j * k;
       E* e = R2 + (size_t)perm[j] * k + i;
@@ -630,7 +629,7 @@ __device__ int qr_jacobi_truncate(typename QA<T>::E* X, bool x_shared, int R, in
     }
   }
   const int sw64 = jacobi_norms<T>(Z, N, k, N, scale, norm, sh);
-  const int kk = jacobi_rank(k, epsrel, norm, perm, sh, sw64, t2);
+  const int kk = jacobi_rank(k, epsrel, norm, perm, sh, sw64, tail2, scale);
   *Wout = Z;
   return kk;
 }

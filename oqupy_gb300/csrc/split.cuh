@@ -89,7 +89,7 @@ __device__ __forceinline__ SplitOut<T> oriented_split(const Acc& A, int R, int N
     return o;
   }
   const int sw64 = jacobi_norms<T>(X, R, N, R, scale, sh.book.norm, &sh.jsh);
-  o.kk = jacobi_rank(N, epsrel, sh.book.norm, sh.book.perm, &sh.jsh, sw64, 0.0);
+  o.kk = jacobi_rank(N, epsrel, sh.book.norm, sh.book.perm, &sh.jsh, sw64, 0.0, scale);
   o.W = X;
   return o;
 }

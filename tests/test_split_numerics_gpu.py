@@ -62,6 +62,27 @@ def test_columns_whose_squares_leave_the_fp32_range(lib, precision, small, R, N,
     assert np.linalg.norm(A - (U * got) @ V.conj().T, 2) < bound
 
 
+@pytest.mark.parametrize("N", [5, 12])
+@pytest.mark.parametrize("scale", [1e-150, 1e150, 1.2e154])
+def test_rank_decision_near_the_ends_of_the_fp64_range(lib, N, scale):
+    """Squares of the single values fit in FP64, their sum need not."""
+    rng = np.random.default_rng(N)
+    s = np.where(np.arange(N) < N - 2, 1.0, 1e-6)
+    A = (unitary(rng, 2 * N, N) * s) @ unitary(rng, N, N).conj().T * scale
+    U, got, V, status = split_probe.split(lib, A, 1e-5)
+    assert status == 0 and len(got) == N - 2
+    np.testing.assert_allclose(got / scale, 1.0, rtol=0, atol=4 * N ** 1.5 * EPS["complex128"])
+
+
+@pytest.mark.parametrize("N", [5, 12])
+@pytest.mark.parametrize("value", [1e160, np.inf, np.nan])
+def test_values_whose_squares_overflow_are_refused(lib, N, value):
+    rng = np.random.default_rng(N)
+    A = unitary(rng, 2 * N, N)
+    A[3, 2] = value
+    assert split_probe.split(lib, A, 1e-8)[3] == -6
+
+
 def test_reciprocal_square_roots(lib):
     """Against 1 / sqrt in extended precision.  FP64: y + y (r / 2 + 3 r^2 / 8)
     with r = 1 - u y^2 for an FP32 estimate y (relative error below 2^-22,
