@@ -1,5 +1,6 @@
 // Host side of the PT-TEMPO and process-tensor sweep C ABI.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -13,6 +14,22 @@
 #include "engine.h"
 
 using namespace otb;
+
+namespace {
+
+// Device memory that all handles of the process together keep for their sweeps.
+constexpr size_t SWEEP_KEEP_BYTES = (size_t)256 << 20;
+std::atomic<size_t> g_sweep_kept{0};
+
+// Makes room for `more` bytes; false if they do not fit.
+bool reserve_kept(size_t more) {
+  size_t kept = g_sweep_kept.load();
+  while (more <= SWEEP_KEEP_BYTES - kept)
+    if (g_sweep_kept.compare_exchange_weak(kept, kept + more)) return true;
+  return false;
+}
+
+}  // namespace
 
 struct otb_pt {
   int n = 0;
@@ -29,15 +46,19 @@ struct otb_pt {
   // completed builds: their bonds on the host (a completed build never changes)
   std::mutex mutex;
   std::vector<std::vector<int2>> final_dims;
-  // workspace of the sweeps, kept between calls up to SWEEP_KEEP_BYTES; a call
-  // that finds it in use (another thread's) allocates its own
+  // workspace of the sweeps, kept between calls while all handles' fit into
+  // SWEEP_KEEP_BYTES; a call that finds it in use (another thread's) or too
+  // small to grow allocates its own
   std::mutex sweep_mutex;
   DevBuf sweep_ws;
+  ~otb_pt() {
+    const size_t kept = sweep_ws.bytes;
+    sweep_ws.release();
+    g_sweep_kept -= kept;
+  }
 };
 
 namespace {
-
-constexpr size_t SWEEP_KEEP_BYTES = (size_t)256 << 20;
 
 otb_status pt_check(otb_pt* h, int32_t inst) {
   if (!h) return set_error(OTB_ERR_INVALID_ARG, "null handle");
@@ -288,7 +309,7 @@ otb_status completed_dims(otb_pt* h, int32_t inst, std::vector<int2>& dims) {
 }
 
 // Device memory of one sweep: the handle's kept workspace when it is free and
-// small enough, else an allocation of its own.
+// large enough or may grow, else an allocation of its own.
 struct SweepWorkspace {
   otb_pt* h;
   std::unique_lock<std::mutex> lock;
@@ -297,12 +318,20 @@ struct SweepWorkspace {
   explicit SweepWorkspace(otb_pt* h_) : h(h_) {}
   bool get(size_t bytes) {
     lock = std::unique_lock<std::mutex>(h->sweep_mutex, std::try_to_lock);
-    if (lock.owns_lock() && bytes <= SWEEP_KEEP_BYTES) {
-      if (h->sweep_ws.bytes < bytes && !h->sweep_ws.alloc(bytes)) return false;
-      p = (char*)h->sweep_ws.p;
-      return true;
+    if (lock.owns_lock()) {
+      DevBuf& ws = h->sweep_ws;
+      if (ws.bytes < bytes && reserve_kept(bytes - ws.bytes)) {
+        if (!ws.alloc(bytes)) {   // (the former workspace is gone too)
+          g_sweep_kept -= bytes;
+          return false;
+        }
+      }
+      if (ws.bytes >= bytes) {
+        p = (char*)ws.p;
+        return true;
+      }
+      lock.unlock();
     }
-    if (lock.owns_lock()) lock.unlock();
     if (!own.alloc(bytes)) return false;
     p = (char*)own.p;
     return true;
