@@ -586,9 +586,11 @@ __global__ void __launch_bounds__(DYN_THREADS) dyn_deriv_kernel(SweepLaunch L) {
 // Many systems: one CTA per SM with its share of them (every load of A serves
 // all of a CTA's systems).  Few: the step's columns are split over up to eight
 // CTAs while a CTA's FP64 work of a step (2 l r D clocks on one SM) is above
-// 3000 clocks: the exchange through the cluster costs about 1000, and below
-// that a step's fixed chain of phases (about 6000 clocks) hides what is saved
-// (8 systems, bond 13: 200 us a sweep on one CTA each, 175 us on eight).
+// 3000 clocks (bond 20 with D = 4).  8 systems, 60 steps, whole calls on 1 / 2 /
+// 4 / 8 CTAs each, sweep and gradient in us: bond 9 202 224 213 215, 390 436 436
+// 437; bond 15 252 249 240 236, 474 474 472 475; bond 37 673 487 398 393, 1381 969
+// 783 769; bond 112 2955 1661 948 611, 6834 4102 2715 1995.  Below the line the
+// cluster's barrier takes what the split saves.
 struct SweepShape {
   int S, C, max_cols;
   size_t stage;   // elements of one staging buffer, 0 = columns read from global memory

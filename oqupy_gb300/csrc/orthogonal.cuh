@@ -34,12 +34,19 @@
 
 namespace otb {
 
-// Splits of fewer columns go straight to the sweeps.  From 8 columns on the
-// products are faster (three builds of 14 steps: 18.2 ms, 19.3 ms with 10, 22.2
-// with 16), but sweeps keep a small column to its own rounding and products only
-// to that of the largest one, which decides exactly tied pairs otherwise: in a
-// mean-field model with such a pair the states' distance from the reference at
-// step 13 is 6e-11 with 10, 12, 16 or no products, 1.1e-10 with 8.
+// Splits of fewer columns go straight to the sweeps.  Sweeps keep a small column to
+// its own rounding, products only to that of the largest one; but the QR's
+// backward error is that of the largest one already, so a split is as accurate
+// either way: singular values and the reconstruction to 4 N^1.5 unit roundoffs of
+// the largest singular value (tests/test_split_numerics_gpu.py; exactly tied pairs
+// over 0 to 9 decades, 8 to 40 columns, 12 operands each: singular values off by
+// at most 9 unit roundoffs with products and 10 with sweeps, the smallest pair by
+// the same 0.2 to 0.5, the reconstruction by at most 15 and 16).  What differs is
+// which vector of a tied pair a truncation at that level keeps.  From 8 columns on
+// the products are faster (three builds of 14 steps: 18.2 ms, 19.3 ms with 10, 22.2
+// with 16); 10 is where the kept vectors of the narrow splits of a mean-field
+// model with such a pair stay those of the sweeps (distance of its states from the
+// reference at step 13: 6e-11 with 10, 12, 16 or no products, 1.1e-10 with 8).
 // Double-float splits never take this way: their products run on the pipe that
 // the sweeps are bound by (95 instances, splits of ~77 x 35: the 12 steps take
 // 196 instead of 174 ms).
