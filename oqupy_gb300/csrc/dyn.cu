@@ -36,7 +36,11 @@ typedef cx<double> zc;
 constexpr int DYN_RB = 32;       // output bond indices per CTA
 constexpr int DYN_THREADS = 128;
 
-__global__ void __launch_bounds__(DYN_THREADS) dyn_step_kernel(DynLaunch L) {
+// Eight CTAs per SM (64 registers): left to itself the compiler takes 32 and
+// spills.  A session of one system: 60 steps at bond 90 (D = 4) 2750 -> 2620 us,
+// 2748 with 40 registers; 24 steps at bond 55 (D = 9) 1840 -> 1605 us; 1024 systems
+// 14.8 -> 14.7 and 8.2 -> 8.1 ms.
+__global__ void __launch_bounds__(DYN_THREADS, 8) dyn_step_kernel(DynLaunch L) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ int last;
   const int h = blockIdx.y;
