@@ -595,6 +595,16 @@ __global__ void __launch_bounds__(DYN_THREADS) dyn_deriv_kernel(SweepLaunch L) {
 // 437; bond 15 252 249 240 236, 474 474 472 475; bond 37 673 487 398 393, 1381 969
 // 783 769; bond 112 2955 1661 948 611, 6834 4102 2715 1995.  Below the line the
 // cluster's barrier takes what the split saves.
+// Two CTAs each as well from half a system to one and a half per SM, where the
+// columns of half a step are too wide to stage (bond 54 on with D = 4, 37 with
+// D = 9), so that several CTAs fit on an SM: a whole system more on one SM than
+// on the next doubles the call, half a one adds a half.  60 steps, bond 60 and 90,
+// one CTA (above 152 systems two systems each) -> two: 77 systems 962 1956 -> 959
+// 1663, 152 systems 1002 1979 -> 984 1692, 153 systems 1701 3412 -> 1355 2406, 228
+// systems 1710 3421 -> 1369 2425; 230 systems 1714 3421 -> 1797 3266.  Gradients,
+// bond 90: 77 systems 7095 -> 6503, 153 systems 11990 -> 10720.  D = 9, bond 55: 77
+// systems 789 -> 778, 153 systems 1431 -> 1195.  Staged columns (bond 36): 153
+// systems 990 -> 1014, 190 systems 996 -> 1269.
 struct SweepShape {
   int S, C, max_cols;
   size_t stage;   // elements of one staging buffer, 0 = columns read from global memory
@@ -606,23 +616,24 @@ static SweepShape sweep_shape(const SweepLaunch& L, int max_s) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   sms = sms > 0 ? sms : 1;
+  const size_t limit = 200 * 1024;
+  const auto cols = [&](int C) { return (L.max_bond + C) / C; };
+  const auto bytes = [&](int S, int C) {
+    return ((size_t)2 * S * L.max_bond * L.D + (size_t)S * cols(C) * L.D + (size_t)4 * S * L.D * L.D) * sizeof(zc);
+  };
+  const auto stage = [&](int C) { return (size_t)L.max_bond * L.D * cols(C); };
+  const auto staged = [&](int S, int C) { return bytes(S, C) + 2 * stage(C) * sizeof(zc) <= limit; };
   SweepShape sh;
   const double clocks = 2.0 * L.max_bond * L.max_bond * L.D;
   sh.C = 1;
   while (sh.C < 8 && 2 * sh.C * L.nh <= sms && clocks > 3000.0 * sh.C) sh.C *= 2;
+  if (2 * L.nh > sms && 2 * L.nh <= 3 * sms && clocks > 3000.0 && !staged(1, 2)) sh.C = 2;
   sh.S = sh.C > 1 ? 1 : std::min(max_s, (L.nh + sms - 1) / sms);
-  const size_t limit = 200 * 1024;
-  for (;; --sh.S) {
-    sh.max_cols = (L.max_bond + sh.C) / sh.C;
-    sh.smem = ((size_t)2 * sh.S * L.max_bond * L.D + (size_t)sh.S * sh.max_cols * L.D +
-               (size_t)4 * sh.S * L.D * L.D) * sizeof(zc);
-    if (sh.smem <= limit || sh.S == 1) break;
-  }
-  sh.stage = (size_t)L.max_bond * L.D * sh.max_cols;
-  if (sh.smem + 2 * sh.stage * sizeof(zc) <= limit)
-    sh.smem += 2 * sh.stage * sizeof(zc);
-  else
-    sh.stage = 0;
+  while (sh.S > 1 && bytes(sh.S, sh.C) > limit) --sh.S;
+  sh.max_cols = cols(sh.C);
+  sh.smem = bytes(sh.S, sh.C);
+  sh.stage = staged(sh.S, sh.C) ? stage(sh.C) : 0;
+  sh.smem += 2 * sh.stage * sizeof(zc);
   return sh;
 }
 
