@@ -415,8 +415,16 @@ __device__ void pt_caps(PtCtx<MIXED>& c, PtShared& sh) {
   __syncthreads();
 }
 
-template <bool MIXED>
-__global__ void __launch_bounds__(PT_THREADS) pt_kernel(PtLaunch L) {
+// CTAS: CTAs per SM that the registers are allocated for.  The mixed form takes
+// 249 registers a thread where it may, which fill an SM with one CTA, and 128
+// otherwise (one CTA alone takes 1.12 times as long with 128: its loops hold
+// fewer rows).  Builds of 24 and 152 process tensors, memory of 10 and 12 steps,
+// on 249 | 128 registers: 49.3 66.3 | 56.2 74.9 ms; of 200 and 304, memory of 12
+// steps, 119 131 | 101 113 ms; of 304, memory of 6 and 20 steps, 28.6 732 | 23.3
+// 623 ms.  So: 128 registers for grids of more CTAs than SMs.  The complex128 form
+// takes 128 either way.
+template <bool MIXED, int CTAS>
+__global__ void __launch_bounds__(PT_THREADS, CTAS) pt_kernel(PtLaunch L) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ PtShared sh;
   for (;;) {
@@ -457,21 +465,25 @@ __global__ void __launch_bounds__(PT_THREADS) pt_kernel(PtLaunch L) {
   }
 }
 
-cudaError_t launch_pt(const PtLaunch& L, int precision, int grid, int block, cudaStream_t stream) {
-  const int smem = 88 * 1024;
-  PtLaunch l2 = L;
-  l2.smem_bytes = smem;
-  cudaError_t e;
-  if (precision == 0) {
-    e = cudaFuncSetAttribute(pt_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    pt_kernel<false><<<grid, block, smem, stream>>>(l2);
-  } else {
-    e = cudaFuncSetAttribute(pt_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    pt_kernel<true><<<grid, block, smem, stream>>>(l2);
-  }
+template <bool MIXED, int CTAS>
+static cudaError_t launch_pt_kernel(const PtLaunch& L, int grid, int block, cudaStream_t stream) {
+  const cudaError_t e =
+      cudaFuncSetAttribute(pt_kernel<MIXED, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem_bytes);
+  if (e != cudaSuccess) return e;
+  pt_kernel<MIXED, CTAS><<<grid, block, L.smem_bytes, stream>>>(L);
   return cudaGetLastError();
+}
+
+cudaError_t launch_pt(const PtLaunch& L, int precision, int grid, int block, cudaStream_t stream) {
+  PtLaunch l2 = L;
+  l2.smem_bytes = 88 * 1024;   // two CTAs per SM
+  if (precision == 0) return launch_pt_kernel<false, 2>(l2, grid, block, stream);
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  return grid > sms ? launch_pt_kernel<true, 2>(l2, grid, block, stream)
+                    : launch_pt_kernel<true, 1>(l2, grid, block, stream);
 }
 
 }  // namespace otb
