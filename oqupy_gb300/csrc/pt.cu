@@ -415,14 +415,13 @@ __device__ void pt_caps(PtCtx<MIXED>& c, PtShared& sh) {
   __syncthreads();
 }
 
-// CTAS: CTAs per SM that the registers are allocated for.  The mixed form takes
-// 249 registers a thread where it may, which fill an SM with one CTA, and 128
-// otherwise (one CTA alone takes 1.12 times as long with 128: its loops hold
-// fewer rows).  Builds of 24 and 152 process tensors, memory of 10 and 12 steps,
-// on 249 | 128 registers: 49.3 66.3 | 56.2 74.9 ms; of 200 and 304, memory of 12
-// steps, 119 131 | 101 113 ms; of 304, memory of 6 and 20 steps, 28.6 732 | 23.3
-// 623 ms.  So: 128 registers for grids of more CTAs than SMs.  The complex128 form
-// takes 128 either way.
+// CTAS: CTAs per SM that the registers are allocated for, 0 = the compiler's
+// choice.  That is 249 registers a thread in the mixed form, which fill an SM with
+// one CTA; the 128 of two spill (one CTA alone takes 1.13 times as long).  Builds of 24
+// and 152 process tensors, memory of 10 and 12 steps, on 249 | 128 registers: 49.3
+// 66.3 | 56.2 74.9 ms; of 200 and 304, memory of 12 steps, 119 131 | 101 113 ms; of
+// 304, memory of 6 and 20 steps, 28.6 732 | 23.3 623 ms.  So: 128 registers for
+// grids of more CTAs than SMs.  The complex128 form takes 128 by itself.
 template <bool MIXED, int CTAS>
 __global__ void __launch_bounds__(PT_THREADS, CTAS) pt_kernel(PtLaunch L) {
   extern __shared__ __align__(16) unsigned char dsm[];
@@ -477,13 +476,13 @@ static cudaError_t launch_pt_kernel(const PtLaunch& L, int grid, int block, cuda
 cudaError_t launch_pt(const PtLaunch& L, int precision, int grid, int block, cudaStream_t stream) {
   PtLaunch l2 = L;
   l2.smem_bytes = 88 * 1024;   // two CTAs per SM
-  if (precision == 0) return launch_pt_kernel<false, 2>(l2, grid, block, stream);
+  if (precision == 0) return launch_pt_kernel<false, 0>(l2, grid, block, stream);
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   return grid > sms ? launch_pt_kernel<true, 2>(l2, grid, block, stream)
-                    : launch_pt_kernel<true, 1>(l2, grid, block, stream);
+                    : launch_pt_kernel<true, 0>(l2, grid, block, stream);
 }
 
 }  // namespace otb
