@@ -32,11 +32,6 @@ template <typename T>
 __device__ __forceinline__ cx<T> cmul(cx<T> a, cx<T> b) {
   return mk<T>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-// conj(a) * b
-template <typename T>
-__device__ __forceinline__ cx<T> cjmul(cx<T> a, cx<T> b) {
-  return mk<T>(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
-}
 // acc += a * b
 template <typename T>
 __device__ __forceinline__ void cfma(cx<T>& acc, cx<T> a, cx<T> b) {
@@ -61,23 +56,6 @@ template <typename T>
 __device__ __forceinline__ cx<T> cconj(cx<T> a) {
   return mk<T>(a.x, -a.y);
 }
-template <typename To, typename From>
-__device__ __forceinline__ cx<To> ccast(cx<From> a) {
-  return mk<To>((To)a.x, (To)a.y);
-}
-
-template <typename T>
-struct num;
-template <>
-struct num<double> {
-  static __device__ __forceinline__ double eps() { return 1.1102230246251565e-16; }
-  static __device__ __forceinline__ double big_zeta() { return 1.0e150; }
-};
-template <>
-struct num<float> {
-  static __device__ __forceinline__ float eps() { return 5.9604645e-08f; }
-  static __device__ __forceinline__ float big_zeta() { return 1.0e18f; }
-};
 
 // Status codes shared with the host (mirrored in include/oqupy_gb300.h).
 enum : int {

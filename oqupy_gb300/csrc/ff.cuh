@@ -42,7 +42,6 @@ __device__ __forceinline__ ff ff_add(ff a, ff b) {
   const float e = __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo));
   return fast_two_sum(s.hi, e);
 }
-__device__ __forceinline__ ff ff_sub(ff a, ff b) { return ff_add(a, ff_make(-b.hi, -b.lo)); }
 __device__ __forceinline__ ff ff_mul(ff a, ff b) {
   const float p = __fmul_rn(a.hi, b.hi);
   float e = __fmaf_rn(a.hi, b.hi, -p);
@@ -50,34 +49,6 @@ __device__ __forceinline__ ff ff_mul(ff a, ff b) {
   e = __fmaf_rn(a.lo, b.hi, e);
   return fast_two_sum(p, e);
 }
-// acc + a * b
-__device__ __forceinline__ ff ff_fma(ff a, ff b, ff acc) { return ff_add(acc, ff_mul(a, b)); }
-
-// 1/sqrt(u) for u > 0: float estimate refined by one Newton step in FF
-__device__ __forceinline__ ff ff_rsqrt(ff u) {
-  const float y0 = rsqrtf(u.hi);
-  const ff y = ff_make(y0, 0.f);
-  const ff e = ff_sub(ff_make(1.f, 0.f), ff_mul(u, ff_mul(y, y)));
-  return ff_add(y, ff_mul(ff_make(0.5f * y0, 0.f), e));
-}
-
-// sqrt(u) for u >= 0: the IEEE float square root refined by one Newton step
-// in FF (y + (u - y^2) / (2 y)); 0 for u <= 0
-__device__ __forceinline__ ff ff_sqrt(ff u) {
-  if (!(u.hi > 0.f)) return ff_make(0.f, 0.f);
-  const float y = __fsqrt_rn(u.hi);
-  const ff e = ff_sub(u, ff_mul(ff_make(y, 0.f), ff_make(y, 0.f)));
-  return ff_add(ff_make(y, 0.f), ff_make(__fdiv_rn(e.hi, 2.f * y), 0.f));
-}
-
-// 1 / b for b != 0: the IEEE float reciprocal refined by one Newton step in
-// FF (y + y (1 - b y))
-__device__ __forceinline__ ff ff_recip(ff b) {
-  const float y = __fdiv_rn(1.f, b.hi);
-  const ff e = ff_sub(ff_make(1.f, 0.f), ff_mul(b, ff_make(y, 0.f)));
-  return ff_add(ff_make(y, 0.f), ff_mul(ff_make(y, 0.f), e));
-}
-
 __device__ __forceinline__ ff ff_shfl_xor(ff v, int off) {
   return ff_make(__shfl_xor_sync(0xffffffffu, v.hi, off, 32), __shfl_xor_sync(0xffffffffu, v.lo, off, 32));
 }
@@ -180,12 +151,6 @@ __device__ __forceinline__ cff cff_conj(cff a) {
   a.y.hi = -a.y.hi;
   a.y.lo = -a.y.lo;
   return a;
-}
-
-__device__ __forceinline__ cff cff_mul(const cff& a, const cff& b) {
-  ccacc f = ccacc_zero();
-  ccacc_fma(f, a, b);
-  return ccacc_cff(f);
 }
 
 __device__ __forceinline__ cx<double> ccacc_value(const ccacc& a) {

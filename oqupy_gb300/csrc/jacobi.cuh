@@ -21,7 +21,6 @@ namespace otb {
 constexpr int JACOBI_MAX_SWEEPS = 60;
 
 struct JacobiShared {
-  double red[33];
   unsigned worst;   // largest relative off-diagonal rotated in the last allowed sweep (float bits)
   unsigned c2max[2], t2max[2];   // largest rotated squared cosine and scaled tangent of a sweep (float bits)
   int noise_converged;
