@@ -535,7 +535,7 @@ def run_pt(args):
         props = [bath.half_step_propagators(a * sx + c * sz, 0.02) for a, c in ab]
         p1 = np.array([p[0] for p in props]); p2 = np.array([p[1] for p in props])
         rho0 = np.tile(np.array([1, 0, 0, 0], dtype=complex), (nh, 1))
-        bm.dynamics(0, p1, p2, rho0)                  # warm-up (graph build)
+        bm.dynamics(0, p1, p2, rho0)                  # warm-up (workspace)
         t0 = time.perf_counter()
         reps = 3
         for _ in range(reps):

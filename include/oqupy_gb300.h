@@ -228,8 +228,7 @@ otb_status otb_pt_get_cap(otb_pt* h, int32_t inst, int32_t step, double* out,
  * prop1/prop2 are n_systems * D * D complex half-step propagators (with any
  * transform_in / transform_out of the process tensor folded in: P1 <- Tin^T P1,
  * P2 <- P2 Tout^T), rho0 is n_systems * D, out receives
- * (num_steps+1) * n_systems * D complex.  The num_steps launches are replayed
- * as one CUDA graph. */
+ * (num_steps+1) * n_systems * D complex.  All steps run in one launch. */
 otb_status otb_dyn_run(otb_pt* h, int32_t inst, int32_t n_systems,
                        const double* prop1, const double* prop2,
                        const double* rho0, int32_t num_steps, double* out,
