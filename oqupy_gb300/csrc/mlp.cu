@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(TC_THREADS)
 // memory as whole row segments (output layer 144 us, 190 without).  A training
 // step of 256 points, where the 1500-column operands were staged element by
 // element and both operands of every weight gradient transposed first: 1020 ->
-// 312 us, launches 45 -> 19.
+// 330 us, launches 45 -> 19.
 //
 // Used when rows are 16-byte aligned; other operands keep the kernel above.
 // Tile width: 256 where that gives every SM a tile, else 128, else 64 (a
